@@ -43,6 +43,8 @@ SIGNATURES = {
     "eppgcn_tile_plan_active_rows": (_I, [_P, _P, _P]),
     "eppgcn_tile_plan_used": (_I, [_P, _P]),
     "eppgcn_update_rows": (_I, [_P, _LL, _P, _LL, _P, _LL, _LL, _P, _P, _LL, _I, _I, _I, _I, _I, _P]),
+    "eppgcn_update_scratch_bytes": (_SZ, [_I, _I, _I]),
+    "eppgcn_update_rows_scratch": (_I, [_P, _LL, _P, _LL, _P, _LL, _LL, _P, _P, _LL, _I, _I, _I, _I, _I, _P, _SZ, _P]),
     "eppgcn_update_listed": (_I, [_P, _LL, _P, _LL, _P, _LL, _LL, _P, _P, _LL, _I, _P, _I, _I, _I, _I, _P]),
     "eppgcn_spmm_tiles_active": (_I, [_P, _LL, _P, _LL, _P, _P, _I, _P]),
     "eppgcn_tile_plan_missing": (_I, [_P, _P, _P, _P, _P, _P]),
@@ -159,9 +161,10 @@ def update_scaled(x, w, scale=None, pad_to=8):
     return full[:, :dout]
 
 
-def update_rows(x, w, scale=None, gate=None, relu_x=False, out=None, rows=None):
-    """With ``rows`` only those rows of ``out``.  ``scale * (f(x) @ w)`` for any width and any strides of ``w``; ``f`` is ReLU with ``relu_x``, and results whose
-    ``gate`` entry is not positive become 0."""
+def update_rows(x, w, scale=None, gate=None, relu_x=False, out=None, rows=None, use_scratch=True):
+    """``scale * (f(x) @ w)`` for any width and any strides of ``w``; ``f`` is ReLU with ``relu_x``, and results whose
+    ``gate`` entry is not positive become 0.  With ``rows`` only those rows of ``out``; without ``use_scratch`` no
+    buffer is given, and a long k is not cut into stretches."""
     n, k, dout = x.size(0), x.size(1), w.size(1)
     if out is None:
         out = torch.empty((n, dout), dtype=torch.float32, device=x.device)
@@ -172,10 +175,15 @@ def update_rows(x, w, scale=None, gate=None, relu_x=False, out=None, rows=None):
                                          0 if gate is None else _row_stride(gate, "gate"), int(relu_x),
                                          _dev(rows, torch.int32, "rows"), rows.numel(), k, dout, 0, _stream()))
         return out
-    check(lib().eppgcn_update_rows(out.data_ptr(), _row_stride(out, "out"), x.data_ptr(), _row_stride(x, "x"), w.data_ptr(),
-                                   w.stride(0), w.stride(1), _dev(scale, torch.float32, "scale"),
-                                   None if gate is None else gate.data_ptr(),
-                                   0 if gate is None else _row_stride(gate, "gate"), int(relu_x), n, k, dout, 0, _stream()))
+    args = (out.data_ptr(), _row_stride(out, "out"), x.data_ptr(), _row_stride(x, "x"), w.data_ptr(),
+            w.stride(0), w.stride(1), _dev(scale, torch.float32, "scale"), None if gate is None else gate.data_ptr(),
+            0 if gate is None else _row_stride(gate, "gate"), int(relu_x), n, k, dout, 0)
+    nbytes = lib().eppgcn_update_scratch_bytes(n, k, dout) if use_scratch else 0
+    if nbytes:
+        scratch = torch.empty(nbytes // 4, dtype=torch.float32, device=x.device)
+        check(lib().eppgcn_update_rows_scratch(*args, scratch.data_ptr(), nbytes, _stream()))
+    else:
+        check(lib().eppgcn_update_rows(*args, _stream()))
     return out
 
 

@@ -226,6 +226,36 @@ torch::Tensor pack_scaled(const eppgcn_tile_plan *plan, const torch::Tensor &x, 
   return full.narrow(1, 0, d);
 }
 
+// Device buffers of a step: allocated as they are asked for; `keep` holds on to all of them (a graph's own buffers).
+struct NetBuffers {
+  bool keep = false;
+  std::vector<torch::Tensor> kept;
+  size_t next = 0;
+  torch::Tensor rows(int64_t n, int64_t ld, const torch::Tensor &like) {
+    if (next < kept.size()) return kept[next++];
+    auto t = at::empty({n, ld}, like.options());
+    if (keep) {
+      kept.push_back(t);
+      ++next;
+    }
+    return t;
+  }
+};
+
+// out[r] = scale[r] * f(x[r]) @ w over n rows (see eppgcn_update_rows); the sums of a long k's stretches lie in a buffer that
+// is taken from `buffers`.
+void update_rows(float *out, int64_t ld_out, const torch::Tensor &x, int64_t ldx, const float *w, int64_t w_row, int64_t w_col,
+                 const float *scale, const float *gate, int64_t ld_gate, bool relu_x, int64_t n, int64_t k, int64_t dout,
+                 int64_t pad_cols, NetBuffers &buffers, void *stream) {
+  const size_t bytes = eppgcn_update_scratch_bytes(static_cast<int>(n), static_cast<int>(k), static_cast<int>(dout));
+  torch::Tensor scratch;
+  if (bytes) scratch = buffers.rows(static_cast<int64_t>(bytes / sizeof(float)), 1, x);
+  epp_check(eppgcn_update_rows_scratch(out, ld_out, x.data_ptr<float>(), ldx, w, w_row, w_col, scale, gate, ld_gate,
+                                       relu_x ? 1 : 0, static_cast<int>(n), static_cast<int>(k), static_cast<int>(dout),
+                                       static_cast<int>(pad_cols), bytes ? scratch.data_ptr<float>() : nullptr, bytes, stream),
+            "eppgcn_update_rows_scratch");
+}
+
 // The dense kernels read x in 16-byte pieces from its start on.
 torch::Tensor aligned16(const torch::Tensor &x) {
   return reinterpret_cast<uintptr_t>(x.data_ptr<float>()) % 16 == 0 ? x : x.clone();
@@ -244,11 +274,10 @@ torch::Tensor update_scaled_padded(const torch::Tensor &x_in, const torch::Tenso
   TORCH_CHECK(degrees.numel() >= n, "degrees must have one entry per vertex");
   const int64_t ld = padded_width(d);
   auto full = at::empty({n, ld}, x.options());
+  NetBuffers buffers;
   if (n > 0)
-    epp_check(eppgcn_update_rows(full.data_ptr<float>(), ld, x.data_ptr<float>(), std::max(x.stride(0), k),
-                                 w.data_ptr<float>(), d, 1, degrees.data_ptr<float>(), nullptr, 0, 0, static_cast<int>(n), static_cast<int>(k),
-                                 static_cast<int>(d), static_cast<int>(ld - d), current_stream()),
-              "eppgcn_update_rows");
+    update_rows(full.data_ptr<float>(), ld, x, std::max(x.stride(0), k), w.data_ptr<float>(), d, 1, degrees.data_ptr<float>(),
+                nullptr, 0, false, n, k, d, ld - d, buffers, current_stream());
   return full.narrow(1, 0, d);
 }
 
@@ -280,11 +309,10 @@ std::vector<torch::Tensor> backward_update(const torch::Tensor &d_prime, const t
   TORCH_CHECK(n < (1LL << 31), "row count exceeds int32");
   TORCH_CHECK(X_in.size(0) == n && X_in.size(1) == din && W.size(1) == dout, "d_output, X and W do not fit together");
   auto d_input = need_d_input ? at::empty({n, din}, d_prime.options()) : at::empty({0}, d_prime.options());
+  NetBuffers buffers;
   if (need_d_input && n > 0)
-    epp_check(eppgcn_update_rows(d_input.data_ptr<float>(), din, d_prime.data_ptr<float>(), dout, W.data_ptr<float>(),
-                                 1, dout, nullptr, nullptr, 0, 0, static_cast<int>(n), static_cast<int>(dout),
-                                 static_cast<int>(din), 0, current_stream()),
-              "eppgcn_update_rows");
+    update_rows(d_input.data_ptr<float>(), din, d_prime, dout, W.data_ptr<float>(), 1, dout, nullptr, nullptr, 0, false, n, dout,
+                din, 0, buffers, current_stream());
   auto d_weight = at::zeros({din, dout}, d_prime.options());
   if (n > 0) add_weight_grad(d_weight.data_ptr<float>(), aligned16(X_in), d_prime, plan, false, current_stream());
   return {d_input, d_weight};
@@ -504,22 +532,6 @@ PlanPtr path_plan(const LayerPath &path, int64_t n) {
   return backward_plan(id, parts, edges, num_parts, n);
 }
 
-// Device buffers of a step: allocated as they are asked for; `keep` holds on to all of them (a graph's own buffers).
-struct NetBuffers {
-  bool keep = false;
-  std::vector<torch::Tensor> kept;
-  size_t next = 0;
-  torch::Tensor rows(int64_t n, int64_t ld, const torch::Tensor &like) {
-    if (next < kept.size()) return kept[next++];
-    auto t = at::empty({n, ld}, like.options());
-    if (keep) {
-      kept.push_back(t);
-      ++next;
-    }
-    return t;
-  }
-};
-
 // One [N, d] matrix per layer, before its activation; all but a `dense_last` last one in rows padded to 32 bytes.
 std::vector<torch::Tensor> run_forward(const torch::Tensor &x, const std::vector<torch::Tensor> &weights,
                                        const eppgcn_tile_plan *plan, const torch::Tensor &degrees, bool dense_last,
@@ -532,11 +544,8 @@ std::vector<torch::Tensor> run_forward(const torch::Tensor &x, const std::vector
     auto tmp = buffers.rows(n, ld, x);
     {
       ScopedMark t(0, 1, 0, clock_stream);
-      epp_check(eppgcn_update_rows(tmp.data_ptr<float>(), ld, in.data_ptr<float>(), std::max(in.stride(0), k),
-                                   w.data_ptr<float>(), d, 1, degrees.data_ptr<float>(), nullptr, 0, i > 0 ? 1 : 0,
-                                   static_cast<int>(n), static_cast<int>(k), static_cast<int>(d),
-                                   static_cast<int>(ld - d), stream),
-                "eppgcn_update_rows");
+      update_rows(tmp.data_ptr<float>(), ld, in, std::max(in.stride(0), k), w.data_ptr<float>(), d, 1,
+                  degrees.data_ptr<float>(), nullptr, 0, i > 0, n, k, d, ld - d, buffers, stream);
     }
     auto out = buffers.rows(n, ld_out, x).narrow(1, 0, d);
     ScopedMark t(1, 0, 0, clock_stream);
@@ -615,10 +624,8 @@ void run_backward(torch::Tensor grad, const torch::Tensor &x, const std::vector<
         epp_check(eppgcn_zero_rows(next.data_ptr<float>(), ldi, static_cast<int>(ldi), zeros.data_ptr<int>(), count, stream),
                   "eppgcn_zero_rows");
     } else {
-      epp_check(eppgcn_update_rows(next.data_ptr<float>(), ldi, d_prime.data_ptr<float>(), ld, weights[i].data_ptr<float>(),
-                                   1, d, degrees.data_ptr<float>(), gate, acts[i - 1].stride(0), 0, static_cast<int>(n),
-                                   static_cast<int>(d), static_cast<int>(din), static_cast<int>(ldi - din), stream),
-                "eppgcn_update_rows");
+      update_rows(next.data_ptr<float>(), ldi, d_prime, ld, weights[i].data_ptr<float>(), 1, d, degrees.data_ptr<float>(), gate,
+                  acts[i - 1].stride(0), false, n, d, din, ldi - din, buffers, stream);
     }
     grad = next;
   }

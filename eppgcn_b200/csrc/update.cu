@@ -10,6 +10,8 @@
 //
 // Both kernels run on the tensor cores with operands split into bf16 pieces that together hold every bit of an fp32
 // value: one for many rows, one for few or long rows that splits k over warps.
+#include <type_traits>
+
 #include "mma_split.cuh"
 
 namespace epp {
@@ -27,6 +29,8 @@ struct UpdateArgs {
   const int *rows;                     // the rows of x and out that are meant, or NULL: rows 0 .. n - 1
   int n, k, dout, owned_cols;          // columns dout .. owned_cols - 1 receive zeros
   int parts;                           // stretches that k is cut into
+  float *scratch;                      // [part][row][scratch_cols] their sums, where there are several
+  int scratch_cols;
   bool relu_x;
   bool x_vec, out_vec;                 // 16-byte pieces possible
   bool whole_cols, gate_vec;           // the same over all columns rounded up to a multiple of 8
@@ -258,24 +262,49 @@ __global__ void __launch_bounds__(kMmaWarps * 32, ManyRowsShape<NT>::RESIDENT) u
 
 // ---------------------------------------------------------------------------
 // Few rows, or rows too long for W to be kept: a block of 8 warps takes a tile of 8 x 16 M rows and a stretch of k, whose
-// part of W it splits into shared memory once for all of its rows; x comes through a ring per warp (cp.async: rows that
-// 16 bytes do not divide are copied word by word, still coalesced and several steps ahead).  k is cut into as many
-// stretches as fill whole waves of the chip; with more than one the scaled sums are added to the cleared result.
-// Bound by latency and by the split's instructions.
+// part of W it splits into shared memory for all of its rows, piece by piece where the stretch does not fit; x comes
+// through a ring per warp (cp.async: rows that 16 bytes do not divide are copied word by word, still coalesced and
+// several steps ahead).  k is cut into as many stretches as fill whole waves of the chip, each with a place of its own in
+// the caller's scratch buffer; add_parts_kernel adds them in the order of k, so that a result has the same bits on every
+// run.  Bound by latency and by the split's instructions.
 // ---------------------------------------------------------------------------
+constexpr int few_rows_resident(int nt) { return nt <= 3 ? 2 : 1; }          // blocks per SM
+constexpr int few_rows_ring(int m) { return (m == 1 ? 6 : 4) * 256 * m; }    // floats of x in flight per warp
+// Steps whose part of W fits beside the rings; a longer stretch takes it in pieces, which every warp has to wait for.
+constexpr int few_rows_most_steps(int nt, int m) {
+  return (113 * 1024 * (few_rows_resident(nt) == 1 ? 2 : 1) - 4 * kMmaWarps * few_rows_ring(m)) / (nt * 768);
+}
 template <int NT, int M>
 struct FewRowsShape {
   static constexpr int STAGES = M == 1 ? 6 : 4;        // steps of x in flight
   static constexpr int STAGE = 256 * M;                // floats
-  static constexpr int RING = STAGES * STAGE;
+  static constexpr int RING = few_rows_ring(M);
   static constexpr int ES = 8 * NT + (NT == 8 && M == 2 ? 0 : 4);
-  static constexpr int RESIDENT = NT <= 3 ? 2 : 1;     // blocks per SM
-  static_assert(16 * M * ES <= RING, "the sums of a warp take the place of its ring");
-  static constexpr int MOST_STEPS = (113 * 1024 * (RESIDENT == 1 ? 2 : 1) - 4 * kMmaWarps * RING) / (NT * 768);
+  static_assert(16 * M * ES <= RING && RING == STAGES * STAGE, "the sums of a warp take the place of its ring");
+  static constexpr int MOST_STEPS = few_rows_most_steps(NT, M);
 };
 
+// Scale, gate and store P neighbouring columns of a result, c .. c + P - 1 of `row`.
+template <int P>
+__device__ __forceinline__ void finish_piece(const UpdateArgs &a, long long row, int c, float (&o)[P]) {
+  const float scale = a.scale ? __ldg(a.scale + row) : 1.f;
+#pragma unroll
+  for (int q = 0; q < P; ++q) {
+    o[q] = c + q < a.dout ? o[q] * scale : 0.f;
+    if (a.gate && c + q < a.dout && __ldg(a.gate + row * a.ld_gate + c + q) <= 0.f) o[q] = 0.f;
+  }
+  float *const dst = a.out + row * a.ld_out + c;
+  if (P == 4 && c + P <= a.owned_cols) {
+    *reinterpret_cast<float4 *>(dst) = make_float4(o[0], o[1], o[2], o[3]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < P; ++q)
+      if (c + q < a.owned_cols) dst[q] = o[q];
+  }
+}
+
 template <int NT, int M>
-__global__ void __launch_bounds__(kMmaWarps * 32, NT <= 3 ? 2 : 1) update_few_rows_kernel(const UpdateArgs all) {
+__global__ void __launch_bounds__(kMmaWarps * 32, few_rows_resident(NT)) update_few_rows_kernel(const UpdateArgs all) {
   const UpdateArgs a = column_block(all, blockIdx.z * 8 * NT, 8 * NT);
   using Shape = FewRowsShape<NT, M>;
   constexpr int S = Shape::STAGES, ES = Shape::ES, QUADS = 2 * NT, ROWS = 16 * M;
@@ -325,21 +354,6 @@ __global__ void __launch_bounds__(kMmaWarps * 32, NT <= 3 ? 2 : 1) update_few_ro
 #pragma unroll
   for (int u = 0; u < S - 1; ++u) stage();
 
-#pragma unroll 4
-  for (int e = threadIdx.x; e < count * NT * 32; e += kMmaWarps * 32) {
-    const int el = e % 32, j = e / 32 % NT, s = e / 32 / NT, c = w_column<NT>(j, el >> 2);
-    float v[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int kk = 16 * (begin + s) + 4 * (el & 3) + q;
-      v[q] = kk < a.k && c < a.dout ? __ldg(a.w + kk * a.w_row + c * a.w_col) : 0.f;
-    }
-    uint2 *const at = few_w + (s * NT + j) * 96 + el;
-    split3(v[0], v[1], at[0].x, at[32].x, at[64].x);
-    split3(v[2], v[3], at[0].y, at[32].y, at[64].y);
-  }
-  __syncthreads();
-
   float top[NT][M][4], rest[NT][M][4];
 #pragma unroll
   for (int j = 0; j < NT; ++j)
@@ -349,7 +363,27 @@ __global__ void __launch_bounds__(kMmaWarps * 32, NT <= 3 ? 2 : 1) update_few_ro
       for (int q = 0; q < 4; ++q) top[j][m][q] = rest[j][m][q] = 0.f;
   const uint2 *wf = few_w + lane;
   int slot = 0;
-  for (int s = 0; s < count; ++s, wf += NT * 96) {
+  for (int s = 0, piece_end = 0; s < count; ++s, wf += NT * 96) {
+    if (s == piece_end) {              // the next piece of W
+      if (s) __syncthreads();          // every warp is done with the one before
+      const int have = min(Shape::MOST_STEPS, count - s);
+#pragma unroll 4
+      for (int e = threadIdx.x; e < have * NT * 32; e += kMmaWarps * 32) {
+        const int el = e % 32, j = e / 32 % NT, u = e / 32 / NT, c = w_column<NT>(j, el >> 2);
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int kk = 16 * (begin + s + u) + 4 * (el & 3) + q;
+          v[q] = kk < a.k && c < a.dout ? __ldg(a.w + kk * a.w_row + c * a.w_col) : 0.f;
+        }
+        uint2 *const at = few_w + (u * NT + j) * 96 + el;
+        split3(v[0], v[1], at[0].x, at[32].x, at[64].x);
+        split3(v[2], v[3], at[0].y, at[32].y, at[64].y);
+      }
+      __syncthreads();
+      wf = few_w + lane;
+      piece_end = s + have;
+    }
     stage();
     cp_wait<S - 1>();
     __syncwarp();
@@ -391,76 +425,127 @@ __global__ void __launch_bounds__(kMmaWarps * 32, NT <= 3 ? 2 : 1) update_few_ro
                                  min(16 * (begin + count), a.k), a.relu_x);
   }
   __syncwarp();
-  if (a.out_vec) {
+  if (a.parts > 1) {
+    float *const dst = a.scratch + (static_cast<long long>(blockIdx.y) * a.n + row0) * a.scratch_cols + blockIdx.z * 8 * NT;
+    for (int e = lane; e < rows * QUADS; e += 32)
+      *reinterpret_cast<float4 *>(dst + static_cast<long long>(e / QUADS) * a.scratch_cols + e % QUADS * 4) =
+          *reinterpret_cast<const float4 *>(ring + e / QUADS * ES + e % QUADS * 4);
+  } else if (a.out_vec) {
     for (int e = lane; e < rows * QUADS; e += 32) {
       const int r = e / QUADS, c = (e % QUADS) * 4;
-      if (c >= a.owned_cols) continue;
-      const long long row = row0 + r;
       const float4 v = *reinterpret_cast<const float4 *>(ring + r * ES + c);
       float o[4] = {v.x, v.y, v.z, v.w};
-      const float s = a.scale ? __ldg(a.scale + row) : 1.f;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        o[q] = c + q < a.dout ? o[q] * s : 0.f;
-        if (a.gate && c + q < a.dout && __ldg(a.gate + row * a.ld_gate + c + q) <= 0.f) o[q] = 0.f;
-      }
-      float *dst = a.out + row * a.ld_out + c;
-      if (c + 4 <= a.owned_cols) {
-        if (a.parts > 1) atomicAdd(reinterpret_cast<float4 *>(dst), make_float4(o[0], o[1], o[2], o[3]));
-        else *reinterpret_cast<float4 *>(dst) = make_float4(o[0], o[1], o[2], o[3]);
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (c + q < a.owned_cols) {
-            if (a.parts > 1) atomicAdd(dst + q, o[q]);
-            else dst[q] = o[q];
-          }
-      }
+      if (c < a.owned_cols) finish_piece(a, row0 + r, c, o);
     }
   } else {
     for (int e = lane; e < rows * 8 * NT; e += 32) {       // word by word, neighbouring lanes on neighbouring words
-      const int r = e / (8 * NT), c = e % (8 * NT);
-      if (c >= a.owned_cols) continue;
-      const long long row = row0 + r;
-      float o = c < a.dout ? ring[r * ES + c] * (a.scale ? __ldg(a.scale + row) : 1.f) : 0.f;
-      if (a.gate && c < a.dout && __ldg(a.gate + row * a.ld_gate + c) <= 0.f) o = 0.f;
-      float *dst = a.out + row * a.ld_out + c;
-      if (a.parts > 1) atomicAdd(dst, o);
-      else *dst = o;
+      float o[1] = {ring[e / (8 * NT) * ES + e % (8 * NT)]};
+      if (e % (8 * NT) < a.owned_cols) finish_piece(a, row0 + e / (8 * NT), e % (8 * NT), o);
     }
   }
   if (threadIdx.x == 0) clock_end(a.mark);
 }
 
-template <int NT, int M>
-int launch_few_rows(UpdateArgs &a, int col_blocks, int sms, cudaStream_t s) {
-  using Shape = FewRowsShape<NT, M>;
-  static_assert(Shape::MOST_STEPS >= 8, "a useful stretch of W fits");
-  // the number of stretches of k that takes the fewest steps over all waves; a block's start and end cost about as
-  // much as four steps, and one more when its sums have to be added
-  const long long tiles = ceil_div_ll(a.n, 16 * M * kMmaWarps), slots = static_cast<long long>(sms) * Shape::RESIDENT;
-  const int steps = (a.k + 15) / 16;
+// The sums of the stretches, added in the order of k: a thread per P columns of a row, 16 loads in flight.  Launched
+// before the kernel that writes them has ended (0.6 us less between the two) and waits for it here.
+template <int P>
+__global__ void __launch_bounds__(128) add_parts_kernel(const UpdateArgs a) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  using Piece = std::conditional_t<P == 4, float4, float>;
+  const int width = (a.owned_cols + P - 1) / P;
+  const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (e < a.n * static_cast<long long>(width)) {
+    const long long row = e / width, hop = static_cast<long long>(a.n) * a.scratch_cols;
+    const int c = static_cast<int>(e % width) * P;
+    const float *from = a.scratch + row * a.scratch_cols + c;
+    alignas(16) float o[P] = {}, v[16][P];
+    for (int p = 0; p < a.parts; p += 16, from += 16 * hop) {
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        if (p + u < a.parts) *reinterpret_cast<Piece *>(v[u]) = *reinterpret_cast<const Piece *>(from + u * hop);
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+#pragma unroll
+        for (int q = 0; q < P; ++q)
+          if (p + u < a.parts) o[q] = p + u ? o[q] + v[u][q] : v[u][q];
+    }
+    finish_piece(a, row, c, o);
+  }
+  if (threadIdx.x == 0) clock_end(a.mark);
+}
+
+// Stretches of k for `tiles` tiles and `slots` resident blocks: the number that takes the fewest steps over all waves.  A
+// block's start and end cost about as much as four steps; with several stretches, adding them costs one, one more for
+// every 8, and one for every 2 MB that their sums are written and read (fitted to sweeps over 24 shapes; a step of a wave
+// takes 0.6 us).
+// No stretch longer than `most_steps`, whose part of W is split once (20000 x 3703 -> 16: 102 us in 11 stretches, 172 in 10).
+int choose_parts(long long tiles, int steps, int most_steps, long long slots, long long result_bytes) {
   long long best = -1;
-  for (int p = (steps + Shape::MOST_STEPS - 1) / Shape::MOST_STEPS; p <= steps && p <= 128; ++p) {
-    const long long cost = ceil_div_ll(tiles * p * col_blocks, slots) * (ceil_div_ll(steps, p) + 4 + (p > 1));
+  const int fewest = (steps + most_steps - 1) / most_steps;
+  int parts = fewest;                                  // rows of more than 128 stretches
+  for (int p = fewest; p <= steps && p <= 128; ++p) {
+    const long long cost = ceil_div_ll(tiles * p, slots) * (ceil_div_ll(steps, p) + 4) +
+                           (p > 1 ? 1 + p / 8 + p * result_bytes / 1000000 : 0);
     if (best < 0 || cost < best) {
       best = cost;
-      a.parts = p;
+      parts = p;
     }
   }
-  if (best < 0) a.parts = (steps + Shape::MOST_STEPS - 1) / Shape::MOST_STEPS;     // rows of more than 128 stretches
-  const int longest = static_cast<int>(ceil_div_ll(steps, a.parts));
-  const int smem = 4 * kMmaWarps * Shape::RING + longest * NT * 768;
+  return parts;
+}
+
+// How a product is run: blocks of 8 * nt output columns; by the many-row kernel or, with m 16-row tiles per warp and k in
+// `parts` stretches, by the other.
+struct UpdateShape {
+  int nt, col_blocks, m, parts;
+  bool many_rows;
+  long long row_floats() const { return 8LL * nt * col_blocks; }
+};
+
+UpdateShape update_shape(int n, int k, int dout, bool listed, int sms) {
+  UpdateShape u{};
+  // blocks of at most 64 columns, about equally wide
+  const int blocks = (dout + 63) / 64;
+  u.nt = ((dout + blocks - 1) / blocks + 7) / 8;
+  u.col_blocks = (dout + 8 * u.nt - 1) / (8 * u.nt);
+  // From one tile of 32 rows per resident warp on, the many-row kernel keeps the chip busy; results of more than four
+  // blocks go through the other, which does not hold W's fragments for every block.
+  u.many_rows = listed || (k <= kMmaMaxK && n >= 32 * kMmaWarps * sms && u.col_blocks <= 4);
+  // 32 rows per warp share W's fragments and give twice the independent products, where there are enough of them
+  u.m = n >= 8192 ? 2 : 1;
+  u.parts = u.many_rows ? 1 : choose_parts(ceil_div_ll(n, 16 * u.m * kMmaWarps) * u.col_blocks, (k + 15) / 16,
+                                           few_rows_most_steps(u.nt, u.m), static_cast<long long>(sms) * few_rows_resident(u.nt),
+                                           4LL * n * u.row_floats());
+  return u;
+}
+
+template <int NT, int M>
+int launch_few_rows(const UpdateArgs &a, int col_blocks, cudaStream_t s) {
+  using Shape = FewRowsShape<NT, M>;
+  static_assert(Shape::MOST_STEPS >= 8, "a useful piece of W fits");
+  const int stretch = static_cast<int>(ceil_div_ll((a.k + 15) / 16, a.parts));
+  const int smem = 4 * kMmaWarps * Shape::RING + (stretch < Shape::MOST_STEPS ? stretch : Shape::MOST_STEPS) * NT * 768;
   static SmemOptIn memo;
   const void *kernel = reinterpret_cast<const void *>(update_few_rows_kernel<NT, M>);
   if (const int rc = smem_opt_in(memo, kernel, 4 * kMmaWarps * Shape::RING + Shape::MOST_STEPS * NT * 768); rc != EPP_OK)
     return rc;
-  if (a.parts > 1) {
-    const int rc = zero_column_block(a.out, a.ld_out, a.owned_cols, a.n, s);
-    if (rc != EPP_OK) return rc;
-  }
+  const long long tiles = ceil_div_ll(a.n, 16 * M * kMmaWarps);
   update_few_rows_kernel<NT, M><<<dim3(static_cast<unsigned>(tiles), a.parts, col_blocks), kMmaWarps * 32, smem, s>>>(a);
   EPP_CHECK_LAUNCH("update_few_rows_kernel");
+  if (a.parts == 1) return EPP_OK;
+  UpdateArgs sum = a;
+  sum.mark = take_mark();
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t launch{};
+  launch.gridDim = dim3(static_cast<unsigned>(ceil_div_ll(a.n * ceil_div_ll(a.owned_cols, a.out_vec ? 4 : 1), 128)));
+  launch.blockDim = dim3(128);
+  launch.stream = s;
+  launch.attrs = &early;
+  launch.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&launch, a.out_vec ? add_parts_kernel<4> : add_parts_kernel<1>, static_cast<const UpdateArgs>(sum));
+  EPP_CHECK_LAUNCH("add_parts_kernel");
   return EPP_OK;
 }
 
@@ -479,15 +564,11 @@ int launch_many_rows(const UpdateArgs &a, int col_blocks, int sms, cudaStream_t 
   return EPP_OK;
 }
 
-// Blocks of 8 * NT output columns.  From one tile of 32 rows per resident warp on, the many-row kernel keeps the chip
-// busy; results of more than four blocks go through the other, which does not hold W's fragments for every block.
 template <int NT>
-int update_block(UpdateArgs &a, int col_blocks, int sms, cudaStream_t s) {
-  if (a.rows) return launch_many_rows<NT, true>(a, col_blocks, sms, s);
-  if (a.k <= kMmaMaxK && a.n >= 32 * kMmaWarps * sms && col_blocks <= 4)
-    return launch_many_rows<NT, false>(a, col_blocks, sms, s);
-  // 32 rows per warp share W's fragments and give twice the independent products, where there are enough of them
-  return a.n >= 8192 ? launch_few_rows<NT, 2>(a, col_blocks, sms, s) : launch_few_rows<NT, 1>(a, col_blocks, sms, s);
+int update_block(const UpdateArgs &a, const UpdateShape &u, int sms, cudaStream_t s) {
+  if (a.rows) return launch_many_rows<NT, true>(a, u.col_blocks, sms, s);
+  if (u.many_rows) return launch_many_rows<NT, false>(a, u.col_blocks, sms, s);
+  return u.m == 2 ? launch_few_rows<NT, 2>(a, u.col_blocks, s) : launch_few_rows<NT, 1>(a, u.col_blocks, s);
 }
 
 }  // namespace
@@ -495,7 +576,8 @@ int update_block(UpdateArgs &a, int col_blocks, int sms, cudaStream_t s) {
 
 static int update_impl(float *out, long long ld_out, const float *x, long long ldx, const float *w, long long w_row,
                        long long w_col, const float *scale, const float *gate, long long ld_gate, int relu_x,
-                       const int *rows, int num_rows, int k, int dout, int pad_cols, void *stream) {
+                       const int *rows, int num_rows, int k, int dout, int pad_cols, void *scratch, size_t scratch_bytes,
+                       void *stream) {
   using namespace epp;
   EPP_REQUIRE(num_rows >= 0 && k >= 1 && dout >= 1, "negative size, k < 1 or dout < 1");
   if (num_rows == 0) return EPP_OK;
@@ -507,9 +589,9 @@ static int update_impl(float *out, long long ld_out, const float *x, long long l
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int sms = 148;
   if (const int rc = device_sm_count(&sms); rc != EPP_OK) return rc;
-  // blocks of at most 64 columns, about equally wide
-  const int blocks = (dout + 63) / 64, width = ((dout + blocks - 1) / blocks + 7) / 8 * 8;
-  EPP_REQUIRE(blocks <= 65535, "more than 4 194 240 columns");
+  EPP_REQUIRE(dout <= 4194240, "more than 4 194 240 columns");
+  EPP_REQUIRE(!scratch || aligned(scratch, 16), "scratch must be 16-byte aligned");
+  const UpdateShape u = update_shape(num_rows, k, dout, rows != nullptr, sms);
   UpdateArgs a{};
   a.out = out; a.ld_out = ld_out; a.x = x; a.ldx = ldx;
   a.w = w; a.w_row = w_row; a.w_col = w_col;
@@ -523,22 +605,44 @@ static int update_impl(float *out, long long ld_out, const float *x, long long l
   a.out_vec = ld_out % 4 == 0 && aligned(out, 16);
   a.whole_cols = a.out_vec && a.owned_cols == round8;
   a.gate_vec = gate && ld_gate % 4 == 0 && ld_gate >= round8 && aligned(gate, 16);
+  // as many stretches as there is room for
+  const size_t part_bytes = sizeof(float) * static_cast<size_t>(num_rows) * u.row_floats();
+  a.parts = u.parts;
+  if (!scratch || scratch_bytes < part_bytes * a.parts) a.parts = scratch ? static_cast<int>(scratch_bytes / part_bytes) : 1;
+  if (a.parts < 1) a.parts = 1;
+  a.scratch = static_cast<float *>(scratch);
+  a.scratch_cols = static_cast<int>(u.row_floats());
   a.mark = take_mark();
-  const int used = (dout + width - 1) / width;
   int rc;
-  switch (width / 8) {
-    case 1:  rc = update_block<1>(a, used, sms, s); break;
-    case 2:  rc = update_block<2>(a, used, sms, s); break;
-    case 3:  rc = update_block<3>(a, used, sms, s); break;
-    case 4:  rc = update_block<4>(a, used, sms, s); break;
-    case 5:  rc = update_block<5>(a, used, sms, s); break;
-    case 6:  rc = update_block<6>(a, used, sms, s); break;
-    case 7:  rc = update_block<7>(a, used, sms, s); break;
-    default: rc = update_block<8>(a, used, sms, s); break;
+  switch (u.nt) {
+    case 1:  rc = update_block<1>(a, u, sms, s); break;
+    case 2:  rc = update_block<2>(a, u, sms, s); break;
+    case 3:  rc = update_block<3>(a, u, sms, s); break;
+    case 4:  rc = update_block<4>(a, u, sms, s); break;
+    case 5:  rc = update_block<5>(a, u, sms, s); break;
+    case 6:  rc = update_block<6>(a, u, sms, s); break;
+    case 7:  rc = update_block<7>(a, u, sms, s); break;
+    default: rc = update_block<8>(a, u, sms, s); break;
   }
   if (rc == EPP_OK && !rows && a.owned_cols < dout + pad_cols)
     rc = zero_column_block(out + a.owned_cols, ld_out, dout + pad_cols - a.owned_cols, num_rows, s);
   return rc;
+}
+
+EPP_EXPORT size_t eppgcn_update_scratch_bytes(int num_rows, int k, int dout) {
+  using namespace epp;
+  int sms = 148;
+  if (num_rows < 1 || k < 1 || dout < 1 || device_sm_count(&sms) != EPP_OK) return 0;
+  const UpdateShape u = update_shape(num_rows, k, dout, false, sms);
+  return u.parts > 1 ? sizeof(float) * static_cast<size_t>(num_rows) * u.row_floats() * u.parts : 0;
+}
+
+EPP_EXPORT int eppgcn_update_rows_scratch(float *out, long long ld_out, const float *x, long long ldx, const float *w,
+                                          long long w_row, long long w_col, const float *scale, const float *gate,
+                                          long long ld_gate, int relu_x, int num_rows, int k, int dout, int pad_cols,
+                                          void *scratch, size_t scratch_bytes, void *stream) {
+  return update_impl(out, ld_out, x, ldx, w, w_row, w_col, scale, gate, ld_gate, relu_x, nullptr, num_rows, k, dout, pad_cols,
+                     scratch, scratch_bytes, stream);
 }
 
 EPP_EXPORT int eppgcn_update_rows(float *out, long long ld_out, const float *x, long long ldx, const float *w,
@@ -546,7 +650,7 @@ EPP_EXPORT int eppgcn_update_rows(float *out, long long ld_out, const float *x, 
                                   long long ld_gate, int relu_x, int num_rows, int k, int dout, int pad_cols,
                                   void *stream) {
   return update_impl(out, ld_out, x, ldx, w, w_row, w_col, scale, gate, ld_gate, relu_x, nullptr, num_rows, k, dout, pad_cols,
-                     stream);
+                     nullptr, 0, stream);
 }
 
 EPP_EXPORT int eppgcn_update_listed(float *out, long long ld_out, const float *x, long long ldx, const float *w,
@@ -557,7 +661,7 @@ EPP_EXPORT int eppgcn_update_listed(float *out, long long ld_out, const float *x
   EPP_REQUIRE(rows || num_listed == 0, "null row list");
   EPP_REQUIRE(k <= 256 && pad_cols < 8, "listed rows have at most 256 columns and 7 of padding");
   return update_impl(out, ld_out, x, ldx, w, w_row, w_col, scale, gate, ld_gate, relu_x, rows, num_listed, k, dout, pad_cols,
-                     stream);
+                     nullptr, 0, stream);
 }
 
 EPP_EXPORT int eppgcn_update_scaled(float *out, long long ld_out, const float *x, long long ldx, const float *w,

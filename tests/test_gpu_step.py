@@ -249,3 +249,19 @@ def test_to_device(cuda, n):
     for t in (torch.arange(n, dtype=torch.int32), torch.arange(2 * n, dtype=torch.int32)[::2]):
         got = gnna.to_device(t, 0)
         assert got.is_cuda and got.dtype == t.dtype and torch.equal(got.cpu(), t)
+
+
+@pytest.mark.parametrize("n,k,dout,ld", [(3327, 3703, 16, 16), (2708, 1433, 7, 7), (19717, 500, 3, 8), (1, 40_000, 8, 8),
+                                         (130, 20_000, 64, 67), (257, 9000, 33, 40), (9001, 700, 22, 24), (500, 300, 130, 132)])
+def test_long_rows_repeat_bit_by_bit(cuda, n, k, dout, ld):
+    """k cut into stretches (and stretches into pieces of W): the same bits on every run, within float64's bound, gate, scale
+    and padding included, for rows of any alignment."""
+    gen = torch.Generator(device=cuda).manual_seed(k)
+    x, w = torch.randn(n, k, device=cuda, generator=gen), torch.randn(k, dout, device=cuda, generator=gen)
+    scale, gate = torch.rand(n, device=cuda, generator=gen) + 0.5, torch.randn(n, dout, device=cuda, generator=gen)
+    want, mag = x.double() @ w.double() * scale.double()[:, None], x.double().abs() @ w.double().abs() * scale.double()[:, None]
+    runs = [capi.update_rows(x, w, scale, gate, out=torch.full((n, ld), 7.0, device=cuda)[:, :dout]) for _ in range(12)]
+    assert ((runs[0].double() - want * (gate > 0)).abs() <= 1e-6 + 2e-6 * mag).all()
+    assert all(torch.equal(runs[0], r) for r in runs[1:])
+    alone = capi.update_rows(x, w, scale, gate, use_scratch=False)          # no buffer: one stretch, W in pieces
+    assert ((alone.double() - want * (gate > 0)).abs() <= 1e-6 + 2e-6 * mag).all()

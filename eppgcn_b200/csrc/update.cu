@@ -51,13 +51,6 @@ __device__ __forceinline__ UpdateArgs column_block(const UpdateArgs &all, int c0
   return a;
 }
 
-// The sum over k0 <= k < k1 by FMA: what a result that came out as NaN is replaced by.
-__device__ __noinline__ float fma_dot(const float *x, const float *w, long long w_row, int k0, int k1, bool relu) {
-  float sum = 0.f;
-  for (int k = k0; k < k1; ++k) sum = fmaf(relu ? max_nan(x[k], 0.f) : x[k], w[k * w_row], sum);
-  return sum;
-}
-
 // Column of W that column `n` of n tile j stands for: two neighbouring n tiles share 16 columns such that a lane of the
 // result holds four in a row; a last, single tile keeps its order.
 template <int NT>
@@ -75,6 +68,55 @@ __device__ __forceinline__ float4 load4(const float *p, int k, int k_end, bool v
   if (k + 3 < k_end) v.w = __ldg(p + 3);
   return v;
 }
+
+// Eight columns of 32 rows by FMA, a row per lane: what results that came out as NaN are replaced by.  x: this lane's row,
+// `wanted` where it has such a result; sums over k0 <= k < k1, k0 a multiple of 4.  Ends as soon as all wanted sums are NaN:
+// a run that has diverged pays for the first 4 k.
+__device__ __forceinline__ void columns_by_fma(float (&sum)[8], const float *x, bool x_vec, const float *w, long long w_row,
+                                               long long w_col, int cols, int k0, int k1, bool relu, bool wanted) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) sum[q] = 0.f;
+  bool open = wanted;
+#pragma unroll 1
+  for (int k = k0, n = 4; k < k1 && __any_sync(kFull, open); k += n, n = 16) {
+    const int end = min(k1, k + n);
+    float v[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float4 t = open ? load4(x + k + 4 * i, k + 4 * i, end, x_vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (relu) t = relu4(t);
+      v[i][0] = t.x; v[i][1] = t.y; v[i][2] = t.z; v[i][3] = t.w;
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (k + u < end && q < cols) sum[q] = fmaf(v[u / 4][u % 4], __ldg(w + (k + u) * w_row + q * w_col), sum[q]);
+    bool number = false;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) number |= q < cols && !isnan(sum[q]);
+    open = wanted && number;
+  }
+}
+
+// Whether W is NaN throughout, as after a step of a run that has diverged: then every result is, and none is to be replaced.
+// For a whole warp.
+__device__ __forceinline__ bool all_nan(const float *w, long long w_row, long long w_col, int k, int cols) {
+  bool nan = true;
+  for (int e = 0; e < k * cols && __all_sync(kFull, nan); e += 4 * kWarp)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int at = e + u * kWarp + (threadIdx.x & 31);
+      if (at < k * cols) nan &= isnan(__ldg(w + at / cols * w_row + at % cols * w_col));
+    }
+  return __all_sync(kFull, nan);
+}
+
+// ---------------------------------------------------------------------------
+// Results that came out as NaN are formed again by FMA behind the hot loop, in us (2 M x 128 -> 16; a lane that walked k
+// for every such result took 3.1 ms wherever a row or a column had one): none 226, W all NaN 243, x all NaN 615, one
+// infinity in x 400, one in W (a column of results) 2000.
+// ---------------------------------------------------------------------------
 
 // ---------------------------------------------------------------------------
 // Many rows: persistent warps over tiles of 32 rows.  W's fragments are split once per block and stay in shared
@@ -244,18 +286,37 @@ __global__ void __launch_bounds__(kMmaWarps * 32, ManyRowsShape<NT>::RESIDENT) u
   if (__any_sync(kFull, nan_seen)) {                   // this warp's tiles once more; a closed gate has made its zeros already
     __syncwarp();
     const int c0 = blockIdx.y * 8 * NT, cols = min(8 * NT, a.dout - c0);
+    int redo = all_nan(a.w + c0 * a.w_col, a.w_row, a.w_col, a.k, cols) ? tiles : first;
 #pragma unroll 1
-    for (int redo = first; redo < tiles; redo += stride)
-#pragma unroll 1
-      for (int e = lane; e < 32 * cols; e += 32) {
-        long long row = static_cast<long long>(redo) * 32 + e / cols;
-        if (row >= a.n) break;
-        if (LIST) row = a.rows[row];
-        const int c = c0 + e % cols;
-        float *at = a.out + row * a.ld_out + c;
-        if (isnan(*at))
-          *at = fma_dot(a.x + row * a.ldx, a.w + c * a.w_col, a.w_row, 0, a.k, a.relu_x) * (a.scale ? a.scale[row] : 1.f);
+    for (; redo < tiles; redo += stride) {
+      const int row0 = redo * 32, rows = min(32, a.n - row0);
+      unsigned bad = 0, bad_cols = 0;                  // rows; eighths of the columns
+#pragma unroll 4
+      for (int e = lane; e < rows * cols; e += 32) {
+        const long long row = LIST ? a.rows[row0 + e / cols] : row0 + e / cols;
+        if (!isnan(a.out[row * a.ld_out + c0 + e % cols])) continue;
+        bad |= 1u << (e / cols);
+        bad_cols |= 1u << (e % cols / 8);
       }
+      bad = __reduce_or_sync(kFull, bad);
+      bad_cols = __reduce_or_sync(kFull, bad_cols);
+      if (!bad) continue;
+      const bool wanted = bad >> lane & 1;
+      const long long row = !wanted ? 0 : LIST ? a.rows[row0 + lane] : row0 + lane;
+#pragma unroll 1
+      for (int c = 0; c < cols; c += 8) {
+        if (!(bad_cols >> (c / 8) & 1)) continue;
+        float sum[8];
+        columns_by_fma(sum, a.x + row * a.ldx, a.x_vec, a.w + (c0 + c) * a.w_col, a.w_row, a.w_col, cols - c, 0, a.k, a.relu_x,
+                       wanted);
+        if (!wanted) continue;
+        float *at = a.out + row * a.ld_out + c0 + c;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (c + q < cols && !isnan(sum[q]) && isnan(at[q])) at[q] = sum[q] * (a.scale ? a.scale[row] : 1.f);
+      }
+      __syncwarp();
+    }
   }
   if (threadIdx.x == 0) clock_end(a.mark);
 }
@@ -418,11 +479,28 @@ __global__ void __launch_bounds__(kMmaWarps * 32, few_rows_resident(NT)) update_
         for (int q = 0; q < 2; ++q)
           ring[(16 * m + 8 * h + g) * ES + w_column<NT>(j, 2 * t + q)] = top[j][m][2 * h + q] + rest[j][m][2 * h + q];
   __syncwarp();
+  unsigned bad = 0, bad_cols = 0;      // rows and eighths of the columns with a NaN: once more, over this stretch
   for (int e = lane; e < rows * 8 * NT; e += 32) {
     const int r = e / (8 * NT), c = e % (8 * NT);
-    if (c < a.dout && isnan(ring[r * ES + c]))
-      ring[r * ES + c] = fma_dot(a.x + (row0 + r) * a.ldx, a.w + c * a.w_col, a.w_row, 16 * begin,
-                                 min(16 * (begin + count), a.k), a.relu_x);
+    if (c >= a.dout || !isnan(ring[r * ES + c])) continue;
+    bad |= 1u << r;
+    bad_cols |= 1u << (c / 8);
+  }
+  bad = __reduce_or_sync(kFull, bad);
+  bad_cols = __reduce_or_sync(kFull, bad_cols);
+  if (bad) {
+    const bool wanted = bad >> lane & 1;
+    const float *const x = a.x + (wanted ? (row0 + lane) * a.ldx : 0);
+#pragma unroll 1
+    for (int c = 0; c < a.dout; c += 8) {
+      if (!(bad_cols >> (c / 8) & 1)) continue;
+      float sum[8];
+      columns_by_fma(sum, x, a.x_vec, a.w + c * a.w_col, a.w_row, a.w_col, a.dout - c, 16 * begin,
+                     min(16 * (begin + count), a.k), a.relu_x, wanted);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (wanted && c + q < a.dout && isnan(ring[lane * ES + c + q])) ring[lane * ES + c + q] = sum[q];
+    }
   }
   __syncwarp();
   if (a.parts > 1) {

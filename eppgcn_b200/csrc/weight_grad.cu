@@ -186,32 +186,82 @@ __global__ void __launch_bounds__(kWgWarps * 32, (WeightGradShape<NT, MI>::RESID
           *reinterpret_cast<float2 *>(ring + (32 * i + 4 * g + 2 * m + h) * (8 * NT) + 8 * j + 2 * t) =
               make_float2(top[j][i][m][2 * h] + rest[j][i][m][2 * h], top[j][i][m][2 * h + 1] + rest[j][i][m][2 * h + 1]);
   __syncthreads();
-  for (int e = threadIdx.x; e < k_have * QUADS; e += kWgWarps * 32) {
-    const int kk = e / QUADS, c = e % QUADS * 4;
-    if (c >= a.dout) continue;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  constexpr int PIECES = (32 * MI * QUADS + kWgWarps * 32 - 1) / (kWgWarps * 32);      // of four columns, per thread
+  float4 v[PIECES];
+  bool bad = false;
+  // has() of a piece: e = threadIdx.x + i * blockDim.x, element (e / QUADS, e % QUADS * 4) of the block's tile
+  auto has = [&](int e, int q) { return e < k_have * QUADS && e % QUADS * 4 + q < a.dout; };
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    const int e = threadIdx.x + i * kWgWarps * 32;
+    v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!has(e, 0)) continue;
     for (int w = 0; w < kWgWarps; ++w) {
-      const float4 o = *reinterpret_cast<const float4 *>(wg_smem + w * Shape::RING + kk * (8 * NT) + c);
-      v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+      const float4 o = *reinterpret_cast<const float4 *>(wg_smem + w * Shape::RING + e / QUADS * (8 * NT) + e % QUADS * 4);
+      v[i].x += o.x; v[i].y += o.y; v[i].z += o.z; v[i].w += o.w;
     }
-    if (isnan(v.x + v.y + v.z + v.w)) {                // an infinity among the operands: the block's rows once more, by FMA
-      v = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int step = static_cast<int>(blockIdx.x) * kWgWarps; step < all; step += stride)
-        for (long long at = 16LL * step; at < 16LL * step + 16 * kWgWarps && at < a.n; ++at) {
-          const long long id = a.rows ? a.rows[at] : at;
-          const float xk = a.relu_x ? max_nan(a.x[id * a.ldx + k0 + kk], 0.f) : a.x[id * a.ldx + k0 + kk];
-          const float *d = a.d + id * a.ldd + c;
-          v.x = fmaf(xk, d[0], v.x);
-          if (c + 1 < a.dout) v.y = fmaf(xk, d[1], v.y);
-          if (c + 2 < a.dout) v.z = fmaf(xk, d[2], v.z);
-          if (c + 3 < a.dout) v.w = fmaf(xk, d[3], v.w);
+    bad |= isnan(v[i].x) || (has(e, 1) && isnan(v[i].y)) || (has(e, 2) && isnan(v[i].z)) || (has(e, 3) && isnan(v[i].w));
+  }
+  if (__syncthreads_or(bad)) {
+    // An infinity or a NaN among the operands: the block's rows once more through the rings, by FMA, until every result that
+    // is to be replaced has become NaN here too or the rows end.  2 M x 128 -> 16: 254 us without a NaN, 264 where d' or x
+    // is NaN throughout, 690 with one infinity in x, 1030 with one in d' (a thread that walked all rows of its block for
+    // every four results: 6.8 to 7.1 ms).
+    float4 sum[PIECES];
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) sum[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    s_step = first;
+    s_slot = 0;
+    ids = load_ids(first);
+#pragma unroll 1
+    for (int u = 0; u < S - 1; ++u) stage();
+    const float *at = wg_smem;
+    for (int step = static_cast<int>(blockIdx.x) * kWgWarps; step < all; step += stride) {
+      stage();
+      cp_wait<S - 1>();
+      __syncthreads();
+      const int warps = min(kWgWarps, all - step);     // that have a step
+      bool open = false;
+#pragma unroll
+      for (int i = 0; i < PIECES; ++i) {
+        const int e = threadIdx.x + i * kWgWarps * 32;
+        if (!has(e, 0)) continue;
+        for (int w = 0; w < warps; ++w) {
+          const float *x_at = at + w * Shape::RING + e / QUADS, *d_at = at + w * Shape::RING + 16 * XS + e % QUADS * 4;
+#pragma unroll
+          for (int r = 0; r < 16; ++r) {
+            const float xk = a.relu_x ? max_nan(x_at[r * XS], 0.f) : x_at[r * XS];
+            const float4 d4 = *reinterpret_cast<const float4 *>(d_at + r * DS);
+            sum[i].x = fmaf(xk, d4.x, sum[i].x);
+            sum[i].y = fmaf(xk, d4.y, sum[i].y);
+            sum[i].z = fmaf(xk, d4.z, sum[i].z);
+            sum[i].w = fmaf(xk, d4.w, sum[i].w);
+          }
         }
+        open |= (isnan(v[i].x) && !isnan(sum[i].x)) || (has(e, 1) && isnan(v[i].y) && !isnan(sum[i].y)) ||
+                (has(e, 2) && isnan(v[i].z) && !isnan(sum[i].z)) || (has(e, 3) && isnan(v[i].w) && !isnan(sum[i].w));
+      }
+      if (!__syncthreads_or(open)) break;
+      at = at == wg_smem + (S - 1) * Shape::STAGE ? wg_smem : at + Shape::STAGE;
     }
-    float *dst = a.dw + (k0 + kk) * a.ld_dw + c;
+    cp_wait<0>();
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+      if (isnan(v[i].x)) v[i].x = sum[i].x;
+      if (isnan(v[i].y)) v[i].y = sum[i].y;
+      if (isnan(v[i].z)) v[i].z = sum[i].z;
+      if (isnan(v[i].w)) v[i].w = sum[i].w;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    const int e = threadIdx.x + i * kWgWarps * 32, c = e % QUADS * 4;
+    if (!has(e, 0)) continue;
+    float *dst = a.dw + (k0 + e / QUADS) * a.ld_dw + c;
     if (a.dw_vec && c + 4 <= a.dout) {
-      atomicAdd(reinterpret_cast<float4 *>(dst), v);
+      atomicAdd(reinterpret_cast<float4 *>(dst), v[i]);
     } else {
-      const float o[4] = {v.x, v.y, v.z, v.w};
+      const float o[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         if (c + q < a.dout) atomicAdd(dst + q, o[q]);

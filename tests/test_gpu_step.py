@@ -265,3 +265,60 @@ def test_long_rows_repeat_bit_by_bit(cuda, n, k, dout, ld):
     assert all(torch.equal(runs[0], r) for r in runs[1:])
     alone = capi.update_rows(x, w, scale, gate, use_scratch=False)          # no buffer: one stretch, W in pieces
     assert ((alone.double() - want * (gate > 0)).abs() <= 1e-6 + 2e-6 * mag).all()
+
+
+@pytest.mark.parametrize("n,k,dout", [(70, 40, 9), (40_000, 33, 22), (40_000, 130, 64), (300, 900, 16), (9000, 400, 70)])
+def test_infinities_and_nans_in_the_other_operand(cuda, n, k, dout):
+    """One column of W or of d' with an infinity, one with both, one with a NaN; ReLU, listed rows, and W all NaN."""
+    gen = torch.Generator(device=cuda).manual_seed(n + k)
+    x = torch.rand(n, k, device=cuda, generator=gen) + 0.5
+    x[n // 2] = -x[n // 2]
+    w, d = torch.rand(k, dout, device=cuda, generator=gen) + 0.5, torch.rand(n, dout, device=cuda, generator=gen) + 0.5
+    inf, nan = float("inf"), float("nan")
+    for m in (w, d):
+        last = m.size(0) - 1
+        m[last, 0], m[0, 3], m[last, 3], m[last // 2, dout - 1] = inf, inf, -inf, nan
+
+    def same(got, want, rtol):
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+        assert torch.allclose(got, want.float(), rtol=rtol, equal_nan=True)
+
+    for relu in (False, True):
+        xd = (x.clamp(min=0) if relu else x).double()
+        same(capi.update_rows(x, w, relu_x=relu), (xd @ w.double()).float(), 1e-5)
+        same(capi.weight_grad_add(torch.zeros(k, dout, device=cuda), x, d, relu_x=relu), (xd.T @ d.double()).float(), 1e-4)
+    if k <= 256:
+        rows = torch.arange(0, n, 3, device=cuda, dtype=torch.int32)
+        got = capi.update_rows(x, w, rows=rows, out=torch.zeros(n, dout, device=cuda))
+        same(got[::3], (x.double() @ w.double()).float()[::3], 1e-5)
+    assert capi.update_rows(x, torch.full_like(w, nan)).isnan().all()
+
+
+def test_a_diverged_run_costs_little_more(cuda):
+    """Where everything is NaN, or one feature infinite, the products keep to the order of their usual time."""
+    n, k, d = 1 << 19, 128, 16
+    x, w, g = (torch.randn(s, device=cuda) for s in ((n, k), (k, d), (n, d)))
+    out, dw = torch.empty(n, d, device=cuda), torch.zeros(k, d, device=cuda)
+    odd = x.clone()
+    odd[n // 3, 7] = float("inf")
+
+    def us(f):
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(4):
+                f()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b) * 250.0)
+        return sorted(times)[1]
+
+    plain_up, plain_dw = us(lambda: capi.update_rows(x, w, out=out)), us(lambda: capi.weight_grad_add(dw, x, g))
+    nan_w, nan_g, nan_x = (torch.full_like(m, float("nan")) for m in (w, g, x))
+    for f, plain, times in [(lambda: capi.update_rows(x, nan_w, out=out), plain_up, 2),
+                            (lambda: capi.update_rows(nan_x, w, out=out), plain_up, 6),
+                            (lambda: capi.update_rows(odd, w, out=out), plain_up, 6),
+                            (lambda: capi.weight_grad_add(dw, x, nan_g), plain_dw, 2),
+                            (lambda: capi.weight_grad_add(dw, odd, g), plain_dw, 8)]:
+        assert us(f) <= times * plain + 20.0

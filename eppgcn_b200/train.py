@@ -32,6 +32,11 @@ from .param import backInputProperty, inputProperty, maskInputProperty
 GNNA = load_gnnadvisor()
 
 
+def _replaced(obj, name, original):
+    """Whether ``obj``'s method is another than this module's: a subclass's, its own, or one put onto the class."""
+    return name in obj.__dict__ or getattr(type(obj), name) is not original
+
+
 class Net(torch.nn.Module):
     """``num_layers`` GCNConv layers, ReLU after all but the last
     (EPPGCN/gcn_main.py:183-208)."""
@@ -58,7 +63,7 @@ class Net(torch.nn.Module):
         weights = []
         for m in (self, *self.convs):
             if (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
-                    or "forward" in m.__dict__):
+                    or _replaced(m, "forward", _NET_FORWARD if m is self else _CONV_FORWARD)):
                 return None
             if m is not self:
                 w = m.weights
@@ -80,6 +85,9 @@ class Net(torch.nn.Module):
             if i < self.num_layers - 1:
                 x = F.relu(x)
         return x
+
+
+_NET_FORWARD, _CONV_FORWARD = Net.forward, GCNConv.forward
 
 
 class Adam(torch.optim.Adam):
@@ -224,8 +232,8 @@ class GCNTrainer:
     # EPPGCN/gcn_main.py:151-168
     def build_back_part(self):
         ds = self.ds
-        own_rule = type(self).choose_back_size is not GCNTrainer.choose_back_size or "choose_back_size" in self.__dict__
-        if (hasattr(GNNA, "compact_back_edges") and self.layers <= 16 and not own_rule
+        if (hasattr(GNNA, "compact_back_edges") and self.layers <= 16
+                and not _replaced(self, "choose_back_size", _CHOOSE_BACK_SIZE)
                 and self.backsize_mode in ("map", "bucket", "constant")):
             # all layers in one go: two synchronisations instead of three per layer
             ids, edges, valid, active = GNNA.compact_back_edges(ds.edge_masks, self.inputInfo.column_index, ds.node_degs)
@@ -259,7 +267,7 @@ class GCNTrainer:
         """The weights, when one epoch can run as three calls of the operator module (see ``Net.native_weights``):
         the gradients are wanted and nothing but the optimizer looks at them on their way."""
         ds = self.ds
-        if not (torch.is_grad_enabled() and hasattr(self.model, "native_weights")
+        if not (torch.is_grad_enabled() and type(self.model) is Net and not _replaced(self, "forward", _TRAINER_FORWARD)
                 and ds.y.dtype == torch.int64 and ds.y.is_cuda and ds.y.is_contiguous() and ds.y.dim() == 1
                 and ds.train_mask.dtype == torch.bool and ds.train_mask.is_cuda and ds.train_mask.is_contiguous()):
             return None
@@ -331,6 +339,9 @@ class GCNTrainer:
             self.back_time += time.perf_counter() - t0
         self.optimizer.step()
         return loss
+
+
+_TRAINER_FORWARD, _CHOOSE_BACK_SIZE = GCNTrainer.forward, GCNTrainer.choose_back_size
 
 
 def build_parser() -> argparse.ArgumentParser:

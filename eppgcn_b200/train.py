@@ -23,6 +23,9 @@ import time
 import torch
 import torch.nn.functional as F
 import torch.nn.modules.module as _hooks
+from torch.autograd import forward_ad
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from . import load_gnnadvisor
 from .gcn_conv import GCNConv
@@ -30,6 +33,20 @@ from .graphs import WORKLOADS, load_workload
 from .param import backInputProperty, inputProperty, maskInputProperty
 
 GNNA = load_gnnadvisor()
+
+
+def _watched():
+    """Whether something of torch looks at single operations or at what autograd saves, so that they have to happen one by
+    one: hooks on all modules, modes (other than a default device's), saved-tensor hooks, anomaly detection, forward-mode
+    differentiation, a functional transform, tracing, autocast."""
+    C = torch._C
+    return (_hooks._has_any_global_hook() or torch.is_autocast_enabled() or torch.is_anomaly_enabled()
+            or C._len_torch_dispatch_stack() > 0
+            or (C._len_torch_function_stack() > 0
+                and not all(isinstance(m, DeviceContext) for m in _get_current_function_mode_stack()))
+            or C._autograd._top_saved_tensors_default_hooks(True) is not None
+            or C._functorch.maybe_current_level() is not None or forward_ad._current_level >= 0
+            or torch.jit.is_tracing() or torch.compiler.is_compiling())
 
 
 def _replaced(obj, name, original):
@@ -56,9 +73,9 @@ class Net(torch.nn.Module):
     def native_weights(self, x):
         """The weights, where the operator module's whole-stack functions compute what the modules would: CUDA
         fp32 tensors, and nothing hooked in, replaced or differentiated between the layers.  None otherwise."""
-        if not (hasattr(GNNA, "net_forward") and GNNA.plans_enabled() and x.is_cuda and x.dtype == torch.float32 and not x.requires_grad
-                and x.dim() == 2 and x.size(0) > 0 and x.is_contiguous()
-                and type(self) is Net and not _hooks._has_any_global_hook() and not torch.is_autocast_enabled()):
+        if not (hasattr(GNNA, "net_forward") and GNNA.plans_enabled() and type(x) in (torch.Tensor, torch.nn.Parameter)
+                and x.is_cuda and x.dtype == torch.float32 and not x.requires_grad
+                and x.dim() == 2 and x.size(0) > 0 and x.is_contiguous() and type(self) is Net and not _watched()):
             return None
         weights = []
         for m in (self, *self.convs):

@@ -365,3 +365,41 @@ def test_a_forward_of_ones_own_is_called(cuda, what, monkeypatch):
         calls.clear()
         loss = tr.train_epoch(timed=epoch == 1)
         assert calls and loss.grad_fn is not None
+
+
+@pytest.mark.parametrize("what", ["saved tensors", "anomaly", "dispatch mode", "function mode", "forward mode", "global hook"])
+def test_whole_steps_give_way_to_what_watches_operations(cuda, what):
+    import contextlib
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    seen = []
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+
+    @contextlib.contextmanager
+    def hook():
+        handle = torch.nn.modules.module.register_module_forward_hook(lambda *a: seen.append(a[0]))
+        yield
+        handle.remove()
+
+    tr = _trainer()
+    assert tr._native_step(tr.ds.x) is not None
+    with {"saved tensors": lambda: torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(t), t)[1], lambda t: t),
+          "anomaly": torch.autograd.detect_anomaly, "dispatch mode": Dispatch, "function mode": Function,
+          "forward mode": torch.autograd.forward_ad.dual_level, "global hook": hook}[what]():
+        assert tr._native_step(tr.ds.x) is None
+        loss = tr.train_epoch()
+        assert loss.grad_fn is not None
+    if what not in ("anomaly", "forward mode"):
+        assert seen
+    with torch.device(cuda):                           # a default device is no observer
+        assert tr._native_step(tr.ds.x) is not None

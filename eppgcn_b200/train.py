@@ -296,6 +296,11 @@ class GCNTrainer:
                 return None
         return weights
 
+    @staticmethod
+    def _add_grads(weights, grads):
+        for w, g in zip(weights, grads):             # an optimizer of one's own may leave gradients to be added to
+            w.grad = g if w.grad is None else w.grad.add_(g)
+
     # EPPGCN/gcn_main.py:225-265
     def train_epoch(self, isFirstIter=False, timed=False, x=None):
         if self.path_from_cache:
@@ -312,8 +317,7 @@ class GCNTrainer:
             loss, *grads = self._step.run(x, weights, info.row_pointers, info.column_index, info.degrees, self.ds.y,
                                           self.ds.train_mask,
                                           [(b.id, b.partPointer, b.edgeList, b.numParts) for b in self.back_props])
-            for w, g in zip(weights, grads):
-                w.grad = g
+            self._add_grads(weights, grads)
             self.optimizer.step()
             return loss
         t0 = time.perf_counter()
@@ -349,8 +353,7 @@ class GCNTrainer:
         else:
             loss, *grads = GNNA.net_backward(rows, sums, x, weights, acts, last.degrees,
                                              [(b.id, b.partPointer, b.edgeList, b.numParts) for b in self.back_props])
-            for w, g in zip(weights, grads):
-                w.grad = g
+            self._add_grads(weights, grads)
         if timed:
             self._sync()
             self.back_time += time.perf_counter() - t0

@@ -403,3 +403,15 @@ def test_whole_steps_give_way_to_what_watches_operations(cuda, what):
         assert seen
     with torch.device(cuda):                           # a default device is no observer
         assert tr._native_step(tr.ds.x) is not None
+
+
+def test_gradients_are_added_to_those_that_are_kept(cuda):
+    tr = _trainer()
+    tr.optimizer = torch.optim.SGD(tr.model.parameters(), lr=0.0)
+    tr.train_epoch()
+    first = [w.grad.clone() for w in tr.model.parameters()]
+    tr.optimizer.zero_grad = lambda *a, **k: None
+    tr.train_epoch()
+    assert tr._step is not None
+    for w, g in zip(tr.model.parameters(), first):
+        assert (w.grad - 2 * g).norm() <= 1e-5 * g.norm()

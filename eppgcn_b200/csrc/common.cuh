@@ -65,12 +65,16 @@ __device__ __forceinline__ unsigned load_acquire_sys(const unsigned *p) {
 // of a replayed graph; here the kernels of an operation leave their own times.
 // The first kernel of an operation closes what is open (whose kernels have all
 // finished: same stream) and opens its slot, every kernel pushes its slot's end
-// forward.  Operations alternate between two slots, so that no block can push the
-// end of the operation that its kernel's first block is about to close.
+// forward.  Operations that follow each other use different slots, so that no
+// block can push the end of the operation that its kernel's first block is about
+// to close: slots 0 and 1 for those that come in pairs (also where a graph replays
+// them), 2 and 3 in turn for those that may follow themselves.
 // ---------------------------------------------------------------------------
+constexpr int kClockSlots = 4;
 struct StreamClock {
-  unsigned long long start[2], end[2];     // ns of the global timer
-  int category[2], layer[2], open[2];
+  unsigned long long start[kClockSlots], end[kClockSlots];     // ns of the global timer
+  int category[kClockSlots], layer[kClockSlots];
+  alignas(16) int open[kClockSlots];
   unsigned long long acc[11];              // closed operations, indexed like the host's accumulators
 };
 struct ClockMark {
@@ -86,9 +90,11 @@ __device__ __forceinline__ unsigned long long global_ns() {
 __device__ __forceinline__ void clock_begin(const ClockMark &m) {
   if (!m.clock || m.category < 0) return;
   StreamClock *c = m.clock;
+  const int4 all = *reinterpret_cast<const int4 *>(c->open);     // at once: the block's work waits for this
+  const int open[kClockSlots] = {all.x, all.y, all.z, all.w};
 #pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    if (!c->open[s]) continue;
+  for (int s = 0; s < kClockSlots; ++s) {
+    if (!open[s]) continue;
     const unsigned long long ns = c->end[s] > c->start[s] ? c->end[s] - c->start[s] : 0;
     c->acc[c->category[s]] += ns;
     if (c->category[s] == 2 && c->layer[s] >= 1 && c->layer[s] <= 6) c->acc[4 + c->layer[s]] += ns;

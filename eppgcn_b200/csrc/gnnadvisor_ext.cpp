@@ -55,7 +55,8 @@ struct ScopedTime {
 };
 
 // The kernels launched in its scope leave their times in the clock of `clock_stream`.  Operations that
-// follow each other use different slots: update 0 and aggregation 1 forward, aggregation 0 and update 1 backward.
+// follow each other use different slots: update 0 and aggregation 1 forward, aggregation 0 and update 1 backward; 2 for
+// one that may be followed by itself.
 struct ScopedMark {
   ScopedMark(int slot, int category, int layer, void *clock_stream) { eppgcn_mark_begin(slot, category, layer, clock_stream); }
   ~ScopedMark() { eppgcn_mark_end(); }
@@ -352,11 +353,12 @@ std::vector<torch::Tensor> spmm_forward(torch::Tensor input, torch::Tensor weigh
   CHECK_I32(row_pointers); CHECK_I32(column_index); CHECK_I32(part_pointers); CHECK_I32(part2Node);
   c10::cuda::CUDAGuard guard(input.device());
   torch::Tensor tmp;
+  const bool planned = plans_enabled() && input.size(0) > 0 && row_pointers.numel() == input.size(0) + 1;
   {
-    ScopedMark t(0, 1, 0, current_stream());
+    ScopedMark t(planned ? 0 : 2, 1, 0, current_stream());
     tmp = update_scaled_padded(input, weight, degrees);
   }
-  if (plans_enabled() && input.size(0) > 0 && row_pointers.numel() == input.size(0) + 1) {
+  if (planned) {
     const PlanPtr plan = forward_plan(row_pointers, column_index);
     ScopedMark t(1, 0, 0, current_stream());
     return {aggregate_planned(plan->handle, tmp, degrees, input.size(0))};
@@ -380,7 +382,8 @@ std::vector<torch::Tensor> spmm_backward(torch::Tensor d_output, torch::Tensor X
   CHECK_I32(row_pointers); CHECK_I32(column_index); CHECK_I32(part_pointers); CHECK_I32(part2Node);
   c10::cuda::CUDAGuard guard(d_output.device());
   torch::Tensor d_input_prime;
-  if (plans_enabled() && d_output.size(0) > 0 && row_pointers.numel() == d_output.size(0) + 1) {
+  const bool planned = plans_enabled() && d_output.size(0) > 0 && row_pointers.numel() == d_output.size(0) + 1;
+  if (planned) {
     const PlanPtr plan = forward_plan(row_pointers, column_index);
     ScopedMark t(0, 2, 0, current_stream());
     d_input_prime = aggregate_planned(plan->handle, pack_scaled(plan->handle, d_output, degrees), degrees, d_output.size(0));
@@ -389,7 +392,7 @@ std::vector<torch::Tensor> spmm_backward(torch::Tensor d_output, torch::Tensor X
     d_input_prime = aggregate_forward(d_output, row_pointers, column_index, degrees, part_pointers, part2Node,
                                       partSize, dimWorker, warpPerBlock);
   }
-  ScopedMark t(1, 3, 0, current_stream());
+  ScopedMark t(planned ? 1 : 2, 3, 0, current_stream());
   return backward_update(d_input_prime, X, W);
 }
 
@@ -409,7 +412,7 @@ void mask_forward(torch::Tensor id, torch::Tensor partPointer, torch::Tensor edg
   TORCH_CHECK(partPointer.numel() == id.numel() + 1 || id.numel() == 0,
               "partPointer must have one more entry than id");
   c10::cuda::CUDAGuard guard(id.device());
-  ScopedMark t(0, 4, 0, current_stream());
+  ScopedMark t(2, 4, 0, current_stream());
   // beyond what L1 holds of a byte per vertex, the marking gathers from a bit per vertex
   if (src_mask.numel() > 131072) {
     auto bits = at::empty({(src_mask.numel() + 31) / 32}, id.options());
@@ -464,7 +467,7 @@ std::vector<torch::Tensor> ours_backward_impl(torch::Tensor d_output, torch::Ten
                                              numParts, partSize, blockx, blocky, current_stream()),
               "eppgcn_spmm_backward_compacted");
   }
-  ScopedMark t(1, 3, 0, current_stream());
+  ScopedMark t(plan ? 1 : 2, 3, 0, current_stream());
   return backward_update(d_input_prime, X, W, plan ? plan->handle : nullptr, need_d_input);
 }
 

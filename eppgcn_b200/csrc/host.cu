@@ -108,16 +108,30 @@ Timers &timers() {
 struct Clocks {
   static constexpr int kPerDevice = 64;
   std::mutex mu;
-  std::map<std::pair<int, void *>, StreamClock *> of_stream;
+  struct Handed {
+    StreamClock *clock;
+    int turn;              // which of slots 2 and 3 the last operation that asked for either was given
+  };
+  std::map<std::pair<int, void *>, Handed> of_stream;
   std::map<int, std::pair<StreamClock *, int>> block;     // per device: its clocks and how many are not handed out
   float spill[11] = {0};
 
-  StreamClock *get(void *stream) {
+  // The clock of `stream` on the current device; `slot` 2 becomes 2 or 3, in turn.
+  StreamClock *get(void *stream, int &slot) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
     std::lock_guard<std::mutex> lock(mu);
+    Handed *h = handed(dev, stream);
+    if (!h) return nullptr;
+    if (slot == 2) {
+      h->turn ^= 1;
+      slot += h->turn;
+    }
+    return h->clock;
+  }
+  Handed *handed(int dev, void *stream) {
     const auto at = of_stream.find({dev, stream});
-    if (at != of_stream.end()) return at->second;
+    if (at != of_stream.end()) return &at->second;
     auto &f = block[dev];
     if (f.second == 0) {
       // allocating and draining synchronise, which a capture forbids: its operations go untimed
@@ -145,7 +159,7 @@ struct Clocks {
       }
       f.second = kPerDevice;
     }
-    return of_stream[{dev, stream}] = f.first + --f.second;
+    return &(of_stream[{dev, stream}] = Handed{f.first + --f.second, 0});
   }
   // Adds what the device has accumulated to `acc` (ms) and starts the clocks anew; waits for the devices.
   void drain(float *acc) {
@@ -162,12 +176,12 @@ struct Clocks {
     for (auto &entry : of_stream) {
       StreamClock h{};
       if (cudaSetDevice(entry.first.first) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
-          cudaMemcpy(&h, entry.second, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess ||
-          cudaMemset(entry.second, 0, sizeof(h)) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+          cudaMemcpy(&h, entry.second.clock, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess ||
+          cudaMemset(entry.second.clock, 0, sizeof(h)) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
         (void)cudaGetLastError();
         continue;
       }
-      for (int s = 0; s < 2; ++s)
+      for (int s = 0; s < kClockSlots; ++s)
         if (h.open[s] && h.end[s] > h.start[s]) {
           const unsigned long long ns = h.end[s] - h.start[s];
           h.acc[h.category[s]] += ns;
@@ -339,7 +353,7 @@ EPP_EXPORT int eppgcn_time_end(int slot, int category, int layer, void *stream) 
 }
 
 EPP_EXPORT int eppgcn_mark_begin(int slot, int category, int layer, void *stream) {
-  EPP_REQUIRE(slot == 0 || slot == 1, "slot must be 0 or 1");
+  EPP_REQUIRE(slot >= 0 && slot <= 2, "slot must be 0, 1 or 2");
   EPP_REQUIRE(category >= 0 && category <= 4, "unknown timer category");
   Timers &t = timers();
   bool on;
@@ -347,7 +361,8 @@ EPP_EXPORT int eppgcn_mark_begin(int slot, int category, int layer, void *stream
     std::lock_guard<std::mutex> lock(t.mu);
     on = t.enabled;
   }
-  t_mark = ClockMark{on ? clocks().get(stream) : nullptr, slot, category, layer};
+  StreamClock *clock = on ? clocks().get(stream, slot) : nullptr;
+  t_mark = ClockMark{clock, slot, category, layer};
   return EPP_OK;
 }
 

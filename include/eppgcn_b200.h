@@ -548,8 +548,8 @@ int eppgcn_timing_enable(int on);                 /* returns previous state */
 int eppgcn_timing_enabled(void);
 /* Device-side alternative to eppgcn_time_begin / _end for a sequence of operations on one stream: the
  * kernels that the calling thread launches between eppgcn_mark_begin and eppgcn_mark_end leave their own
- * times, without events (so a captured graph may hold them).  Consecutive operations of a stream alternate
- * slot 0 and 1. */
+ * times, without events (so a captured graph may hold them).  Consecutive operations of a stream have
+ * different slots: 0 and 1 where they come in pairs, 2 where an operation may follow itself. */
 int eppgcn_mark_begin(int slot, int category, int layer, void *stream);
 int eppgcn_mark_end(void);
 int eppgcn_time_begin(void *stream);              /* slot handle, or -1 when off */

@@ -415,3 +415,37 @@ def test_gradients_are_added_to_those_that_are_kept(cuda):
     assert tr._step is not None
     for w, g in zip(tr.model.parameters(), first):
         assert (w.grad - 2 * g).norm() <= 1e-5 * g.norm()
+
+
+@pytest.mark.parametrize("plans", [True, False])
+def test_operation_times_agree_with_events(cuda, plans, monkeypatch):
+    """The kernels' own times, against events around the calls: the same operation several times in a row (each closes the
+    one before), and pairs."""
+    import eppgcn_b200
+    from tests.helpers import t
+    gnna = eppgcn_b200.load_gnnadvisor()
+    if not plans:
+        monkeypatch.setenv("EPPGCN_B200_GROUP_KERNEL", "1")
+    n, e, repeats = 400_000, 6_000_000, 6
+    rng = np.random.Generator(np.random.PCG64(3))
+    indptr = np.concatenate([[0], np.cumsum(rng.multinomial(e, np.ones(n) / n))]).astype(np.int32)
+    col, row = t(rng.integers(0, n, e).astype(np.int32), cuda), t(indptr, cuda)
+    pp, p2n = gnna.build_part(15, row)
+    src = torch.rand(n, device=cuda) < 0.5
+    ngh, mask, deg = torch.zeros_like(src), torch.full((e,), -1, dtype=torch.int32, device=cuda), torch.zeros(n, dtype=torch.int32, device=cuda)
+    x, w, scale = torch.randn(n, 32, device=cuda), torch.randn(32, 16, device=cuda), torch.rand(n, device=cuda)
+    for f, categories in [(lambda: gnna.mask_forward(p2n, pp, col, src, ngh, mask, deg, 3, 1, 4, 16), (4,)),
+                          (lambda: gnna.forward(x, w, row, col, scale, pp, p2n, 15, 16, 8), (0, 1)),
+                          (lambda: gnna.backward(x, x, torch.eye(32, device=cuda), row, col, scale, pp, p2n, 15, 16, 8), (2, 3))]:
+        for _ in range(2):
+            f()
+        before = capi.time_read()
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda._sleep(2_000_000)                   # the calls queue up behind it: no gaps between their kernels
+        a.record()
+        for _ in range(repeats):
+            f()
+        b.record()
+        b.synchronize()
+        told, whole = sum(capi.time_read()[c] - before[c] for c in categories), a.elapsed_time(b)
+        assert 0.6 * whole <= told <= 1.02 * whole + 0.01, (categories, told, whole)

@@ -110,6 +110,9 @@ std::pair<torch::Tensor, int> missing_rows(const PlanPtr &plan, const PlanPtr &o
               "eppgcn_tile_plan_missing");
     plan->missing_count = rows[n].item<int>();
     plan->missing = rows.narrow(0, 0, plan->missing_count).clone();
+    // the next question may come from another stream
+    const cudaError_t e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
+    TORCH_CHECK(e == cudaSuccess, "listing the missing rows failed: ", cudaGetErrorString(e));
     plan->other = of;
   }
   return {plan->missing, plan->missing_count};

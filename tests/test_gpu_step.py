@@ -449,3 +449,27 @@ def test_operation_times_agree_with_events(cuda, plans, monkeypatch):
         b.synchronize()
         told, whole = sum(capi.time_read()[c] - before[c] for c in categories), a.elapsed_time(b)
         assert 0.6 * whole <= told <= 1.02 * whole + 0.01, (categories, told, whole)
+
+
+def test_whole_steps_on_two_streams(cuda):
+    """The rows that a plan is asked about on one stream are read by a step on another without waiting for it."""
+    from eppgcn_b200 import graphs, train
+    n, rng = 70_000, np.random.Generator(np.random.PCG64(1))
+    src, dst = rng.integers(0, n, 120_000), rng.integers(0, n, 120_000)
+    order = np.lexsort((dst, src))
+    g = graphs.Graph(np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32), dst[order].astype(np.int32))
+    ds = graphs.SyntheticDataset(g, 20, 5, 3, 0.05, seed=5)
+    ds.y = torch.randint(5, (n,), generator=torch.Generator().manual_seed(1))
+    tr = train.GCNTrainer(ds, hidden=16, seed=2)
+    tr.optimizer = torch.optim.SGD(tr.model.parameters(), lr=0.0)
+    torch.cuda.synchronize()
+    grads = []
+    for stream in (torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.current_stream()):
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(5_000_000)
+            tr.train_epoch()
+            grads.append([w.grad for w in tr.model.parameters()])
+    torch.cuda.synchronize()
+    for other in grads[1:]:
+        for a, b in zip(grads[0], other):
+            assert (a - b).norm() <= 1e-5 * b.norm() and b.norm() > 0

@@ -15,6 +15,7 @@
 //     1023 parts per vertex, cuCompactor.cu:500,527) and returns num_edges + 1
 //     entries, one more than the reference, so the closing pointer always fits.
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -86,14 +87,22 @@ struct PlanKey {
   }
 };
 
+// Memory that torch gave out for one stream is about to be used on another, perhaps still when it is given back.
+void used_on_current_stream(const torch::Tensor &t, void *home) {
+  const auto stream = at::cuda::getCurrentCUDAStream(t.get_device());
+  if (static_cast<void *>(stream.stream()) != home) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), stream);
+}
+
 // A plan and its device arrays; callers hold it while they launch on it (or keep a graph that does).
 struct Plan {
   eppgcn_tile_plan *handle = nullptr;
   torch::Tensor buffer;
+  void *home = nullptr;                // the stream that buffer was allocated on
   // the rows that another plan (the one asked about last) names as sources and this one has no edge for
   mutable std::mutex mu;
   mutable std::weak_ptr<const Plan> other;
   mutable torch::Tensor missing;
+  mutable void *missing_home = nullptr;
   mutable int missing_count = 0;
   ~Plan() { eppgcn_tile_plan_destroy(handle); }
 };
@@ -113,8 +122,10 @@ std::pair<torch::Tensor, int> missing_rows(const PlanPtr &plan, const PlanPtr &o
     // the next question may come from another stream
     const cudaError_t e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
     TORCH_CHECK(e == cudaSuccess, "listing the missing rows failed: ", cudaGetErrorString(e));
+    plan->missing_home = current_stream();
     plan->other = of;
   }
+  if (plan->missing_count) used_on_current_stream(plan->missing, plan->missing_home);
   return {plan->missing, plan->missing_count};
 }
 
@@ -138,11 +149,13 @@ class PlanCache {
     for (PlanEntry &e : entries_)
       if (e.key == key) {
         e.last_use = ++clock_;
+        used_on_current_stream(e.plan->buffer, e.plan->home);
         return e.plan;
       }
     const size_t bytes = eppgcn_tile_plan_bytes(edges, static_cast<int>(rows), static_cast<int>(sources));
     auto plan = std::make_shared<Plan>();
     plan->buffer = at::empty({static_cast<int64_t>((bytes + 7) / 8)}, opts.dtype(at::kLong));
+    plan->home = current_stream();
     epp_check(build(plan->buffer.data_ptr(), bytes, &plan->handle), "eppgcn_tile_plan");
     if (entries_.size() >= kCapacity) {
       size_t oldest = 0;

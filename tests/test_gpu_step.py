@@ -473,3 +473,25 @@ def test_whole_steps_on_two_streams(cuda):
     for other in grads[1:]:
         for a, b in zip(grads[0], other):
             assert (a - b).norm() <= 1e-5 * b.norm() and b.norm() > 0
+
+
+def test_plans_are_given_up_while_another_stream_uses_them(cuda):
+    """A plan's memory belongs to the stream that it was made on; it is not handed out again while another still reads it."""
+    import eppgcn_b200
+    from tests.helpers import random_csr, t
+    gnna = eppgcn_b200.load_gnnadvisor()
+    indptr, indices = random_csr(3000, 8.0, 4)
+    row, col = t(indptr, cuda), t(indices, cuda)
+    pp, p2n = gnna.build_part(8, row)
+    x, w, deg = torch.randn(3000, 24, device=cuda), torch.randn(24, 16, device=cuda), torch.rand(3000, device=cuda)
+    gnna.clear_plans()
+    want = gnna.forward(x, w, row, col, deg, pp, p2n, 8, 16, 8)[0]
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(50_000_000)
+        got = gnna.forward(x, w, row, col, deg, pp, p2n, 8, 16, 8)[0]
+    gnna.clear_plans()
+    rest = [torch.zeros(size, dtype=torch.int32, device=cuda) for size in range(1 << 10, 1 << 18, 1 << 12)]   # harmless ids
+    torch.cuda.synchronize()
+    assert rest and (got - want).norm() <= 1e-6 * want.norm()

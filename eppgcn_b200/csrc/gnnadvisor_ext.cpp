@@ -246,7 +246,7 @@ torch::Tensor pack_scaled(const eppgcn_tile_plan *plan, const torch::Tensor &x, 
 // Device buffers of a step: allocated as they are asked for; `keep` holds on to all of them (a graph's own buffers).
 struct NetBuffers {
   bool keep = false;
-  std::vector<torch::Tensor> kept;
+  std::vector<torch::Tensor> kept, also;
   size_t next = 0;
   torch::Tensor rows(int64_t n, int64_t ld, const torch::Tensor &like) {
     if (next < kept.size()) return kept[next++];
@@ -256,6 +256,10 @@ struct NetBuffers {
       ++next;
     }
     return t;
+  }
+  // A plan's own array that the step reads: a plan may replace it while a graph still does.
+  void hold(const torch::Tensor &t) {
+    if (keep) also.push_back(t);
   }
 };
 
@@ -634,6 +638,7 @@ void run_backward(torch::Tensor grad, const torch::Tensor &x, const std::vector<
     const float *gate = acts[i - 1].data_ptr<float>();
     if (by_rows) {
       const auto [zeros, count] = missing_rows(plans[i], plans[i - 1], n, stream);
+      buffers.hold(zeros);
       epp_check(eppgcn_update_listed(next.data_ptr<float>(), ldi, d_prime.data_ptr<float>(), ld,
                                      weights[i].data_ptr<float>(), 1, d, degrees.data_ptr<float>(), gate,
                                      acts[i - 1].stride(0), 0, rows, listed, static_cast<int>(d), static_cast<int>(din),

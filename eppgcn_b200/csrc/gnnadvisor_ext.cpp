@@ -145,6 +145,7 @@ class PlanCache {
   PlanPtr get(const PlanKey &key, const torch::Tensor &key_a, const torch::Tensor &key_b,
               int64_t edges, int64_t rows, int64_t sources, Build build) {
     const auto opts = key_a.options();
+    PlanEntry dropped;                 // given up after the lock: letting go of a tensor may wait for the interpreter's lock
     std::lock_guard<std::mutex> lock(mu_);
     for (PlanEntry &e : entries_)
       if (e.key == key) {
@@ -161,6 +162,7 @@ class PlanCache {
       size_t oldest = 0;
       for (size_t i = 1; i < entries_.size(); ++i)
         if (entries_[i].last_use < entries_[oldest].last_use) oldest = i;
+      dropped = std::move(entries_[oldest]);
       entries_.erase(entries_.begin() + static_cast<std::ptrdiff_t>(oldest));
     }
     entries_.push_back(PlanEntry{key, plan, key_a, key_b, ++clock_});
@@ -168,8 +170,9 @@ class PlanCache {
   }
 
   void clear() {
+    std::vector<PlanEntry> dropped;
     std::lock_guard<std::mutex> lock(mu_);
-    entries_.clear();
+    dropped.swap(entries_);
   }
 
   size_t size() {
@@ -1263,7 +1266,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   py::class_<NetStep>(m, "NetStep", "a training step's forward, loss and backward in one call (not in the reference)")
       .def(py::init<>())
       .def("run", &NetStep::run, py::call_guard<py::gil_scoped_release>())
-      .def("replays", &NetStep::replays);
+      .def("replays", &NetStep::replays, py::call_guard<py::gil_scoped_release>());
   m.def("adam_step", &adam_step, "Adam step over a list of parameters (not in the reference)");
   m.def("to_device", &to_device, "a host tensor on a CUDA device, large ones by several threads (not in the reference)",
         py::call_guard<py::gil_scoped_release>());

@@ -495,3 +495,39 @@ def test_plans_are_given_up_while_another_stream_uses_them(cuda):
     rest = [torch.zeros(size, dtype=torch.int32, device=cuda) for size in range(1 << 10, 1 << 18, 1 << 12)]   # harmless ids
     torch.cuda.synchronize()
     assert rest and (got - want).norm() <= 1e-6 * want.norm()
+
+
+def test_plan_cache_under_several_threads(cuda):
+    """Steps that run without the interpreter's lock, operators that hold it, and more plans than are kept."""
+    import threading
+    import eppgcn_b200
+    from tests.helpers import random_csr, t
+    gnna = eppgcn_b200.load_gnnadvisor()
+    tr = _trainer()
+    stop, errors = threading.Event(), []
+
+    def work(f):
+        try:
+            while not stop.is_set():
+                f()
+        except Exception as e:                         # noqa: BLE001
+            errors.append(e)
+
+    def operators():
+        for seed in range(20):
+            indptr, indices = random_csr(60, 3.0, seed)
+            row, col = t(indptr, cuda), t(indices, cuda)
+            pp, p2n = gnna.build_part(4, row)
+            gnna.forward(torch.ones(60, 8, device=cuda), torch.ones(8, 8, device=cuda), row, col, torch.ones(60, device=cuda),
+                         pp, p2n, 4, 16, 8)
+        gnna.clear_plans()
+
+    threads = [threading.Thread(target=work, args=(f,), daemon=True)
+               for f in (operators, operators, tr.train_epoch, lambda: tr._step and tr._step.replays())]
+    for th in threads:
+        th.start()
+    stop.wait(3.0)
+    stop.set()
+    for th in threads:
+        th.join(60.0)
+    assert not errors and not any(th.is_alive() for th in threads)

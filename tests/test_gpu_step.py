@@ -531,3 +531,69 @@ def test_plan_cache_under_several_threads(cuda):
     for th in threads:
         th.join(60.0)
     assert not errors and not any(th.is_alive() for th in threads)
+
+
+@pytest.mark.parametrize("n,pairs,hubs,dims,ratio,symmetric", [
+    (70_000, 200_000, False, (20, 16, 5), 0.05, True), (70_000, 120_000, False, (20, 16, 16, 5), 0.05, False),
+    (66_000, 150_000, False, (33, 16, 47), 0.3, True), (90_001, 300_000, True, (24, 16, 22), 0.5, True),
+    (100_003, 400_000, True, (64, 64, 64, 32), 0.05, True), (66_000, 250_000, True, (96, 16, 16, 16, 22), 0.1, False),
+    (5000, 20_000, True, (1433, 16, 7), 0.3, True)])
+def test_step_against_float64_with_its_own_gates(cuda, n, pairs, hubs, dims, ratio, symmetric):
+    """Every layer's result and every gradient at the sizes where the backward walks the path's rows.  An activation that
+    rounds to the other side of zero would hide behind a loose bound; the code's own results are the reference's inputs and
+    gates here, and what is left is the rounding of 32-bit sums: below 5e-7 of a gradient's norm, asserted at 2e-6."""
+    import eppgcn_b200
+    from eppgcn_b200 import graphs, train
+    gnna = eppgcn_b200.load_gnnadvisor()
+    rng = np.random.Generator(np.random.PCG64(n))
+    src, dst = rng.integers(0, n, pairs), rng.integers(0, n, pairs)
+    if hubs:                                           # a third of the endpoints on 50 vertices: rows summed in many pieces
+        dst[::3] = rng.integers(0, 50, len(dst[::3])) * (n // 50)
+    if symmetric:
+        indptr, indices = graphs.csr_from_pairs(n, src, dst)
+    else:
+        key = np.unique(src * n + dst)
+        indptr = np.concatenate([[0], np.cumsum(np.bincount(key // n, minlength=n))]).astype(np.int32)
+        indices = (key % n).astype(np.int32)
+    ds = graphs.SyntheticDataset(graphs.Graph(indptr, indices), dims[0], dims[-1], len(dims) - 1, ratio, seed=5)
+    ds.y = torch.randint(dims[-1], (n,), generator=torch.Generator().manual_seed(1))
+    tr = train.GCNTrainer(ds, hidden=dims[1], seed=2)
+    info, weights = tr.inputInfo, [w.detach() for w in tr.model.parameters()]
+    deg, mask = ds.degrees.double()[:, None], ds.train_mask
+
+    def aggregate(rows, cols, m):
+        return deg * torch.zeros_like(m).index_add_(0, rows.long(), (deg * m)[cols.long()])
+
+    edge_rows = torch.repeat_interleave(torch.arange(n, device=cuda), (info.row_pointers[1:] - info.row_pointers[:-1]).long())
+    acts = gnna.net_forward(ds.x, weights, info.row_pointers, info.column_index, ds.degrees)
+    inputs = [ds.x.double()] + [a.double().clamp(min=0) for a in acts[:-1]]
+    for h, w, got in zip(inputs, weights, acts):
+        want = aggregate(edge_rows, info.column_index, h @ w.double())
+        mag = aggregate(edge_rows, info.column_index, h.abs() @ w.double().abs())
+        assert ((got.double() - want).abs() <= 1e-7 + 3e-6 * mag).all()
+
+    paths = [(b.id, b.partPointer, b.edgeList, b.numParts) for b in tr.back_props]
+    logp = torch.log_softmax(acts[-1].double(), 1)
+    onehot = torch.nn.functional.one_hot(ds.y, dims[-1]).double()
+    want_loss = -(logp * onehot).sum(1)[mask].mean().item()
+    g, want = (logp.exp() - onehot) * mask[:, None] / int(mask.sum()), []
+    for i in reversed(range(len(weights))):
+        b = tr.back_props[i]
+        d_prime = aggregate(b.id[:b.valid_len], b.edgeList[:b.valid_len], g)
+        want.insert(0, inputs[i].T @ d_prime)
+        if i:
+            g = d_prime @ weights[i].double().T * (acts[i - 1] > 0)
+
+    def same(loss, grads):
+        assert abs(loss.item() - want_loss) <= 1e-6 * want_loss
+        for got, ref in zip(grads, want):
+            assert ref.norm() > 0 and (got.double() - ref).norm() <= 2e-6 * ref.norm()
+
+    rows, sums = gnna.net_loss(acts[-1], ds.y, mask, ds.degrees, *paths[-1])
+    loss, *grads = gnna.net_backward(rows, sums, ds.x, weights, acts, ds.degrees, paths)
+    same(loss, grads)
+    if not hubs:                                       # a repeated forward has the same bits, so the whole step has these gates
+        step = gnna.NetStep()
+        for _ in range(4):
+            loss, *grads = step.run(ds.x, weights, info.row_pointers, info.column_index, ds.degrees, ds.y, mask, paths)
+            same(loss, grads)

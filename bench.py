@@ -639,7 +639,7 @@ def run_gpu(args):
         ev1.record(stream)
         torch.cuda.synchronize()
         epoch_full = {"ms": round(ev0.elapsed_time(ev1) / args.steps, 4),
-                      "what": "forward + log_softmax/nll_loss + backward + Adam through GCNConv, X resident"}
+                      "what": "GCNTrainer.train_epoch: forward, masked NLL loss and backward as one whole step, then Adam; X resident"}
         del tr, ds2
 
     # -- the reference's own kernels on this GPU, in a child process -----------------

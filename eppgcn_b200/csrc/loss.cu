@@ -44,7 +44,7 @@ __device__ __forceinline__ void add_loss(double loss, int count, double *sums) {
 
 // Up to 64 columns.  A warp reads the flags of 32 rows at a time and queues the rows that have something to do; as soon
 // as 32 are queued every lane takes one, whole, in registers.  Eight lanes per row with shuffles between them spent 970
-// instructions on 32 rows, queued or not: 110 us on 2 M rows x 22 classes with 10 % of them labelled, 41 now.
+// instructions on 32 rows, queued or not: 110 us on 2 M rows x 22 classes with 10 % of them labelled, 40 now (104 with half).
 template <int QUADS>
 __global__ void __launch_bounds__(256) masked_nll_kernel(const float *__restrict__ z, long long ldz,
                                                          const long long *__restrict__ labels,

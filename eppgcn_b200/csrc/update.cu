@@ -120,8 +120,8 @@ __device__ __forceinline__ bool all_nan(const float *w, long long w_row, long lo
 
 // ---------------------------------------------------------------------------
 // Many rows: persistent warps over tiles of 32 rows.  W's fragments are split once per block and stay in shared
-// memory; steps of 16 k are loaded two to four ahead, across tiles.  2 M x 128 -> 16: 240 us = 5.1 TB/s; 1 M x 128 ->
-// 64: 360 us (524 by FMA), bound by the rate of mma.sync.
+// memory; steps of 16 k are loaded two to four ahead, across tiles.  2 M x 128 -> 16: 226 us = 5.3 TB/s; 1 M x 128 ->
+// 64: 326 us (524 by FMA), tensor pipe 59 % busy at one block per SM, bound by dependent products.
 // ---------------------------------------------------------------------------
 template <int NT>
 struct ManyRowsShape {
@@ -589,7 +589,10 @@ UpdateShape update_shape(int n, int k, int dout, bool listed, int sms) {
   // From one tile of 32 rows per resident warp on, the many-row kernel keeps the chip busy; results of more than four
   // blocks go through the other, which does not hold W's fragments for every block.
   u.many_rows = listed || (k <= kMmaMaxK && n >= 32 * kMmaWarps * sms && u.col_blocks <= 4);
-  // 32 rows per warp share W's fragments and give twice the independent products, where there are enough of them
+  // 32 rows per warp share W's fragments and give twice the independent products.  With 16 and
+  // with 32 rows, in us: 8192 x 1433 -> 32 30.3 and 29.0, -> 64 54.4 and 46.9, 24000 x 1433 -> 32 93 and 78; but -> 64 155
+  // and 172, 16384 x 1433 -> 16 38.6 and 51.8, and with short k 16 rows are faster throughout (16384 x 16 -> 16 3.6 and
+  // 4.7).  The line at 8192 rows fits the wide results only.
   u.m = n >= 8192 ? 2 : 1;
   u.parts = u.many_rows ? 1 : choose_parts(ceil_div_ll(n, 16 * u.m * kMmaWarps) * u.col_blocks, (k + 15) / 16,
                                            few_rows_most_steps(u.nt, u.m), static_cast<long long>(sms) * few_rows_resident(u.nt),

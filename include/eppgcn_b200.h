@@ -111,7 +111,8 @@ int eppgcn_spmm_backward_compacted(float *d_in, long long d_in_ld, const float *
  * number of edges and keeps its own padded copy of the edge list, so that the
  * lanes of a warp always work on rows of one length class, every row of up to
  * 64 edges is stored exactly once, and only longer rows are cleared first and
- * summed with vector atomics.
+ * summed with vector atomics, so the last bits of rows with more than 128 edges
+ * (three pieces or more) vary from run to run.
  *
  *   out[r][:] = row_scale[r] * sum over edges e of row r:  src[col_idx[e]][:]
  *
@@ -200,7 +201,11 @@ int eppgcn_debug_status(int *out4, int reset);
  *
  *   out[r][c] = scale[r] * sum_k x[r][k] * w[k][c]        c < dout <= 32
  *
- * FP32 FMA on the CUDA cores (no reduced-precision tensor-core path).
+ * At fp32 accuracy, on the tensor cores: operands are cut into three bf16 pieces
+ * that hold all 24 bits, and sums are kept in fp32.  The 2-norm error against
+ * float64 is at most that of an fp32 FMA chain (9.5e-8 for 128 normal terms).
+ * Infinities and NaN come out as a plain fp32 sum gives them.  Results have the
+ * same bits on every run.
  * x    [num_rows] rows of stride ldx floats, w [k] rows of stride ldw floats,
  * out  rows of stride ld_out floats; the call writes columns 0..dout-1 and
  *      zero-fills the pad_cols columns after them (ld_out >= dout + pad_cols).
@@ -222,8 +227,9 @@ int eppgcn_update_scaled(float *out, long long ld_out, const float *x, long long
  *
  *   dw[kk][c] = sum_r x[r][kk] * d[r][c]        dw dense [k][dout], overwritten
  *
- * FP32 FMA; partial sums of row slabs are combined with atomics, so the
- * summation order varies from run to run.  dout <= 32 and k * dout <= 4096
+ * At fp32 accuracy by the same products of bf16 pieces; partial sums of row
+ * slabs are combined with atomics, so the summation order, and with it the last
+ * bits, vary from run to run.  dout <= 32 and k * dout <= 4096
  * (after rounding both up to multiples of 4), else EPP_ERR_TOO_LARGE.
  * x and d must be 16-byte aligned; strides that are multiples of 4 floats are
  * read with 16-byte copies.

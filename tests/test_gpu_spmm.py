@@ -133,7 +133,7 @@ def test_backward_train_ratios(cuda, ratio):
                                       (333, 130, 32), (2049, 16, 22), (64, 7, 5)])
 @pytest.mark.parametrize("scaled", [True, False])
 def test_update_scaled(cuda, n, k, dout, scaled):
-    """diag(scale) (X W) with FP32 FMA against float64; K-long fp32 dot products."""
+    """diag(scale) (X W) at fp32 accuracy against float64; K-long fp32 dot products."""
     rng = np.random.Generator(np.random.PCG64(n + k + dout))
     kp = (k + 3) // 4 * 4
     x_full = torch.full((n, kp), float("nan"), device=cuda)                  # row stride padded to 16 bytes
@@ -179,7 +179,7 @@ def test_forward_prescaled_rows(cuda, dim):
                                       (100_003, 128, 16), (4097, 128, 32), (70_000, 16, 22), (3000, 200, 20),
                                       (2000, 1000, 4), (999, 22, 16), (777, 40, 28), (50_000, 64, 32), (9, 3, 1)])
 def test_weight_grad(cuda, n, k, dout):
-    """X^T d' with FP32 FMA and atomically combined slabs, against float64."""
+    """X^T d' at fp32 accuracy with atomically combined slabs, against float64."""
     rng = np.random.Generator(np.random.PCG64(n + k))
     x = rng.standard_normal((n, k)).astype(np.float32)
     d = rng.standard_normal((n, dout)).astype(np.float32)
@@ -199,7 +199,7 @@ def test_weight_grad_limits(cuda):
 
 
 def test_operator_backward_products_match_float64(cuda):
-    """ours_backward's d_input and d_weight through the FMA kernels (Din 128 -> four 32-column launches)."""
+    """ours_backward's d_input and d_weight through this library's kernels (Din 128 -> four 32-column launches)."""
     import eppgcn_b200
     gnna = eppgcn_b200.load_gnnadvisor()
     indptr, indices = random_csr(**GRAPHS["hubs"])
@@ -279,7 +279,7 @@ def test_weight_grad_over_the_rows_of_a_path(cuda):
 @pytest.mark.parametrize("din,dout", [(128, 64), (64, 64), (64, 32), (40, 36)])
 def test_operator_handles_wide_layers_without_library_gemms(cuda, din, dout):
     """forward and ours_backward for layers wider than one 32-column block (the 3-layer configuration:
-    128 -> 64 -> 64 -> 32): update, d_input and d_weight go through this library's FMA kernels block
+    128 -> 64 -> 64 -> 32): update, d_input and d_weight go through this library's kernels block
     by block and match float64."""
     import eppgcn_b200
     gnna = eppgcn_b200.load_gnnadvisor()

@@ -597,3 +597,22 @@ def test_step_against_float64_with_its_own_gates(cuda, n, pairs, hubs, dims, rat
         for _ in range(4):
             loss, *grads = step.run(ds.x, weights, info.row_pointers, info.column_index, ds.degrees, ds.y, mask, paths)
             same(loss, grads)
+
+
+def test_long_rows_with_less_room_than_is_of_use(cuda):
+    """Fewer stretches in a smaller buffer, none in one that holds not even two; a misaligned one is refused."""
+    n, k, dout = 1000, 3000, 7
+    x, w, lib = torch.randn(n, k, device=cuda), torch.randn(k, dout, device=cuda), capi.lib()
+    want, mag = x.double() @ w.double(), x.double().abs() @ w.double().abs()
+    most, part = lib.eppgcn_update_scratch_bytes(n, k, dout), 4 * n * 8
+    assert most % part == 0 and most >= 4 * part and lib.eppgcn_update_scratch_bytes(n, 16, dout) == 0
+    room = torch.empty(most // 4 + 4, device=cuda)
+    args = lambda out: (out.data_ptr(), dout, x.data_ptr(), k, w.data_ptr(), dout, 1, None, None, 0, 0, n, k, dout, 0)  # noqa: E731
+    for given in (0, part - 4, part, 2 * part + 4, 3 * part, most):
+        room.fill_(float("nan"))
+        out = torch.empty(n, dout, device=cuda)
+        capi.check(lib.eppgcn_update_rows_scratch(*args(out), room.data_ptr(), given, None))
+        torch.cuda.synchronize()
+        assert ((out.double() - want).abs() <= 1e-6 + 2e-6 * mag).all()
+        assert room[given // 4:].isnan().all()                              # nothing beyond the room that was given
+    assert lib.eppgcn_update_rows_scratch(*args(out), room.data_ptr() + 4, most, None) == capi.EPP_ERR_BAD_ARG

@@ -14,14 +14,14 @@
 // zero-filled and written again.
 //
 // Work unit.  A "sub-warp" of L = ceil(columns / 4) lanes (four columns per
-// lane: 4 lanes for 16 columns, 6 for 22; eight from 33 columns on) owns one row of the
+// lane: 4 lanes for 16 columns, 6 for 22; eight from 25 columns on) owns one row of the
 // current class, a warp owns floor(32 / L) consecutive rows of that class ("a tile"),
 // and tiles are dealt to the persistent warps in descending class order.  All
-// sub-warps of a warp therefore run the same number of batches of eight
-// independent 16-byte row loads, close their rows at the same instruction, and
+// sub-warps of a warp therefore run the same number of batches of eight (four
+// with eight columns per lane) independent row loads, close their rows at the same instruction, and
 // no lane ever waits for a neighbour's longer row -- the cost the group kernel
-// (spmm.cu) pays for groups of mixed length.  In the three narrow classes a
-// sub-warp packs 8, 4 or 2 rows into one batch.
+// (spmm.cu) pays for groups of mixed length.  In the classes narrower than a
+// batch a sub-warp packs several rows into one.
 //
 // Source rows already carry their source-side factor (the update step, or the
 // backward's packing step, folds it in); the destination-side factor is
@@ -47,10 +47,7 @@ constexpr unsigned kAtomicBit = 0x80000000u;    // in a rank's row id: the piece
 // takes up to 8 rows): divisible by every rows-per-tile value floor(32 / L), L = 1..32.
 constexpr int kRankPad = 480;
 constexpr int kTileThreads = EPP_TILE_THREADS;
-template <int C>
-struct TileResident {                            // blocks per SM with C columns per lane
-  static constexpr int blocks = C == 8 ? 2 : EPP_TILE_MINB;
-};
+constexpr int kTileResident = EPP_TILE_MINB;     // blocks per SM
 
 // Classes in processing order (widest first).  Class k covers ranks
 // [rank_off[k], rank_off[k+1]) and slots [slot_off[k], slot_off[k+1]); a rank
@@ -116,10 +113,13 @@ __device__ __forceinline__ void debug_report(int code, int value, int limit, int
 }
 #endif
 
-__device__ __forceinline__ void load8(const int *p, int (&c)[8]) {
-  const int4 a = __ldg(reinterpret_cast<const int4 *>(p));
-  const int4 b = __ldg(reinterpret_cast<const int4 *>(p) + 1);
-  c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w; c[4] = b.x; c[5] = b.y; c[6] = b.z; c[7] = b.w;
+template <int B>
+__device__ __forceinline__ void load_ids(const int *p, int (&c)[B]) {
+#pragma unroll
+  for (int i = 0; i < B; i += 4) {
+    const int4 a = __ldg(reinterpret_cast<const int4 *>(p + i));
+    c[i] = a.x; c[i + 1] = a.y; c[i + 2] = a.z; c[i + 3] = a.w;
+  }
 }
 
 // The lane's C columns of a source row (4 or 8; 32 bytes in one load are new with sm_100).
@@ -152,19 +152,50 @@ __device__ __forceinline__ void write_cols(float *dst, const float (&acc)[C], fl
     else store_row<4>(dst + h, val, min(4, n - h), OV);
   }
 }
-template <int OV, int C>
-__device__ __forceinline__ void put_row(const TileArgs &a, float *out_lane, int rid, const float (&acc)[C], int n,
-                                        bool has_cols) {
-  if (rid == -1 || !has_cols) return;
-  const int row = static_cast<int>(static_cast<unsigned>(rid) & ~kAtomicBit);
-#ifdef EPP_DEBUG_BOUNDS
-  if (row >= a.num_rows) {
-    debug_report(2, row, a.num_rows, -1);
-    return;
+// The rows of a narrow class's batch: PER rows of W neighbouring edges each, all of a sub-warp.  Ids and factors of all
+// rows are asked for at once, behind the batch's row loads.  One row after the other, each with two loads that depend on
+// each other in front of its store, made such a tile as long as a dozen batches: 13 M edges on 1.13 M vertices x 16
+// columns 118 us, 106 now; 35.6 M edges on 2.1 M vertices, half of them with their self loop only, 244 and 225.
+template <int OV, int C, int B, int W>
+__device__ __forceinline__ void close_narrow(const TileArgs &a, float *out_lane, const int *row_of, const int (&c)[B],
+                                             const float (&v)[B][C], int n, bool has_cols) {
+  constexpr int PER = B / W;
+  int rid[PER];
+  if constexpr (PER == 1) {
+    rid[0] = __ldg(row_of);
+  } else if constexpr (PER == 2) {
+    const int2 r = __ldg(reinterpret_cast<const int2 *>(row_of));
+    rid[0] = r.x; rid[1] = r.y;
+  } else {
+#pragma unroll
+    for (int i = 0; i < PER; i += 4) {
+      const int4 r = __ldg(reinterpret_cast<const int4 *>(row_of + i));
+      rid[i] = r.x; rid[i + 1] = r.y; rid[i + 2] = r.z; rid[i + 3] = r.w;
+    }
   }
+  float scale[PER];
+#pragma unroll
+  for (int r = 0; r < PER; ++r) {
+    scale[r] = 1.f;
+    const int row = static_cast<int>(static_cast<unsigned>(rid[r]) & ~kAtomicBit);
+#ifdef EPP_DEBUG_BOUNDS
+    if (rid[r] != -1 && row >= a.num_rows) {
+      debug_report(2, row, a.num_rows, -1);
+      rid[r] = -1;
+    }
 #endif
-  const float s = a.row_scale ? __ldg(a.row_scale + row) : 1.f;
-  write_cols<OV, C>(out_lane + static_cast<long long>(row) * a.out_ld, acc, s, n, rid < 0 || a.accumulate);
+    if (rid[r] != -1 && a.row_scale) scale[r] = __ldg(a.row_scale + row);
+  }
+#pragma unroll
+  for (int r = 0; r < PER; ++r) {
+    float acc[C] = {};
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+      if (c[W * r + j] >= 0) add_cols<C>(acc, v[W * r + j]);
+    if (rid[r] == -1 || !has_cols) continue;
+    const int row = static_cast<int>(static_cast<unsigned>(rid[r]) & ~kAtomicBit);
+    write_cols<OV, C>(out_lane + static_cast<long long>(row) * a.out_ld, acc, scale[r], n, rid[r] < 0 || a.accumulate);
+  }
 }
 
 // Position of a tile: its class, and the first rank and slot of this
@@ -174,10 +205,11 @@ struct TilePos {
   int rank;
   long long slot;
 };
+template <int B>
 __device__ __forceinline__ TilePos locate(const ClassTable &t, int G, int tile, int sub, int &k) {
   while (k + 1 < t.count && tile >= t.tile_begin[k + 1]) ++k;
   const int w = t.width[k];
-  const int per_sub = w >= 8 ? 1 : 8 / w;                    // rows of one sub-warp in this tile
+  const int per_sub = w >= B ? 1 : B / w;                    // rows of one sub-warp in this tile
   const int first = ((tile - t.tile_begin[k]) * G + sub) * per_sub;
   TilePos p;
   p.width = w;
@@ -186,8 +218,8 @@ __device__ __forceinline__ TilePos locate(const ClassTable &t, int G, int tile, 
   return p;
 }
 
-template <int OV, int C>
-__global__ void __launch_bounds__(kTileThreads, TileResident<C>::blocks) tiled_spmm_kernel(const TileArgs a) {
+template <int OV, int C, int B>
+__global__ void __launch_bounds__(kTileThreads, kTileResident) tiled_spmm_kernel(const TileArgs a) {
   if (blockIdx.x == 0 && threadIdx.x == 0) clock_begin(a.mark);
   const int G = kWarp / a.lanes;               // rows (of the wide classes) per tile
   const int lane = threadIdx.x & 31;
@@ -208,23 +240,23 @@ __global__ void __launch_bounds__(kTileThreads, TileResident<C>::blocks) tiled_s
   if (tile >= a.num_tiles) return;
 
   int k = 0;
-  TilePos pos = locate(a.t, G, tile, sub, k);
-  int c[8];
-  load8(a.slots + pos.slot, c);
-  int rid_wide = pos.width >= 8 ? __ldg(a.row_of + pos.rank) : -1;
+  TilePos pos = locate<B>(a.t, G, tile, sub, k);
+  int c[B];
+  load_ids<B>(a.slots + pos.slot, c);
+  int rid_wide = pos.width >= B ? __ldg(a.row_of + pos.rank) : -1;
   for (; tile < a.num_tiles; tile += stride) {
     // the position of this warp's next tile, its first eight ids and its row id are fetched behind
     // this tile's row loads
     const int next = tile + stride;
     TilePos npos = pos;
     int kn = k;
-    if (next < a.num_tiles) npos = locate(a.t, G, next, sub, kn);
-    int cn[8];
+    if (next < a.num_tiles) npos = locate<B>(a.t, G, next, sub, kn);
+    int cn[B];
     int rid_next = -1;
-    float v[8][C];
+    float v[B][C];
     auto gather = [&]() {
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
+      for (int u = 0; u < B; ++u) {
 #ifdef EPP_DEBUG_BOUNDS
         if (c[u] >= a.num_sources) {
           debug_report(1, c[u], a.num_sources, tile);
@@ -237,11 +269,11 @@ __global__ void __launch_bounds__(kTileThreads, TileResident<C>::blocks) tiled_s
     };
     auto prefetch_next = [&]() {
       if (next < a.num_tiles) {
-        load8(a.slots + npos.slot, cn);
-        if (npos.width >= 8) rid_next = __ldg(a.row_of + npos.rank);
+        load_ids<B>(a.slots + npos.slot, cn);
+        if (npos.width >= B) rid_next = __ldg(a.row_of + npos.rank);
       }
     };
-    if (pos.width >= 8) {
+    if (pos.width >= B) {
       // one row per sub-warp, width/8 batches; the row's factor is asked for before the first batch
       int rid = rid_wide;
       const int row = static_cast<int>(static_cast<unsigned>(rid) & ~kAtomicBit);
@@ -255,53 +287,29 @@ __global__ void __launch_bounds__(kTileThreads, TileResident<C>::blocks) tiled_s
       float acc[C] = {};
       const int *cp = a.slots + pos.slot;
 #pragma unroll 1
-      for (int b = 0; b < pos.width; b += 8) {
+      for (int b = 0; b < pos.width; b += B) {
         gather();
-        if (b + 8 < pos.width) load8(cp + b + 8, cn);
+        if (b + B < pos.width) load_ids<B>(cp + b + B, cn);
         else prefetch_next();
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+        for (int u = 0; u < B; ++u)
           if (c[u] >= 0) add_cols<C>(acc, v[u]);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) c[u] = cn[u];
+        for (int u = 0; u < B; ++u) c[u] = cn[u];
       }
       if (rid != -1 && has_cols) {
         write_cols<OV, C>(out_lane + static_cast<long long>(row) * a.out_ld, acc, scale, n, rid < 0 || a.accumulate);
       }
     } else {
-      // narrow classes: 8 / 4 / 2 rows of 1 / 2 / 4 slots in one batch; a row's id and factor are
-      // fetched when it is written (these classes hold a few per cent of the edges)
+      // narrow classes: rows of 1, 2 or (with a batch of 8) 4 slots, several in one batch
       gather();
       prefetch_next();
-      const int *rid = a.row_of + pos.rank;
-      if (pos.width == 1) {
+      const int *row_of = a.row_of + pos.rank;
+      if (pos.width == 1) close_narrow<OV, C, B, 1>(a, out_lane, row_of, c, v, n, has_cols);
+      else if (B == 4 || pos.width == 2) close_narrow<OV, C, B, 2>(a, out_lane, row_of, c, v, n, has_cols);
+      else close_narrow<OV, C, B, 4>(a, out_lane, row_of, c, v, n, has_cols);
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          float acc[C] = {};
-          if (c[r] >= 0) add_cols<C>(acc, v[r]);
-          put_row<OV, C>(a, out_lane, __ldg(rid + r), acc, n, has_cols);
-        }
-      } else if (pos.width == 2) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          float acc[C] = {};
-#pragma unroll
-          for (int j = 0; j < 2; ++j)
-            if (c[2 * r + j] >= 0) add_cols<C>(acc, v[2 * r + j]);
-          put_row<OV, C>(a, out_lane, __ldg(rid + r), acc, n, has_cols);
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          float acc[C] = {};
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (c[4 * r + j] >= 0) add_cols<C>(acc, v[4 * r + j]);
-          put_row<OV, C>(a, out_lane, __ldg(rid + r), acc, n, has_cols);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) c[u] = cn[u];
+      for (int u = 0; u < B; ++u) c[u] = cn[u];
     }
     pos = npos;
     k = kn;
@@ -754,7 +762,7 @@ int build_plan(eppgcn_tile_plan **out_plan, void *dev_buf, size_t dev_bytes, con
   return EPP_OK;
 }
 
-template <int OV, int C>
+template <int OV, int C, int B>
 int launch_tiles(TileArgs &a, cudaStream_t s) {
   int num_sms = 0;
   if (const int rc = device_sm_count(&num_sms); rc != EPP_OK) return rc;
@@ -764,14 +772,14 @@ int launch_tiles(TileArgs &a, cudaStream_t s) {
   for (int k = 0; k < a.t.count; ++k) {
     const int w = a.t.width[k];
     a.t.tile_begin[k] = static_cast<int>(tiles);
-    tiles += (a.t.rank_off[k + 1] - a.t.rank_off[k]) / (G * (w >= 8 ? 1 : 8 / w));
+    tiles += (a.t.rank_off[k + 1] - a.t.rank_off[k]) / (G * (w >= B ? 1 : B / w));
   }
   for (int k = a.t.count; k <= kMaxClasses; ++k) a.t.tile_begin[k] = static_cast<int>(tiles);
   a.num_tiles = static_cast<int>(tiles);
   long long blocks = ceil_div_ll(tiles, kTileThreads / kWarp);
-  const long long cap = static_cast<long long>(num_sms) * TileResident<C>::blocks;
+  const long long cap = static_cast<long long>(num_sms) * kTileResident;
   if (blocks > cap) blocks = cap;
-  tiled_spmm_kernel<OV, C><<<static_cast<unsigned>(blocks), kTileThreads, 0, s>>>(a);
+  tiled_spmm_kernel<OV, C, B><<<static_cast<unsigned>(blocks), kTileThreads, 0, s>>>(a);
   EPP_CHECK_LAUNCH("tiled_spmm_kernel");
   return EPP_OK;
 }
@@ -867,9 +875,11 @@ static int run_tiles(float *out, long long out_ld, const float *src, long long s
   EPP_REQUIRE(src, "null pointer");
   EPP_REQUIRE(src_ld % 4 == 0 && src_ld >= (dim + 3) / 4 * 4 && src_ld <= 0x3fffffffLL && aligned(src, 16),
               "source rows must be 16-byte aligned and padded to a multiple of 4 floats");
-  // Eight columns per lane (one 32-byte load each) where a row is longer than 32: half the instructions per row, 64 columns
-  // 672 -> 651 us on 34.6 M edges; with 16 columns the smaller number of resident warps costs more (254 -> 276 us).
-  const int cols = dim > 32 && src_ld % 8 == 0 && aligned(src, 32) ? 8 : 4;
+  // Eight columns per lane (one 32-byte load each), four edges in flight, from 25 columns on: half the instructions per
+  // edge at the same number of resident warps.  us with four and with eight columns per lane: 34.6 M edges x 64 columns 672
+  // and 530 (602 with eight edges in flight and fewer warps), x 32 321 and 281, 10.7 M edges x 32 140 and 124; but 35.6 M
+  // edges x 16 225 and 265, x 24 350 and 363.
+  const int cols = dim > 24 && src_ld % 8 == 0 && aligned(src, 32) ? 8 : 4;
   for (int col0 = 0; col0 < dim; col0 += 128) {
     TileArgs a{};
     a.out = out + col0; a.out_ld = out_ld; a.src = src + col0; a.src_ld = src_ld;
@@ -879,8 +889,8 @@ static int run_tiles(float *out, long long out_ld, const float *src, long long s
     a.accumulate = accumulate;
     a.mark = take_mark();
     int rc;
-    if (cols == 8) rc = ovec == 4 ? launch_tiles<4, 8>(a, s) : ovec == 2 ? launch_tiles<2, 8>(a, s) : launch_tiles<1, 8>(a, s);
-    else rc = ovec == 4 ? launch_tiles<4, 4>(a, s) : ovec == 2 ? launch_tiles<2, 4>(a, s) : launch_tiles<1, 4>(a, s);
+    if (cols == 8) rc = ovec == 4 ? launch_tiles<4, 8, 4>(a, s) : ovec == 2 ? launch_tiles<2, 8, 4>(a, s) : launch_tiles<1, 8, 4>(a, s);
+    else rc = ovec == 4 ? launch_tiles<4, 4, 8>(a, s) : ovec == 2 ? launch_tiles<2, 4, 8>(a, s) : launch_tiles<1, 4, 8>(a, s);
     if (rc != EPP_OK) return rc;
   }
   return EPP_OK;

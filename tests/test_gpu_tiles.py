@@ -69,6 +69,15 @@ def test_forward_dims(cuda, graph, dim):
     assert_close(got, want, 2e-5, 2e-6, what=f"tiled forward {graph} dim {dim}")
 
 
+@pytest.mark.parametrize("graph", ["hubs", "loops", "sparse", "wide"])
+@pytest.mark.parametrize("dim", [24, 25, 28, 31, 39, 47, 121, 136])
+def test_rows_padded_to_32_bytes(cuda, graph, dim):
+    """Eight columns per lane from 25 columns on; a last piece of 1 .. 8 columns."""
+    indptr, indices = random_csr(**GRAPHS[graph])
+    got, want, _ = forward_case(cuda, indptr, indices, dim, pad_to=8)
+    assert_close(got, want, 2e-5, 2e-6, what=f"tiled forward {graph} dim {dim}, rows of {(dim + 7) // 8 * 8}")
+
+
 def test_plan_counts(cuda):
     indptr, indices = random_csr(**GRAPHS["hubs"])
     n = len(indptr) - 1

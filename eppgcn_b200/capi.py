@@ -50,6 +50,12 @@ SIGNATURES = {
     "eppgcn_tile_plan_missing": (_I, [_P, _P, _P, _P, _P, _P]),
     "eppgcn_zero_rows": (_I, [_P, _LL, _I, _P, _I, _P]),
     "eppgcn_weight_grad_add": (_I, [_P, _P, _LL, _P, _LL, _P, _I, _I, _I, _I, _P]),
+    "eppgcn_spmm_tiles_relu": (_I, [_P, _LL, _P, _LL, _P, _P, _I, _P]),
+    "eppgcn_spmm_tiles_gated": (_I, [_P, _LL, _P, _LL, _P, _P, _P, _LL, _I, _I, _P]),
+    "eppgcn_tile_plan_from_ids_of": (_I, [_P, _P, _SZ, _P, _P, _LL, _I, _I, _P, _P, _P]),
+    "eppgcn_tile_plan_edge_hashes": (_I, [_P, _P, _P, _P]),
+    "eppgcn_head_supported": (_I, [_I, _I]),
+    "eppgcn_head_step": (_I, [_P, _LL, _P, _P, _P, _LL, _P, _P, _P, _P, _P, _I, _I, _I, _P]),
     "eppgcn_masked_nll": (_I, [_P, _LL, _P, _P, _LL, _P, _P, _P, _P, _I, _I, _P]),
     "eppgcn_adam_step": (_I, [_I, _P, _P, _P, _P, _P, _P, _P, C.c_double, C.c_double, C.c_double, C.c_double, _P]),
     "eppgcn_mean_grads": (_I, [_P, _I, _P, _P, _P, _P, _P]),
@@ -208,6 +214,19 @@ def masked_nll(logits, labels, mask, used, scale=None):
     return grad[:, :c], sums
 
 
+def head_step(s, w, labels, mask, used, scale=None):
+    """``(gradient rows, dw, sums)`` of a last layer ``z = s @ w`` over aggregated rows, see ``eppgcn_head_step``."""
+    n, (k, c) = s.size(0), w.shape
+    grad = torch.zeros((n, (k + 7) // 8 * 8), dtype=torch.float32, device=s.device)
+    dw = torch.zeros_like(w)
+    sums = torch.zeros(2, dtype=torch.float64, device=s.device)
+    check(lib().eppgcn_head_step(grad.data_ptr(), grad.stride(0), dw.data_ptr(), sums.data_ptr(), s.data_ptr(),
+                                 _row_stride(s, "s"), _dev(w, torch.float32, "w"), _dev(labels, torch.int64, "labels"),
+                                 _dev(mask, torch.bool, "mask"), _dev(used, torch.uint8, "used"),
+                                 _dev(scale, torch.float32, "scale"), n, k, c, _stream()))
+    return grad[:, :k], dw, sums
+
+
 def weight_grad(x, d, plan=None):
     """``x.T @ d`` for a tall ``x [N, k]`` and ``d [N, dout]``; with a tile ``plan`` only over the
     rows that have edges in it (the other rows of ``d`` are zero by construction)."""
@@ -344,6 +363,28 @@ def spmm_tiles(src, plan, row_scale=None, out=None):
         _out_rows(out, n, dim, "out"), _row_stride(out, "out"), src.data_ptr(), ld, plan._handle,
         None if row_scale is None else _dev(row_scale, torch.float32, "row_scale"), dim, _stream()))
     return out
+
+
+def spmm_tiles_finished(src, plan, row_scale, gate=None, every_row=True, out=None):
+    """``y = spmm_tiles(src, plan, row_scale)`` as ``row_scale * relu(y)``, or with a gate as ``row_scale * y`` where the
+    gate is not zero; ``out``: rows padded to 4 floats."""
+    n, dim = plan.info["rows"], src.size(1)
+    if out is None:
+        out = torch.empty(n, (dim + 3) // 4 * 4, device=src.device, dtype=torch.float32)[:, :dim]
+    args = (out.data_ptr(), out.stride(0), src.data_ptr(), _row_stride(src, "src"), plan._handle,
+            _dev(row_scale, torch.float32, "row_scale"))
+    if gate is None:
+        check(lib().eppgcn_spmm_tiles_relu(*args, dim, _stream()))
+    else:
+        check(lib().eppgcn_spmm_tiles_gated(*args, gate.data_ptr(), gate.stride(0), dim, int(every_row), _stream()))
+    return out
+
+
+def edge_hashes(plan, of):
+    """The four sums of ``eppgcn_tile_plan_edge_hashes``."""
+    sums = torch.zeros(4, dtype=torch.int64, device="cuda")
+    check(lib().eppgcn_tile_plan_edge_hashes(plan._handle, of._handle, sums.data_ptr(), _stream()))
+    return sums.tolist()
 
 
 def spmm_tiles_add(src, plan, row_scale, out):

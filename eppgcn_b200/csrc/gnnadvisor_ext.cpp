@@ -104,6 +104,9 @@ struct Plan {
   mutable torch::Tensor missing;
   mutable void *missing_home = nullptr;
   mutable int missing_count = 0;
+  // whether this plan is the transposed of the rows of another (the one asked about last) that it gathers from
+  mutable std::weak_ptr<const Plan> forward;
+  mutable bool transposed = false;
   ~Plan() { eppgcn_tile_plan_destroy(handle); }
 };
 using PlanPtr = std::shared_ptr<const Plan>;
@@ -129,6 +132,25 @@ std::pair<torch::Tensor, int> missing_rows(const PlanPtr &plan, const PlanPtr &o
   return {plan->missing, plan->missing_count};
 }
 
+// Whether a path's plan holds, of the rows that it gathers from, exactly the edges that the graph's plan has, turned round
+// (always so on a symmetric graph).  Worked out at the first question (one synchronisation) from the plans' own edges,
+// which never change, and kept with the plan.
+bool transposed_rows(const PlanPtr &path, const PlanPtr &graph, void *stream) {
+  std::lock_guard<std::mutex> lock(path->mu);
+  if (path->forward.lock() != graph) {
+    auto sums = at::empty({4}, path->buffer.options());
+    used_on_current_stream(graph->buffer, graph->home);
+    epp_check(eppgcn_tile_plan_edge_hashes(path->handle, graph->handle,
+                                           reinterpret_cast<unsigned long long *>(sums.data_ptr<int64_t>()), stream),
+              "eppgcn_tile_plan_edge_hashes");
+    const auto host = sums.cpu();
+    const int64_t *h = host.data_ptr<int64_t>();
+    path->transposed = h[0] == h[2] && h[1] == h[3];
+    path->forward = graph;
+  }
+  return path->transposed;
+}
+
 struct PlanEntry {
   PlanKey key;
   PlanPtr plan;
@@ -143,7 +165,7 @@ class PlanCache {
   // Finds the plan of `key`, or builds it with `build(buffer_ptr, buffer_bytes, &plan)`.
   template <typename Build>
   PlanPtr get(const PlanKey &key, const torch::Tensor &key_a, const torch::Tensor &key_b,
-              int64_t edges, int64_t rows, int64_t sources, Build build) {
+              int64_t edges, int64_t rows, int64_t sources, Build build, const PlanPtr &graph = nullptr) {
     const auto opts = key_a.options();
     PlanEntry dropped;                 // given up after the lock: letting go of a tensor may wait for the interpreter's lock
     std::lock_guard<std::mutex> lock(mu_);
@@ -157,7 +179,8 @@ class PlanCache {
     auto plan = std::make_shared<Plan>();
     plan->buffer = at::empty({static_cast<int64_t>((bytes + 7) / 8)}, opts.dtype(at::kLong));
     plan->home = current_stream();
-    epp_check(build(plan->buffer.data_ptr(), bytes, &plan->handle), "eppgcn_tile_plan");
+    epp_check(build(plan->buffer.data_ptr(), bytes, plan.get()), "eppgcn_tile_plan");
+    plan->forward = graph;             // the build has looked whether the plan is transposed
     if (entries_.size() >= kCapacity) {
       size_t oldest = 0;
       for (size_t i = 1; i < entries_.size(); ++i)
@@ -202,24 +225,30 @@ PlanPtr forward_plan(const torch::Tensor &row_pointers, const torch::Tensor &col
   PlanKey key{row_pointers.data_ptr(), column_index.data_ptr(), row_pointers.numel(), column_index.numel(), n, e,
               static_cast<uint32_t>(row_pointers._version()), static_cast<uint32_t>(column_index._version()),
               row_pointers.get_device()};
-  return plan_cache().get(key, row_pointers, column_index, e, n, n, [&](void *buf, size_t bytes, eppgcn_tile_plan **plan) {
-    return eppgcn_tile_plan_from_csr(plan, buf, bytes, row_pointers.data_ptr<int>(), column_index.data_ptr<int>(),
+  return plan_cache().get(key, row_pointers, column_index, e, n, n, [&](void *buf, size_t bytes, Plan *plan) {
+    return eppgcn_tile_plan_from_csr(&plan->handle, buf, bytes, row_pointers.data_ptr<int>(), column_index.data_ptr<int>(),
                                      static_cast<int>(n), e, static_cast<int>(n), current_stream());
   });
 }
 
+// `graph`: the forward plan that transposed_rows will ask about, answered on the way where the plan is made.
 PlanPtr backward_plan(const torch::Tensor &id, const torch::Tensor &partPointer, const torch::Tensor &edgeList,
-                      int numParts, int64_t n) {
+                      int numParts, int64_t n, const PlanPtr &graph = nullptr) {
   // the path's edge count closes the part pointers; it is read once, when the plan is made
   PlanKey key{id.data_ptr(), edgeList.data_ptr(), id.numel(), partPointer.numel(), n, numParts,
               static_cast<uint32_t>(id._version()), static_cast<uint32_t>(edgeList._version()), id.get_device()};
-  return plan_cache().get(key, id, edgeList, id.numel(), n, n, [&](void *buf, size_t bytes, eppgcn_tile_plan **plan) {
+  return plan_cache().get(key, id, edgeList, id.numel(), n, n, [&](void *buf, size_t bytes, Plan *plan) {
     const int64_t valid = numParts > 0 ? partPointer[numParts].item<int>() : 0;
     TORCH_CHECK(valid >= 0 && valid <= id.numel() && valid <= edgeList.numel(),
                 "partPointer[numParts] is not an edge count of the compacted lists");
-    return eppgcn_tile_plan_from_ids(plan, buf, bytes, id.data_ptr<int>(), edgeList.data_ptr<int>(), valid,
-                                     static_cast<int>(n), static_cast<int>(n), current_stream());
-  });
+    int transposed = 0;
+    if (graph) used_on_current_stream(graph->buffer, graph->home);
+    const int rc = eppgcn_tile_plan_from_ids_of(&plan->handle, buf, bytes, id.data_ptr<int>(), edgeList.data_ptr<int>(), valid,
+                                                static_cast<int>(n), static_cast<int>(n), graph ? graph->handle : nullptr,
+                                                &transposed, current_stream());
+    plan->transposed = transposed != 0;
+    return rc;
+  }, graph);
 }
 
 // sum over the plan's edges of rows that already carry their source factor; destination factor `degrees`
@@ -550,22 +579,34 @@ void check_labels(const torch::Tensor &labels, const torch::Tensor &mask, int64_
   TORCH_CHECK(labels.numel() == n && mask.numel() == n, "labels and mask must have one entry per vertex");
 }
 
-PlanPtr path_plan(const LayerPath &path, int64_t n) {
+PlanPtr path_plan(const LayerPath &path, int64_t n, const PlanPtr &graph = nullptr) {
   const auto &[id, parts, edges, num_parts] = path;
   CHECK_INPUT(id); CHECK_INPUT(parts); CHECK_INPUT(edges);
   CHECK_I32(id); CHECK_I32(parts); CHECK_I32(edges);
   TORCH_CHECK(num_parts >= 0 && (num_parts == 0 || num_parts < parts.numel()),
               "partPointer must hold numParts + 1 entries");
-  return backward_plan(id, parts, edges, num_parts, n);
+  return backward_plan(id, parts, edges, num_parts, n, graph);
 }
 
-// One [N, d] matrix per layer, before its activation; all but a `dense_last` last one in rows padded to 32 bytes.
+// One [N, d] matrix per layer, before its activation; all but a `dense_last` last one in rows padded to 32 bytes.  With
+// `head`, which stops in front of the last layer's product, the last two are the source rows of its aggregation,
+// degrees * relu(result), and the aggregated rows.
 std::vector<torch::Tensor> run_forward(const torch::Tensor &x, const std::vector<torch::Tensor> &weights,
                                        const eppgcn_tile_plan *plan, const torch::Tensor &degrees, bool dense_last,
-                                       NetBuffers &buffers, void *stream, void *clock_stream) {
+                                       bool head, NetBuffers &buffers, void *stream, void *clock_stream) {
   const int64_t n = x.size(0);
   std::vector<torch::Tensor> acts;
   for (size_t i = 0; i < weights.size(); ++i) {
+    if (head && i + 1 == weights.size()) {
+      const int64_t k = weights[i].size(0), ld = padded_width(k);
+      auto out = buffers.rows(n, ld, x).narrow(1, 0, k);
+      ScopedMark t(0, 0, 0, clock_stream);
+      epp_check(eppgcn_spmm_tiles(out.data_ptr<float>(), ld, acts.back().data_ptr<float>(), ld, plan,
+                                  degrees.data_ptr<float>(), static_cast<int>(ld), stream),
+                "eppgcn_spmm_tiles");
+      acts.push_back(out);
+      break;
+    }
     const torch::Tensor &in = i ? acts.back() : x, &w = weights[i];
     const int64_t k = in.size(1), d = w.size(1), ld = padded_width(d), ld_out = dense_last && i + 1 == weights.size() ? d : ld;
     auto tmp = buffers.rows(n, ld, x);
@@ -577,12 +618,45 @@ std::vector<torch::Tensor> run_forward(const torch::Tensor &x, const std::vector
     auto out = buffers.rows(n, ld_out, x).narrow(1, 0, d);
     ScopedMark t(1, 0, 0, clock_stream);
     // padded rows are aggregated whole (their padding is zero on both sides): 16-byte stores, plain clearing
-    epp_check(eppgcn_spmm_tiles(out.data_ptr<float>(), ld_out, tmp.data_ptr<float>(), ld, plan,
-                                degrees.data_ptr<float>(), static_cast<int>(ld_out), stream),
+    auto *tiles = head && i + 2 == weights.size() ? eppgcn_spmm_tiles_relu : eppgcn_spmm_tiles;
+    epp_check(tiles(out.data_ptr<float>(), ld_out, tmp.data_ptr<float>(), ld, plan, degrees.data_ptr<float>(),
+                    static_cast<int>(ld_out), stream),
               "eppgcn_spmm_tiles");
     acts.push_back(out);
   }
   return acts;
+}
+
+// Whether the last layer's rows are aggregated before its product where only the results count: the gather is narrower.
+bool aggregates_first(const std::vector<torch::Tensor> &weights) {
+  return weights.size() >= 2 && padded_width(weights.back().size(0)) < padded_width(weights.back().size(1));
+}
+
+// The same in a training step, where loss and gradients of the last layer are then one kernel over the labelled rows.  Its
+// weight gradient is S^T g of the aggregated rows S instead of X^T A g: the same on the path's edges turned round, which
+// `transposed_rows` looks at.  A wider gather pays on small graphs, where one kernel for four counts.
+bool ends_in_head(const std::vector<torch::Tensor> &weights, int64_t n) {
+  if (weights.size() < 2) return false;
+  const int64_t k = weights.back().size(0), c = weights.back().size(1);
+  return c <= 64 && eppgcn_head_supported(static_cast<int>(k), static_cast<int>(c)) &&
+         (padded_width(k) <= padded_width(c) || n < 65536);
+}
+
+// Loss, the last layer's weight gradient (added to dw) and the gradient rows of its aggregation's source.
+torch::Tensor run_head(const torch::Tensor &s, const torch::Tensor &w, const torch::Tensor &labels, const torch::Tensor &mask,
+                       const torch::Tensor &degrees, const eppgcn_tile_plan *plan, float *dw, double *sums,
+                       NetBuffers &buffers, void *stream, void *clock_stream) {
+  const int64_t n = s.size(0), k = s.size(1), ld = padded_width(k);
+  const unsigned char *used = nullptr;
+  epp_check(eppgcn_tile_plan_used(plan, &used), "eppgcn_tile_plan_used");
+  auto grad = buffers.rows(n, ld, s);
+  ScopedMark t(2, 3, 0, clock_stream);
+  epp_check(eppgcn_head_step(grad.data_ptr<float>(), ld, dw, sums, s.data_ptr<float>(), s.stride(0), w.data_ptr<float>(),
+                             reinterpret_cast<const long long *>(labels.data_ptr<int64_t>()),
+                             reinterpret_cast<const unsigned char *>(mask.data_ptr<bool>()), used, degrees.data_ptr<float>(),
+                             static_cast<int>(n), static_cast<int>(k), static_cast<int>(w.size(1)), stream),
+            "eppgcn_head_step");
+  return grad.narrow(1, 0, k);
 }
 
 // Gradient rows of the loss, without the mean's divisor; adds to sums (float64[2]).
@@ -615,9 +689,36 @@ std::vector<int64_t> sum_offsets(const std::vector<torch::Tensor> &weights, int6
 // Adds the weight gradients' sums to `sums` (cleared; laid out by sum_offsets).
 void run_backward(torch::Tensor grad, const torch::Tensor &x, const std::vector<torch::Tensor> &weights,
                   const std::vector<torch::Tensor> &acts, const torch::Tensor &degrees, const std::vector<PlanPtr> &plans,
-                  float *sums, const std::vector<int64_t> &offsets, NetBuffers &buffers, void *stream, void *clock_stream) {
+                  float *sums, const std::vector<int64_t> &offsets, bool head, NetBuffers &buffers, void *stream,
+                  void *clock_stream) {
   const int64_t n = x.size(0);
+  auto clear_missing = [&](const torch::Tensor &rows_of, size_t i) {      // rows off path i that path i - 1 gathers
+    const auto [zeros, count] = missing_rows(plans[i], plans[i - 1], n, stream);
+    buffers.hold(zeros);
+    const int ld = static_cast<int>(rows_of.stride(0));
+    if (count)
+      epp_check(eppgcn_zero_rows(rows_of.data_ptr<float>(), ld, ld, zeros.data_ptr<int>(), count, stream), "eppgcn_zero_rows");
+  };
   for (size_t i = weights.size(); i-- > 0;) {
+    if (head && i + 1 == weights.size()) {
+      // grad already is the gradient of the aggregated rows: aggregated, gated and scaled in one pass
+      const int64_t k = weights[i].size(0), ld = padded_width(k);
+      const int *rows = nullptr;
+      int listed = 0;
+      epp_check(eppgcn_tile_plan_active_rows(plans[i]->handle, &rows, &listed), "eppgcn_tile_plan_active_rows");
+      const bool by_rows = n >= 65536 && listed < n / 4 * 3;
+      auto next = buffers.rows(n, ld, x).narrow(1, 0, k);
+      {
+        ScopedMark t(1, 2, static_cast<int>(i) + 1, clock_stream);
+        epp_check(eppgcn_spmm_tiles_gated(next.data_ptr<float>(), ld, grad.data_ptr<float>(), grad.stride(0), plans[i]->handle,
+                                          degrees.data_ptr<float>(), acts[i - 1].data_ptr<float>(), acts[i - 1].stride(0),
+                                          static_cast<int>(ld), by_rows ? 0 : 1, stream),
+                  "eppgcn_spmm_tiles_gated");
+      }
+      if (by_rows) clear_missing(next, i);
+      grad = next;
+      continue;
+    }
     const int64_t d = weights[i].size(1), ld = padded_width(d);
     auto d_prime = buffers.rows(n, ld, x).narrow(1, 0, d);
     // Rows off the path are zero in d' and in the next gradient.  Where they are many, neither is written nor read: the
@@ -645,16 +746,12 @@ void run_backward(torch::Tensor grad, const torch::Tensor &x, const std::vector<
     auto next = buffers.rows(n, ldi, x).narrow(1, 0, din);
     const float *gate = acts[i - 1].data_ptr<float>();
     if (by_rows) {
-      const auto [zeros, count] = missing_rows(plans[i], plans[i - 1], n, stream);
-      buffers.hold(zeros);
       epp_check(eppgcn_update_listed(next.data_ptr<float>(), ldi, d_prime.data_ptr<float>(), ld,
                                      weights[i].data_ptr<float>(), 1, d, degrees.data_ptr<float>(), gate,
                                      acts[i - 1].stride(0), 0, rows, listed, static_cast<int>(d), static_cast<int>(din),
                                      static_cast<int>(ldi - din), stream),
                 "eppgcn_update_listed");
-      if (count)
-        epp_check(eppgcn_zero_rows(next.data_ptr<float>(), ldi, static_cast<int>(ldi), zeros.data_ptr<int>(), count, stream),
-                  "eppgcn_zero_rows");
+      clear_missing(next, i);
     } else {
       update_rows(next.data_ptr<float>(), ldi, d_prime, ld, weights[i].data_ptr<float>(), 1, d, degrees.data_ptr<float>(), gate,
                   acts[i - 1].stride(0), false, n, d, din, ldi - din, buffers, stream);
@@ -689,8 +786,28 @@ std::vector<torch::Tensor> net_forward(torch::Tensor x, std::vector<torch::Tenso
   check_graph(x, row_pointers, column_index);
   c10::cuda::CUDAGuard guard(x.device());
   NetBuffers buffers;
-  return run_forward(aligned16(x), weights, forward_plan(row_pointers, column_index)->handle, degrees, true, buffers,
+  return run_forward(aligned16(x), weights, forward_plan(row_pointers, column_index)->handle, degrees, true, false, buffers,
                      current_stream(), current_stream());
+}
+
+// net_logits(x, weights, row_pointers, column_index, degrees) -> the last of net_forward's results
+torch::Tensor net_logits(torch::Tensor x, std::vector<torch::Tensor> weights, torch::Tensor row_pointers,
+                         torch::Tensor column_index, torch::Tensor degrees) {
+  check_net(x, weights, degrees);
+  check_graph(x, row_pointers, column_index);
+  c10::cuda::CUDAGuard guard(x.device());
+  NetBuffers buffers;
+  void *stream = current_stream();
+  const bool first = aggregates_first(weights);
+  const auto rows = run_forward(aligned16(x), weights, forward_plan(row_pointers, column_index)->handle, degrees, true, first,
+                                buffers, stream, stream).back();
+  if (!first) return rows;
+  const int64_t n = x.size(0), k = rows.size(1), d = weights.back().size(1);
+  auto out = at::empty({n, d}, x.options());
+  ScopedMark t(1, 1, 0, stream);
+  update_rows(out.data_ptr<float>(), d, rows, rows.stride(0), weights.back().data_ptr<float>(), d, 1, nullptr, nullptr, 0, false,
+              n, k, d, 0, buffers, stream);
+  return out;
 }
 
 // net_loss(logits, labels, mask, degrees, id, partPointer, edgeList, numParts of the last layer's path)
@@ -724,7 +841,7 @@ std::vector<torch::Tensor> net_backward(torch::Tensor grad, torch::Tensor sums, 
   const auto offsets = sum_offsets(weights, &total);
   auto dw_sums = at::zeros({total}, x.options());
   NetBuffers buffers;
-  run_backward(grad, aligned16(x), weights, acts, degrees, plans, dw_sums.data_ptr<float>(), offsets, buffers,
+  run_backward(grad, aligned16(x), weights, acts, degrees, plans, dw_sums.data_ptr<float>(), offsets, false, buffers,
                current_stream(), current_stream());
   return finish_step(weights, dw_sums.data_ptr<float>(), sums.data_ptr<double>(), offsets, current_stream());
 }
@@ -782,16 +899,21 @@ class NetStep {
     }
     plans_.clear();
     const PlanPtr plan = forward_plan(row_pointers, column_index);
-    for (const LayerPath &p : paths) plans_.push_back(path_plan(p, x.size(0)));
+    const bool may_head = ends_in_head(weights, x.size(0));
+    for (const LayerPath &p : paths)
+      plans_.push_back(path_plan(p, x.size(0), may_head && &p == &paths.back() ? plan : nullptr));
+    const bool head = may_head && transposed_rows(plans_.back(), plan, stream);
     auto all = [&](const torch::Tensor &x16, NetBuffers &buffers, void *on) {
       const cudaError_t e = cudaMemsetAsync(sums_.data_ptr(), 0, sizeof(float) * total_, static_cast<cudaStream_t>(on));
       TORCH_CHECK(e == cudaSuccess, "clearing the sums failed: ", cudaGetErrorString(e));
       float *sums = sums_.data_ptr<float>();
-      auto acts = run_forward(x16, weights, plan->handle, degrees, false, buffers, on, stream);
-      auto grad = run_loss(acts.back(), labels, mask, degrees, plans_.back()->handle, reinterpret_cast<double *>(sums),
-                           buffers, on);
+      auto acts = run_forward(x16, weights, plan->handle, degrees, false, head, buffers, on, stream);
+      auto *loss = reinterpret_cast<double *>(sums);
+      auto grad = head ? run_head(acts.back(), weights.back(), labels, mask, degrees, plans_.back()->handle,
+                                  sums + offsets_.back(), loss, buffers, on, stream)
+                       : run_loss(acts.back(), labels, mask, degrees, plans_.back()->handle, loss, buffers, on);
       acts.pop_back();
-      run_backward(grad, x16, weights, acts, degrees, plans_, sums, offsets_, buffers, on, stream);
+      run_backward(grad, x16, weights, acts, degrees, plans_, sums, offsets_, head, buffers, on, stream);
     };
     sums_ = at::empty({total_}, x.options());
     const auto x16 = aligned16(x);
@@ -1263,6 +1385,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("ours_backward_weight_only", &ours_backward_weight_only,
         "ours_backward without the input gradient: [empty, d_weight] (not in the reference)");
   m.def("net_forward", &net_forward, "forward of a stack of layers with ReLU between them (not in the reference)");
+  m.def("net_logits", &net_logits, "the last of net_forward's results (not in the reference)");
   m.def("net_loss", &net_loss, "masked mean NLL of the logits and its gradient rows (not in the reference)");
   m.def("net_backward", &net_backward, "loss and weight gradients of a stack of layers (not in the reference)");
   m.def("compact_back_edges", &compact_back_edges, "compact_back_edge of several layers at once (not in the reference)");

@@ -1,0 +1,439 @@
+// The last layer of a training step behind its aggregation, in one pass over the labelled rows:
+//
+//   z = s * W,   loss += logsumexp(z) - z[y],   g = softmax(z) - onehot(y),   dW += s^T * g,
+//   grad = scale * (g * W^T)
+//
+// where s is a row of the aggregated hidden matrix.  Aggregating first is the same sum in another order, at the width of
+// the hidden layer instead of the classes', and leaves the layer's products to the rows that the loss looks at; their
+// results stay in registers: the logits, their gradient and the layer's two gradient products cost no memory traffic
+// beyond s and grad.  As separate kernels (update of every row, loss, weight gradient, update of the path's rows) 16 -> 22
+// on 1.13 M rows, half of them labelled, took 258 us, 66 here; 16 -> 47 on 1 M rows, 30 % labelled, 334 and 71.  Bound by
+// instructions (1000 for 16 rows, issue slots 52 % busy at 16 warps per SM): 2.5 and 3.5 times the time of its bytes.
+//
+// A warp queues rows that have something to do (as the loss kernel does) and takes 16 at a time, the next 16 on their way.
+// Everything is in the fragment layouts of mma.m16n8k16 (mma_split.cuh): four lanes hold a row, lane t its features
+// 4t .. 4t + 3 of every 16 and classes 8j + 2t, + 1.  Probabilities come out where the next product reads its left
+// operand, and movmatrix turns rows into the contracted index for dW.
+#include "mma_split.cuh"
+
+namespace epp {
+namespace {
+
+constexpr int kHeadWarps = 8;
+constexpr long long kNoLabel = -100;          // nll_loss's ignore_index
+
+struct HeadArgs {
+  const float *s;
+  long long ld_s;
+  const float *w;                              // [k][classes]
+  const long long *labels;
+  const unsigned char *mask, *used;
+  const float *scale;
+  float *grad;
+  long long ld_grad;
+  float *dw;                                   // [k][classes], added to
+  double *sums;                                // {loss, labelled rows}, added to
+  int n, k, classes;
+  bool flags_vec;                              // four flags in one load
+  ClockMark mark;
+};
+
+// An 8 x 8 tile of 16-bit pieces with rows and columns exchanged.
+__device__ __forceinline__ unsigned transpose8(unsigned v) {
+  unsigned r;
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
+
+// KT pieces of 16 features, NT pieces of 8 classes; rows are looked over PER per lane at a time.
+template <int KT, int NT, int PER>
+__global__ void __launch_bounds__(kHeadWarps * 32, KT * NT <= 3 ? 2 : 1) head_kernel(const HeadArgs a) {
+  constexpr int CT = (NT + 1) / 2, F = 16 * KT;
+  constexpr int kUnlabelled = -1, kWrongLabel = -2;
+  __shared__ uint2 s_w[KT * NT * 96], s_wt[CT * 2 * KT * 96];      // fragments: [step][tile][piece][lane]
+  __shared__ float s_dw[F * 8 * NT];
+  __shared__ int2 s_queue[kHeadWarps][256];    // row | top bit where its gradient is wanted; whether it has a label
+  __shared__ double s_loss[kHeadWarps];
+  __shared__ int s_count[kHeadWarps];
+  if (blockIdx.x == 0 && threadIdx.x == 0) clock_begin(a.mark);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  auto weight = [&](int f, int c) { return f < a.k && c < a.classes ? __ldg(a.w + static_cast<long long>(f) * a.classes + c) : 0.f; };
+  for (int e = threadIdx.x; e < KT * NT * 32; e += blockDim.x) {
+    const int l = e % 32, j = e / 32 % NT, f = 16 * (e / 32 / NT) + 4 * (l & 3), c = 8 * j + (l >> 2);
+    uint2 *const at = s_w + e / 32 * 96 + l;
+    split3(weight(f, c), weight(f + 1, c), at[0].x, at[32].x, at[64].x);
+    split3(weight(f + 2, c), weight(f + 3, c), at[0].y, at[32].y, at[64].y);
+  }
+  for (int e = threadIdx.x; e < CT * 2 * KT * 32; e += blockDim.x) {
+    const int l = e % 32, j = e / 32 % (2 * KT), c = 16 * (e / 32 / (2 * KT)) + 2 * (l & 3), n8 = l >> 2;
+    const int f = 16 * (j / 2) + 4 * (n8 / 2) + n8 % 2 + 2 * (j % 2);      // two tiles share 16 features: a lane holds 4 in a row
+    uint2 *const at = s_wt + e / 32 * 96 + l;
+    split3(weight(f, c), weight(f, c + 1), at[0].x, at[32].x, at[64].x);
+    split3(weight(f, c + 8), weight(f, c + 9), at[0].y, at[32].y, at[64].y);
+  }
+  __syncthreads();
+
+  double loss = 0.0;
+  int count = 0;
+  float dw_top[KT][NT][1][4], dw_rest[KT][NT][1][4];
+#pragma unroll
+  for (int s = 0; s < KT; ++s)
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) dw_top[s][j][0][q] = dw_rest[s][j][0][q] = 0.f;
+
+  // 16 rows: of this lane rows g and g + 8, their entries in the queue, labels y, features v
+  auto half = [&](const int (&entry)[2], const long long (&label)[2], const float (&scale)[2], const float4 (&v)[2][KT]) {
+    int y[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      y[h] = label[h] == kNoLabel ? kUnlabelled : label[h] >= 0 && label[h] < a.classes ? static_cast<int>(label[h]) : kWrongLabel;
+    unsigned x[KT][1][3][4];
+#pragma unroll
+    for (int s = 0; s < KT; ++s) {
+      split3(v[0][s].x, v[0][s].y, x[s][0][0][0], x[s][0][1][0], x[s][0][2][0]);
+      split3(v[1][s].x, v[1][s].y, x[s][0][0][1], x[s][0][1][1], x[s][0][2][1]);
+      split3(v[0][s].z, v[0][s].w, x[s][0][0][2], x[s][0][1][2], x[s][0][2][2]);
+      split3(v[1][s].z, v[1][s].w, x[s][0][0][3], x[s][0][1][3], x[s][0][2][3]);
+    }
+    float z[NT][4];                            // rows g: 0, 1; g + 8: 2, 3
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      float top[1][4] = {}, rest[1][4] = {};
+#pragma unroll
+      for (int s = 0; s < KT; ++s) {
+        const uint2 *f = s_w + (s * NT + j) * 96 + lane;
+        multiply_split(top, rest, x[s], f[0], f[32], f[64]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        z[j][q] = top[0][q] + rest[0][q];
+        bad |= isnan(z[j][q]);
+      }
+    }
+    if (__any_sync(kFull, bad)) {              // an infinity has no pieces: as a plain sum gives it
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float *p = a.s + static_cast<long long>(entry[h] & 0x7fffffff) * a.ld_s;
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int c = 8 * j + 2 * t + q;
+            if (y[h] == kUnlabelled || c >= a.classes || !isnan(z[j][2 * h + q])) continue;
+            float sum = 0.f;
+#pragma unroll 1
+            for (int f = 0; f < a.k; ++f) sum = fmaf(__ldg(p + f), __ldg(a.w + static_cast<long long>(f) * a.classes + c), sum);
+            z[j][2 * h + q] = sum;
+          }
+      }
+    }
+    const int own = a.classes - 2 * t;         // of this lane, class 8j + q exists where 8j + q < own; only the last piece's may not
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int at = y[h] - 2 * t;             // the label is this lane's class 8j + q where at = 8j + q
+      float top = -INFINITY, sum = 0.f, picked = 0.f;
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          float &e = z[j][2 * h + q];
+          if (j == NT - 1 && 8 * j + q >= own) e = -INFINITY;
+          top = fmaxf(top, e);
+        }
+      top = fmaxf(top, __shfl_xor_sync(kFull, top, 1));
+      top = fmaxf(top, __shfl_xor_sync(kFull, top, 2));
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          float &e = z[j][2 * h + q];
+          e -= top;
+          if (8 * j + q == at) picked = e;
+          e = j == NT - 1 && 8 * j + q >= own ? 0.f : expf(e);
+          sum += e;
+        }
+      sum += __shfl_xor_sync(kFull, sum, 1);
+      sum += __shfl_xor_sync(kFull, sum, 2);
+      const bool labelled = y[h] != kUnlabelled;
+      if (labelled && y[h] >= 0 && (y[h] & 7) >> 1 == t) loss += static_cast<double>(logf(sum) - picked);
+      if (y[h] == kWrongLabel && t == 0) loss += static_cast<double>(NAN);
+      count += labelled && t == 0;
+      const float inv = 1.f / sum;
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          float &e = z[j][2 * h + q];
+          e = fmaf(e, inv, 8 * j + q == at ? -1.f : 0.f);
+        }
+      if (entry[h] >= 0 || !labelled) {        // no gradient of these, whatever their logits
+#pragma unroll
+        for (int j = 0; j < NT; ++j) z[j][2 * h] = z[j][2 * h + 1] = 0.f;
+      }
+    }
+    // g * W^T, and s^T * g with the rows as the contracted index
+    float out_top[2 * KT][1][4], out_rest[2 * KT][1][4];
+#pragma unroll
+    for (int j = 0; j < 2 * KT; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) out_top[j][0][q] = out_rest[j][0][q] = 0.f;
+    unsigned xt[KT][1][3][4];
+#pragma unroll
+    for (int s = 0; s < KT; ++s)
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        xt[s][0][p][0] = transpose8(x[s][0][p][0]);
+        xt[s][0][p][1] = transpose8(x[s][0][p][2]);
+        xt[s][0][p][2] = transpose8(x[s][0][p][1]);
+        xt[s][0][p][3] = transpose8(x[s][0][p][3]);
+      }
+#pragma unroll
+    for (int s = 0; s < CT; ++s) {
+      unsigned p[1][3][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int j = 2 * s + i;
+        if (j < NT) {
+          split3(z[j < NT ? j : 0][0], z[j < NT ? j : 0][1], p[0][0][2 * i], p[0][1][2 * i], p[0][2][2 * i]);
+          split3(z[j < NT ? j : 0][2], z[j < NT ? j : 0][3], p[0][0][2 * i + 1], p[0][1][2 * i + 1], p[0][2][2 * i + 1]);
+          uint2 b[3];
+#pragma unroll
+          for (int q = 0; q < 3; ++q) b[q] = make_uint2(transpose8(p[0][q][2 * i]), transpose8(p[0][q][2 * i + 1]));
+#pragma unroll
+          for (int f = 0; f < KT; ++f) multiply_split(dw_top[f][j < NT ? j : 0], dw_rest[f][j < NT ? j : 0], xt[f], b[0], b[1], b[2]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 3; ++q) p[0][q][2 * i] = p[0][q][2 * i + 1] = 0u;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 2 * KT; ++j) {
+        const uint2 *f = s_wt + (s * 2 * KT + j) * 96 + lane;
+        multiply_split(out_top[j], out_rest[j], p, f[0], f[32], f[64]);
+      }
+    }
+    bad = false;
+#pragma unroll
+    for (int j = 0; j < 2 * KT; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        out_top[j][0][q] += out_rest[j][0][q];
+        bad |= isnan(out_top[j][0][q]);
+      }
+    if (__any_sync(kFull, bad)) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float sum[2 * KT][2] = {};
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+#pragma unroll 1
+            for (int from = 0; from < 4; ++from) {
+              const float e = __shfl_sync(kFull, z[j][2 * h + q], (lane & ~3) | from);
+              const int c = 8 * j + 2 * from + q;
+              if (c >= a.classes) continue;
+#pragma unroll
+              for (int o = 0; o < 2 * KT; ++o)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                  const int f = 16 * (o / 2) + 4 * t + 2 * (o % 2) + i;
+                  if (f < a.k) sum[o][i] = fmaf(e, __ldg(a.w + static_cast<long long>(f) * a.classes + c), sum[o][i]);
+                }
+            }
+#pragma unroll
+        for (int o = 0; o < 2 * KT; ++o)
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            if (isnan(out_top[o][0][2 * h + i])) out_top[o][0][2 * h + i] = sum[o][i];
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (entry[h] >= 0) continue;
+      const long long row = entry[h] & 0x7fffffff;
+      const bool zero = y[h] == kUnlabelled;
+#pragma unroll
+      for (int s = 0; s < KT; ++s)
+        if (16 * s + 4 * t < a.ld_grad)
+          *reinterpret_cast<float4 *>(a.grad + row * a.ld_grad + 16 * s + 4 * t) =
+              zero ? make_float4(0.f, 0.f, 0.f, 0.f)
+                   : make_float4(out_top[2 * s][0][2 * h] * scale[h], out_top[2 * s][0][2 * h + 1] * scale[h],
+                                 out_top[2 * s + 1][0][2 * h] * scale[h], out_top[2 * s + 1][0][2 * h + 1] * scale[h]);
+    }
+  };
+
+  int2 *const queue = s_queue[warp];
+  const long long stride = static_cast<long long>(gridDim.x) * kHeadWarps * kWarp * PER;
+  long long base = (static_cast<long long>(blockIdx.x) * kHeadWarps + warp) * kWarp * PER;
+  int first = 0, queued = 0;                   // the queue: a ring of 256
+  unsigned f_used = 0, f_mask = 0;             // flags of the next rows, one or four per lane, on their way
+  auto flags = [&]() {
+    const long long r = base + PER * lane;
+    f_used = f_mask = 0;
+    if (PER == 4 && a.flags_vec && r + 4 <= a.n) {
+      f_used = __ldg(reinterpret_cast<const unsigned *>(a.used + r));
+      f_mask = __ldg(reinterpret_cast<const unsigned *>(a.mask + r));
+    } else {
+#pragma unroll
+      for (int i = 0; i < PER; ++i)
+        if (r + i < a.n) {
+          f_used |= static_cast<unsigned>(a.used[r + i]) << 8 * i;
+          f_mask |= static_cast<unsigned>(a.mask[r + i]) << 8 * i;
+        }
+    }
+  };
+  flags();
+  int entry[2][2];                             // two units of 16 rows: one in work, the next one's rows on their way
+  long long label[2][2];
+  float scale[2][2];
+  float4 v[2][2][KT];
+  bool have = false;
+#pragma unroll 1
+  while (true) {
+#pragma unroll 1
+    while (queued < 16 && base < a.n) {
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const bool wanted = f_used >> 8 * i & 0xff, labelled = f_mask >> 8 * i & 0xff;
+        const unsigned todo = __ballot_sync(kFull, wanted || labelled);
+        if (wanted || labelled)
+          queue[(first + queued + __popc(todo & ((1u << lane) - 1u))) & 255] =
+              make_int2(static_cast<int>(static_cast<unsigned>(base + PER * lane + i) | (wanted ? 0x80000000u : 0u)), labelled);
+        queued += __popc(todo);
+      }
+      base += stride;
+      flags();
+    }
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int2 e = 8 * h + g < queued ? queue[(first + 8 * h + g) & 255] : make_int2(0, 0);
+      const long long row = e.x & 0x7fffffff;
+      label[1][h] = e.y ? __ldg(a.labels + row) : kNoLabel;
+      const float *p = a.s + row * a.ld_s + 4 * t;
+#pragma unroll
+      for (int s = 0; s < KT; ++s)
+        v[1][h][s] = e.y && 16 * s + 4 * t < a.ld_s ? __ldg(reinterpret_cast<const float4 *>(p + 16 * s))
+                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+      scale[1][h] = e.x < 0 && a.scale ? __ldg(a.scale + row) : 1.f;
+      entry[1][h] = e.x;
+    }
+    __syncwarp();
+    if (have) half(entry[0], label[0], scale[0], v[0]);
+    have = queued > 0;
+    if (!have) break;
+    const int taken = min(queued, 16);
+    first += taken;
+    queued -= taken;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      entry[0][h] = entry[1][h];
+      label[0][h] = label[1][h];
+      scale[0][h] = scale[1][h];
+#pragma unroll
+      for (int s = 0; s < KT; ++s) v[0][h][s] = v[1][h][s];
+    }
+  }
+
+  // the block's loss and dW, warp after warp in one buffer
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) loss += __shfl_xor_sync(kFull, loss, off);
+  count = __reduce_add_sync(kFull, count);
+  if (lane == 0) {
+    s_loss[warp] = loss;
+    s_count[warp] = count;
+  }
+#pragma unroll 1
+  for (int w = 0; w < kHeadWarps; ++w) {
+    if (w == warp) {
+#pragma unroll
+      for (int s = 0; s < KT; ++s)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int pos = g + 8 * (q / 2), f = 16 * s + 4 * (pos % 8 / 2) + pos % 2 + 2 * (pos / 8);
+            float *const at = s_dw + f * (8 * NT) + 8 * j + 2 * t + q % 2;
+            *at = (w ? *at : 0.f) + (dw_top[s][j][0][q] + dw_rest[s][j][0][q]);
+          }
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < kHeadWarps; ++i) {
+      s_loss[0] += s_loss[i];
+      s_count[0] += s_count[i];
+    }
+    if (s_count[0]) {
+      atomicAdd(a.sums, s_loss[0]);
+      atomicAdd(a.sums + 1, static_cast<double>(s_count[0]));
+    }
+  }
+  for (int e = threadIdx.x; e < F * 8 * NT; e += blockDim.x) {
+    const int f = e / (8 * NT), c = e % (8 * NT);
+    if (f < a.k && c < a.classes) atomicAdd(a.dw + static_cast<long long>(f) * a.classes + c, s_dw[e]);
+  }
+  if (threadIdx.x == 0) clock_end(a.mark);
+}
+
+template <int KT, int NT>
+int launch_head(const HeadArgs &a, int sms, cudaStream_t s) {
+  // four flags per lane on large graphs, whose labelled rows are far between; on small ones as many warps as there are 32 rows
+  const long long most = static_cast<long long>(sms) * (KT * NT <= 3 ? 2 : 1), chunks = ceil_div_ll(a.n, kHeadWarps * kWarp);
+  if (chunks >= 8 * most) head_kernel<KT, NT, 4><<<static_cast<unsigned>(most), kHeadWarps * 32, 0, s>>>(a);
+  else head_kernel<KT, NT, 1><<<static_cast<unsigned>(chunks < most ? chunks : most), kHeadWarps * 32, 0, s>>>(a);
+  EPP_CHECK_LAUNCH("head_kernel");
+  return EPP_OK;
+}
+
+}  // namespace
+}  // namespace epp
+
+EPP_EXPORT int eppgcn_head_supported(int k, int classes) {
+  return k >= 1 && classes >= 1 && ((k <= 16 && classes <= 64) || (k <= 32 && classes <= 48));
+}
+
+EPP_EXPORT int eppgcn_head_step(float *grad, long long ld_grad, float *dw, double *sums, const float *s, long long ld_s,
+                                const float *w, const long long *labels, const unsigned char *mask, const unsigned char *used,
+                                const float *row_scale, int num_rows, int k, int num_classes, void *stream) {
+  using namespace epp;
+  EPP_REQUIRE(num_rows >= 0 && k >= 1 && num_classes >= 1, "negative size, k < 1 or no class");
+  if (!eppgcn_head_supported(k, num_classes)) {
+    set_error("eppgcn_head_step handles 16 columns and 64 classes or 32 and 48, got %d and %d", k, num_classes);
+    return EPP_ERR_TOO_LARGE;
+  }
+  if (num_rows == 0) return EPP_OK;
+  EPP_REQUIRE(grad && dw && sums && s && w && labels && mask && used, "null pointer");
+  EPP_REQUIRE(ld_s % 4 == 0 && ld_s >= (k + 3) / 4 * 4 && aligned(s, 16), "rows must be 16-byte aligned and padded to a multiple of 4 floats");
+  EPP_REQUIRE(ld_grad % 4 == 0 && ld_grad >= (k + 3) / 4 * 4 && aligned(grad, 16),
+              "gradient rows must be 16-byte aligned and padded to a multiple of 4 floats");
+  int sms = 148;
+  if (const int rc = device_sm_count(&sms); rc != EPP_OK) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const HeadArgs a{s, ld_s, w, labels, mask, used, row_scale, grad, ld_grad, dw, sums, num_rows, k, num_classes, aligned(mask, 4) && aligned(used, 4), take_mark()};
+  const int nt = (num_classes + 7) / 8;
+  if (k <= 16) {
+    switch (nt) {
+      case 1:  return launch_head<1, 1>(a, sms, st);
+      case 2:  return launch_head<1, 2>(a, sms, st);
+      case 3:  return launch_head<1, 3>(a, sms, st);
+      case 4:  return launch_head<1, 4>(a, sms, st);
+      case 5:  return launch_head<1, 5>(a, sms, st);
+      case 6:  return launch_head<1, 6>(a, sms, st);
+      case 7:  return launch_head<1, 7>(a, sms, st);
+      default: return launch_head<1, 8>(a, sms, st);
+    }
+  }
+  switch (nt) {
+    case 1:  return launch_head<2, 1>(a, sms, st);
+    case 2:  return launch_head<2, 2>(a, sms, st);
+    case 3:  return launch_head<2, 3>(a, sms, st);
+    case 4:  return launch_head<2, 4>(a, sms, st);
+    case 5:  return launch_head<2, 5>(a, sms, st);
+    default: return launch_head<2, 6>(a, sms, st);
+  }
+}

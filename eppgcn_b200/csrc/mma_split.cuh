@@ -27,12 +27,6 @@
 
 namespace epp {
 
-// max(a, b) that keeps a NaN, as relu does.
-__device__ __forceinline__ float max_nan(float a, float b) {
-  float r;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-  return r;
-}
 __device__ __forceinline__ float4 relu4(const float4 &v) {
   return make_float4(max_nan(v.x, 0.f), max_nan(v.y, 0.f), max_nan(v.z, 0.f), max_nan(v.w, 0.f));
 }

@@ -9,6 +9,13 @@ namespace epp {
 
 inline bool aligned(const void *p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) % bytes) == 0; }
 
+// max(a, b) that keeps a NaN, as relu does.
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 // Writes n (<= VEC) floats starting at p with the widest store `ovec` allows
 // (ovec = 4, 2 or 1: p and the row stride are aligned to that many floats).
 template <int VEC>

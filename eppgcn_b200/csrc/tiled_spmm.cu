@@ -96,9 +96,17 @@ struct TileArgs {
   int lanes;                      // lanes per row, ceil(dim / 4)
   int num_rows, num_sources;      // limits of the ids (looked at by the bounds-checking build only)
   int accumulate;                 // 1: every row is added to what `out` holds (red.global.add) instead of stored
+  const float *gate;              // with Finish::kGate
+  long long ld_gate;
   ClockMark mark;
   ClassTable t;
 };
+
+// What becomes of a row sum y = factor * sum: the row itself; the source row of the next layer's aggregation,
+// factor * relu(y); or, backward, the source row of the next gradient's, factor * y where the gate is not zero.  A pass
+// over the result of its own would read and write it once more: 25 - 30 us on 1.13 M rows of 64 bytes.  The rows that
+// are summed with atomics are finished by a kernel behind the tiles.
+enum Finish { kPlain = 0, kRelu = 1, kGate = 2 };
 
 // Bounds-checking build (-DEPP_DEBUG_BOUNDS), the stand-in for a memory checker: every source id and
 // every row id is compared with its limit before it is used; an offender is not dereferenced, the
@@ -140,24 +148,45 @@ __device__ __forceinline__ void add_cols(float (&acc)[C], const float (&v)[C]) {
   for (int i = 0; i < C; ++i) acc[i] += v[i];
 }
 
+template <int F>
+__device__ __forceinline__ void finish_piece(float (&y)[4], float scale, const float4 &gate) {
+  const float g[4] = {gate.x, gate.y, gate.z, gate.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (F == kRelu) y[i] = scale * max_nan(y[i], 0.f);
+    if (F == kGate) y[i] = g[i] == 0.f ? 0.f : scale * y[i];
+  }
+}
+
 // The first n of the lane's columns of a row sum, times the row's destination-side factor: a plain store, or an atomic
 // add for a piece of a hub row.
-template <int OV, int C>
-__device__ __forceinline__ void write_cols(float *dst, const float (&acc)[C], float scale, int n, bool add) {
+template <int OV, int C, int F>
+__device__ __forceinline__ void write_cols(const TileArgs &a, float *out_lane, int row, int fcol, const float (&acc)[C], float scale,
+                                           int n, bool add) {
+  float *const dst = out_lane + static_cast<long long>(row) * a.out_ld;
 #pragma unroll
   for (int h = 0; h < C; h += 4) {
     if (n <= h) break;
-    const float val[4] = {acc[h] * scale, acc[h + 1] * scale, acc[h + 2] * scale, acc[h + 3] * scale};
-    if (add) add_row<4>(dst + h, val, min(4, n - h), OV);
-    else store_row<4>(dst + h, val, min(4, n - h), OV);
+    float val[4] = {acc[h] * scale, acc[h + 1] * scale, acc[h + 2] * scale, acc[h + 3] * scale};
+    if (add) {
+      add_row<4>(dst + h, val, min(4, n - h), OV);
+      continue;
+    }
+    if (F == kGate) {
+      const float4 g = __ldg(reinterpret_cast<const float4 *>(a.gate + fcol + h + static_cast<long long>(row) * a.ld_gate));
+      finish_piece<F>(val, scale, g);
+    } else {
+      finish_piece<F>(val, scale, make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+    store_row<4>(dst + h, val, min(4, n - h), OV);
   }
 }
 // The rows of a narrow class's batch: PER rows of W neighbouring edges each, all of a sub-warp.  Ids and factors of all
 // rows are asked for at once, behind the batch's row loads.  One row after the other, each with two loads that depend on
 // each other in front of its store, made such a tile as long as a dozen batches: 13 M edges on 1.13 M vertices x 16
 // columns 118 us, 106 now; 35.6 M edges on 2.1 M vertices, half of them with their self loop only, 244 and 225.
-template <int OV, int C, int B, int W>
-__device__ __forceinline__ void close_narrow(const TileArgs &a, float *out_lane, const int *row_of, const int (&c)[B],
+template <int OV, int C, int B, int F, int W>
+__device__ __forceinline__ void close_narrow(const TileArgs &a, float *out_lane, int fcol, const int *row_of, const int (&c)[B],
                                              const float (&v)[B][C], int n, bool has_cols) {
   constexpr int PER = B / W;
   int rid[PER];
@@ -194,7 +223,7 @@ __device__ __forceinline__ void close_narrow(const TileArgs &a, float *out_lane,
       if (c[W * r + j] >= 0) add_cols<C>(acc, v[W * r + j]);
     if (rid[r] == -1 || !has_cols) continue;
     const int row = static_cast<int>(static_cast<unsigned>(rid[r]) & ~kAtomicBit);
-    write_cols<OV, C>(out_lane + static_cast<long long>(row) * a.out_ld, acc, scale[r], n, rid[r] < 0 || a.accumulate);
+    write_cols<OV, C, F>(a, out_lane, row, fcol, acc, scale[r], n, rid[r] < 0 || (F == kPlain && a.accumulate));
   }
 }
 
@@ -218,7 +247,7 @@ __device__ __forceinline__ TilePos locate(const ClassTable &t, int G, int tile, 
   return p;
 }
 
-template <int OV, int C, int B>
+template <int OV, int C, int B, int F>
 __global__ void __launch_bounds__(kTileThreads, kTileResident) tiled_spmm_kernel(const TileArgs a) {
   if (blockIdx.x == 0 && threadIdx.x == 0) clock_begin(a.mark);
   const int G = kWarp / a.lanes;               // rows (of the wide classes) per tile
@@ -298,16 +327,16 @@ __global__ void __launch_bounds__(kTileThreads, kTileResident) tiled_spmm_kernel
         for (int u = 0; u < B; ++u) c[u] = cn[u];
       }
       if (rid != -1 && has_cols) {
-        write_cols<OV, C>(out_lane + static_cast<long long>(row) * a.out_ld, acc, scale, n, rid < 0 || a.accumulate);
+        write_cols<OV, C, F>(a, out_lane, row, fcol, acc, scale, n, rid < 0 || (F == kPlain && a.accumulate));
       }
     } else {
       // narrow classes: rows of 1, 2 or (with a batch of 8) 4 slots, several in one batch
       gather();
       prefetch_next();
       const int *row_of = a.row_of + pos.rank;
-      if (pos.width == 1) close_narrow<OV, C, B, 1>(a, out_lane, row_of, c, v, n, has_cols);
-      else if (B == 4 || pos.width == 2) close_narrow<OV, C, B, 2>(a, out_lane, row_of, c, v, n, has_cols);
-      else close_narrow<OV, C, B, 4>(a, out_lane, row_of, c, v, n, has_cols);
+      if (pos.width == 1) close_narrow<OV, C, B, F, 1>(a, out_lane, fcol, row_of, c, v, n, has_cols);
+      else if (B == 4 || pos.width == 2) close_narrow<OV, C, B, F, 2>(a, out_lane, fcol, row_of, c, v, n, has_cols);
+      else close_narrow<OV, C, B, F, 4>(a, out_lane, fcol, row_of, c, v, n, has_cols);
 #pragma unroll
       for (int u = 0; u < B; ++u) c[u] = cn[u];
     }
@@ -333,6 +362,26 @@ __global__ void __launch_bounds__(256) zero_listed_rows_kernel(float *out, long 
     else if constexpr (W == 2) *reinterpret_cast<float2 *>(p) = make_float2(0.f, 0.f);
     else *p = 0.f;
   }
+}
+
+// Rows that were summed with atomics, once all of their pieces are in.
+template <int F>
+__global__ void __launch_bounds__(256) finish_rows_kernel(const TileArgs a, const int *__restrict__ rows, int count) {
+  const int quads = (a.dim + 3) / 4;
+  const long long total = static_cast<long long>(count) * quads;
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const long long row = __ldg(rows + i / quads);
+    const int col = static_cast<int>(i % quads) * 4;
+    float4 *const at = reinterpret_cast<float4 *>(a.out + row * a.out_ld + col);
+    float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (F == kGate) g = __ldg(reinterpret_cast<const float4 *>(a.gate + row * a.ld_gate + col));
+    const float4 t = *at;
+    float y[4] = {t.x, t.y, t.z, t.w};
+    finish_piece<F>(y, a.row_scale ? __ldg(a.row_scale + row) : 1.f, g);
+    *at = make_float4(y[0], y[1], y[2], y[3]);
+  }
+  if (threadIdx.x == 0) clock_end(a.mark);
 }
 
 // Class of a row (or of the remainder piece of a hub row) with `len` edges, as
@@ -654,10 +703,63 @@ PlanLayout plan_layout(long long num_edges, int num_rows, int num_sources) {
   return l;
 }
 
+// Sums over the edges of a plan of two hashes of (row, source), or of (source, row) for the rows that `only` names.
+__device__ __forceinline__ unsigned long long mix64(unsigned long long v) {       // the finaliser of MurmurHash3
+  v = (v ^ (v >> 33)) * 0xff51afd7ed558ccdULL;
+  v = (v ^ (v >> 33)) * 0xc4ceb9fe1a85ec53ULL;
+  return v ^ (v >> 33);
+}
+__global__ void __launch_bounds__(256) hash_edges_kernel(const int *__restrict__ slots, const int *__restrict__ row_of,
+                                                         const ClassTable t, long long count,
+                                                         const unsigned char *__restrict__ only, unsigned long long *sums) {
+  unsigned long long h0 = 0, h1 = 0;
+  int k = 0;
+  for (long long at = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4; at < count;
+       at += static_cast<long long>(gridDim.x) * blockDim.x * 4) {
+    while (k + 1 < t.count && at >= t.slot_off[k + 1]) ++k;
+    const int w = t.width[k];
+    const int4 ids = __ldg(reinterpret_cast<const int4 *>(slots + at));
+    const int c[4] = {ids.x, ids.y, ids.z, ids.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (c[q] < 0) continue;
+      const int row = static_cast<int>(static_cast<unsigned>(__ldg(row_of + t.rank_off[k] + (at + q - t.slot_off[k]) / w)) & ~kAtomicBit);
+      if (only && !only[row]) continue;
+      const unsigned long long e = only ? static_cast<unsigned long long>(c[q]) << 32 | static_cast<unsigned>(row)
+                                        : static_cast<unsigned long long>(row) << 32 | static_cast<unsigned>(c[q]);
+      h0 += mix64(e);
+      h1 += mix64(e + 0x9e3779b97f4a7c15ULL);
+    }
+  }
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) {
+    h0 += __shfl_xor_sync(kFull, h0, off);
+    h1 += __shfl_xor_sync(kFull, h1, off);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(sums, h0);
+    atomicAdd(sums + 1, h1);
+  }
+}
+
+int hash_edges(const eppgcn_tile_plan *plan, const eppgcn_tile_plan *of, unsigned long long *sums, cudaStream_t s) {
+  EPP_CUDA_TRY(cudaMemsetAsync(sums, 0, 4 * sizeof(unsigned long long), s));
+  for (int i = 0; i < 2; ++i) {
+    const eppgcn_tile_plan *p = i ? of : plan;
+    if (p->num_slots == 0) continue;
+    const long long blocks = std::min<long long>(ceil_div_ll(p->num_slots, 4 * 256), 148 * 8);
+    hash_edges_kernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(p->slots, p->row_of, p->table, p->num_slots,
+                                                                    i ? plan->used : nullptr, sums + 2 * i);
+    EPP_CHECK_LAUNCH("hash_edges_kernel");
+  }
+  return EPP_OK;
+}
+
 // Builds the plan from the bounds of the rows' edges in `col_dev`.  `ids`: the row of every edge, where the bounds
-// have yet to be found; else `row_ptr`.
+// have yet to be found; else `row_ptr`.  With `of`, *transposed is what eppgcn_tile_plan_edge_hashes tells of the two.
 int build_plan(eppgcn_tile_plan **out_plan, void *dev_buf, size_t dev_bytes, const int *row_ptr, const int *ids,
-               const int *col_dev, long long num_edges, int num_rows, int num_sources, cudaStream_t s) {
+               const int *col_dev, long long num_edges, int num_rows, int num_sources, cudaStream_t s,
+               const eppgcn_tile_plan *of = nullptr, int *transposed = nullptr) {
   const PlanLayout l = plan_layout(num_edges, num_rows, num_sources);
   if (dev_bytes < l.total) {
     set_error("plan buffer too small: %zu bytes given, %zu needed", dev_bytes, l.total);
@@ -753,7 +855,14 @@ int build_plan(eppgcn_tile_plan **out_plan, void *dev_buf, size_t dev_bytes, con
         col_dev, plan.seg_start, plan.seg_len, plan.slots, t, slot_off, plan.used, num_sources);
     EPP_CHECK_LAUNCH("fill_slots_kernel");
   }
+  unsigned long long sums[4] = {0};
+  if (of) {                                           // seg_start, at least 64 words, has served its purpose
+    auto *sums_dev = reinterpret_cast<unsigned long long *>(plan.seg_start);
+    if (const int rc = hash_edges(&plan, of, sums_dev, s); rc != EPP_OK) return rc;
+    EPP_CUDA_TRY(cudaMemcpyAsync(sums, sums_dev, sizeof(sums), cudaMemcpyDeviceToHost, s));
+  }
   EPP_CUDA_TRY(cudaStreamSynchronize(s));             // the plan may be used on any stream from here on
+  if (of) *transposed = sums[0] == sums[2] && sums[1] == sums[3];
   *out_plan = new (std::nothrow) eppgcn_tile_plan(plan);
   if (!*out_plan) {
     set_error("out of host memory");
@@ -762,7 +871,7 @@ int build_plan(eppgcn_tile_plan **out_plan, void *dev_buf, size_t dev_bytes, con
   return EPP_OK;
 }
 
-template <int OV, int C, int B>
+template <int OV, int C, int B, int F>
 int launch_tiles(TileArgs &a, cudaStream_t s) {
   int num_sms = 0;
   if (const int rc = device_sm_count(&num_sms); rc != EPP_OK) return rc;
@@ -779,7 +888,7 @@ int launch_tiles(TileArgs &a, cudaStream_t s) {
   long long blocks = ceil_div_ll(tiles, kTileThreads / kWarp);
   const long long cap = static_cast<long long>(num_sms) * kTileResident;
   if (blocks > cap) blocks = cap;
-  tiled_spmm_kernel<OV, C, B><<<static_cast<unsigned>(blocks), kTileThreads, 0, s>>>(a);
+  tiled_spmm_kernel<OV, C, B, F><<<static_cast<unsigned>(blocks), kTileThreads, 0, s>>>(a);
   EPP_CHECK_LAUNCH("tiled_spmm_kernel");
   return EPP_OK;
 }
@@ -809,14 +918,22 @@ EPP_EXPORT int eppgcn_tile_plan_from_csr(eppgcn_tile_plan **plan, void *dev_buf,
 EPP_EXPORT int eppgcn_tile_plan_from_ids(eppgcn_tile_plan **plan, void *dev_buf, size_t dev_bytes,
                                          const int *ids, const int *col_idx, long long num_edges, int num_rows,
                                          int num_sources, void *stream) {
+  return eppgcn_tile_plan_from_ids_of(plan, dev_buf, dev_bytes, ids, col_idx, num_edges, num_rows, num_sources, nullptr, nullptr,
+                                      stream);
+}
+
+EPP_EXPORT int eppgcn_tile_plan_from_ids_of(eppgcn_tile_plan **plan, void *dev_buf, size_t dev_bytes,
+                                            const int *ids, const int *col_idx, long long num_edges, int num_rows,
+                                            int num_sources, const eppgcn_tile_plan *of, int *transposed, void *stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   EPP_REQUIRE(plan && dev_buf && num_rows >= 0 && num_edges >= 0 && num_sources >= 0, "bad argument");
   EPP_REQUIRE(num_edges < (1LL << 31), "edge count exceeds int32");
   EPP_REQUIRE(reinterpret_cast<uintptr_t>(dev_buf) % 256 == 0, "plan buffer must be 256-byte aligned");
   EPP_REQUIRE(num_edges == 0 || (ids && col_idx), "null pointer");
+  EPP_REQUIRE(!of || (transposed && num_sources >= of->num_rows && of->num_sources >= num_rows), "the plans cover different vertices");
   // without an edge the list may be null: an empty stand-in says that these are ids, not offsets
   return build_plan(plan, dev_buf, dev_bytes, nullptr, ids ? ids : reinterpret_cast<const int *>(dev_buf), col_idx,
-                    num_edges, num_rows, num_sources, s);
+                    num_edges, num_rows, num_sources, s, of, transposed);
 }
 
 EPP_EXPORT int eppgcn_pack_scaled_rows(float *dst, long long dst_ld, const float *x, long long ldx,
@@ -868,9 +985,25 @@ EPP_EXPORT int eppgcn_tile_plan_used(const eppgcn_tile_plan *plan, const unsigne
   return EPP_OK;
 }
 
+// How the row sums are finished, and by what gate.
+struct FinishBy {
+  int how;
+  const float *gate;
+  long long ld_gate;
+};
+
+template <int F>
+static int launch_columns(TileArgs &a, int cols, int ovec, cudaStream_t s) {
+  if constexpr (F == kPlain) {
+    if (ovec == 2) return cols == 8 ? launch_tiles<2, 8, 4, F>(a, s) : launch_tiles<2, 4, 8, F>(a, s);
+    if (ovec == 1) return cols == 8 ? launch_tiles<1, 8, 4, F>(a, s) : launch_tiles<1, 4, 8, F>(a, s);
+  }
+  return cols == 8 ? launch_tiles<4, 8, 4, F>(a, s) : launch_tiles<4, 4, 8, F>(a, s);
+}
+
 // The tile launches of one aggregation (one unless the row is wider than 128 columns).
 static int run_tiles(float *out, long long out_ld, const float *src, long long src_ld, const eppgcn_tile_plan *plan,
-                     const float *row_scale, int dim, int ovec, int accumulate, cudaStream_t s) {
+                     const float *row_scale, int dim, int ovec, int accumulate, const FinishBy &finish, cudaStream_t s) {
   if (plan->num_ranks == 0) return EPP_OK;
   EPP_REQUIRE(src, "null pointer");
   EPP_REQUIRE(src_ld % 4 == 0 && src_ld >= (dim + 3) / 4 * 4 && src_ld <= 0x3fffffffLL && aligned(src, 16),
@@ -887,18 +1020,25 @@ static int run_tiles(float *out, long long out_ld, const float *src, long long s
     a.dim = dim - col0 < 128 ? dim - col0 : 128; a.lanes = lanes_for_dim(a.dim, cols); a.t = plan->table;
     a.num_rows = plan->num_rows; a.num_sources = plan->num_sources;
     a.accumulate = accumulate;
+    a.gate = finish.gate ? finish.gate + col0 : nullptr; a.ld_gate = finish.ld_gate;
     a.mark = take_mark();
-    int rc;
-    if (cols == 8) rc = ovec == 4 ? launch_tiles<4, 8, 4>(a, s) : ovec == 2 ? launch_tiles<2, 8, 4>(a, s) : launch_tiles<1, 8, 4>(a, s);
-    else rc = ovec == 4 ? launch_tiles<4, 4, 8>(a, s) : ovec == 2 ? launch_tiles<2, 4, 8>(a, s) : launch_tiles<1, 4, 8>(a, s);
+    const int rc = finish.how == kRelu   ? launch_columns<kRelu>(a, cols, ovec, s)
+                   : finish.how == kGate ? launch_columns<kGate>(a, cols, ovec, s)
+                                         : launch_columns<kPlain>(a, cols, ovec, s);
     if (rc != EPP_OK) return rc;
+    if (finish.how == kPlain || plan->hub_rows == 0) continue;
+    const long long blocks = std::min<long long>(ceil_div_ll(static_cast<long long>(plan->hub_rows) * ((a.dim + 3) / 4), 256), 148 * 8);
+    a.mark = take_mark();
+    if (finish.how == kRelu) finish_rows_kernel<kRelu><<<static_cast<unsigned>(blocks), 256, 0, s>>>(a, plan->zero_rows, plan->hub_rows);
+    else finish_rows_kernel<kGate><<<static_cast<unsigned>(blocks), 256, 0, s>>>(a, plan->zero_rows, plan->hub_rows);
+    EPP_CHECK_LAUNCH("finish_rows_kernel");
   }
   return EPP_OK;
 }
 
 // `every_row`: rows without edges become zero; else they are left as they are.
 static int aggregate(float *out, long long out_ld, const float *src, long long src_ld, const eppgcn_tile_plan *plan,
-                     const float *row_scale, int dim, bool every_row, void *stream) {
+                     const float *row_scale, int dim, bool every_row, const FinishBy &finish, void *stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   EPP_REQUIRE(plan, "null plan");
   EPP_REQUIRE(dim >= 1, "dim < 1");
@@ -910,6 +1050,11 @@ static int aggregate(float *out, long long out_ld, const float *src, long long s
   int ovec = 1;
   if (out_ld % 4 == 0 && aligned(out, 16)) ovec = 4;
   else if (out_ld % 2 == 0 && aligned(out, 8)) ovec = 2;
+  if (finish.how != kPlain) {
+    EPP_REQUIRE(ovec == 4 && out_ld >= (dim + 3) / 4 * 4, "finished rows must be 16-byte aligned and padded to a multiple of 4 floats");
+    EPP_REQUIRE(finish.how != kGate || (finish.gate && finish.ld_gate % 4 == 0 && finish.ld_gate >= (dim + 3) / 4 * 4 &&
+                                        aligned(finish.gate, 16)), "gate rows must be like the result's");
+  }
   // rows without edges and rows that are summed with atomics start from zero
   const int num_zero = every_row ? plan->num_zero : plan->hub_rows;      // hub rows come first in the list
   if (every_row && plan->zero_all) {
@@ -927,17 +1072,28 @@ static int aggregate(float *out, long long out_ld, const float *src, long long s
     else zero_listed_rows_kernel<1><<<g, 256, 0, s>>>(out, out_ld, dim, plan->zero_rows, num_zero, mark);
     EPP_CHECK_LAUNCH("zero_listed_rows_kernel");
   }
-  return run_tiles(out, out_ld, src, src_ld, plan, row_scale, dim, ovec, 0, s);
+  return run_tiles(out, out_ld, src, src_ld, plan, row_scale, dim, ovec, 0, finish, s);
 }
 
 EPP_EXPORT int eppgcn_spmm_tiles(float *out, long long out_ld, const float *src, long long src_ld,
                                  const eppgcn_tile_plan *plan, const float *row_scale, int dim, void *stream) {
-  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, true, stream);
+  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, true, {kPlain, nullptr, 0}, stream);
 }
 
 EPP_EXPORT int eppgcn_spmm_tiles_active(float *out, long long out_ld, const float *src, long long src_ld,
                                         const eppgcn_tile_plan *plan, const float *row_scale, int dim, void *stream) {
-  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, false, stream);
+  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, false, {kPlain, nullptr, 0}, stream);
+}
+
+EPP_EXPORT int eppgcn_spmm_tiles_relu(float *out, long long out_ld, const float *src, long long src_ld,
+                                      const eppgcn_tile_plan *plan, const float *row_scale, int dim, void *stream) {
+  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, true, {kRelu, nullptr, 0}, stream);
+}
+
+EPP_EXPORT int eppgcn_spmm_tiles_gated(float *out, long long out_ld, const float *src, long long src_ld,
+                                       const eppgcn_tile_plan *plan, const float *row_scale, const float *gate,
+                                       long long ld_gate, int dim, int every_row, void *stream) {
+  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, every_row != 0, {kGate, gate, ld_gate}, stream);
 }
 
 // Rows that `of` names as sources and `plan` has no edge for.
@@ -971,6 +1127,14 @@ EPP_EXPORT int eppgcn_tile_plan_missing(const eppgcn_tile_plan *plan, const eppg
   return EPP_OK;
 }
 
+EPP_EXPORT int eppgcn_tile_plan_edge_hashes(const eppgcn_tile_plan *plan, const eppgcn_tile_plan *of,
+                                            unsigned long long *sums_dev, void *stream) {
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  EPP_REQUIRE(plan && of && sums_dev, "null pointer");
+  EPP_REQUIRE(plan->num_sources >= of->num_rows && of->num_sources >= plan->num_rows, "the plans cover different vertices");
+  return hash_edges(plan, of, sums_dev, s);
+}
+
 EPP_EXPORT int eppgcn_zero_rows(float *out, long long out_ld, int dim, const int *rows, int count, void *stream) {
   EPP_REQUIRE(count >= 0 && dim >= 1 && out_ld >= dim, "bad size");
   if (count == 0) return EPP_OK;
@@ -995,7 +1159,7 @@ EPP_EXPORT int eppgcn_spmm_tiles_add(float *out, long long out_ld, const float *
   int ovec = 1;
   if (out_ld % 4 == 0 && aligned(out, 16)) ovec = 4;
   else if (out_ld % 2 == 0 && aligned(out, 8)) ovec = 2;
-  return run_tiles(out, out_ld, src, src_ld, plan, row_scale, dim, ovec, 1, s);
+  return run_tiles(out, out_ld, src, src_ld, plan, row_scale, dim, ovec, 1, {kPlain, nullptr, 0}, s);
 }
 
 EPP_EXPORT int eppgcn_debug_status(int *out4, int reset) {

@@ -94,8 +94,7 @@ class Net(torch.nn.Module):
         if not torch.is_grad_enabled() and (isBackModeNet or not isFirstIter):
             weights = self.native_weights(x)
             if weights is not None:
-                return GNNA.net_forward(x, weights, inputInfo.row_pointers, inputInfo.column_index,
-                                        inputInfo.degrees)[-1]
+                return GNNA.net_logits(x, weights, inputInfo.row_pointers, inputInfo.column_index, inputInfo.degrees)
         for i, conv in enumerate(self.convs):
             info = inputInfo.set_input() if i == 0 else inputInfo.set_hidden()
             x = conv(x, info, mask_props[i], back_props[i], isFirstIter, isBackModeNet)

@@ -171,6 +171,23 @@ int eppgcn_spmm_tiles(float *out, long long out_ld, const float *src, long long 
 /* eppgcn_spmm_tiles without clearing the rows that have no edge (they keep what they hold). */
 int eppgcn_spmm_tiles_active(float *out, long long out_ld, const float *src, long long src_ld,
                              const eppgcn_tile_plan *plan, const float *row_scale, int dim, void *stream);
+/* eppgcn_spmm_tiles whose rows y = row_scale * sum leave finished: as the source rows of a next aggregation,
+ * row_scale * relu(y); or, backward, row_scale * y where gate != 0 and zero elsewhere (rows without an edge are cleared
+ * with every_row != 0).  16-byte aligned result and gate rows, padded to a multiple of 4 floats. */
+int eppgcn_spmm_tiles_relu(float *out, long long out_ld, const float *src, long long src_ld,
+                           const eppgcn_tile_plan *plan, const float *row_scale, int dim, void *stream);
+int eppgcn_spmm_tiles_gated(float *out, long long out_ld, const float *src, long long src_ld,
+                            const eppgcn_tile_plan *plan, const float *row_scale, const float *gate, long long ld_gate,
+                            int dim, int every_row, void *stream);
+/* sums_dev[0..1]: two 64-bit hash sums over the edges (row, source) of `plan`; sums_dev[2..3]: the same over the edges of
+ * `of` taken as (source, row), of the rows that `plan` names as sources.  Equal pairs: what `plan` gathers from a row,
+ * `of` gathers into it -- `plan` is the transposed of those rows of `of` (up to hash collisions, 2^-64 each). */
+int eppgcn_tile_plan_edge_hashes(const eppgcn_tile_plan *plan, const eppgcn_tile_plan *of, unsigned long long *sums_dev,
+                                 void *stream);
+/* eppgcn_tile_plan_from_ids that answers this question at once: *transposed = whether the pairs are equal. */
+int eppgcn_tile_plan_from_ids_of(eppgcn_tile_plan **plan, void *dev_buf, size_t dev_bytes,
+                                 const int *ids, const int *col_idx, long long num_edges, int num_rows,
+                                 int num_sources, const eppgcn_tile_plan *of, int *transposed, void *stream);
 /* The rows that the edges of `of` name as sources and that have no edge in `plan` (both over the same vertices), in any
  * order: what a step over the active rows of `plan` leaves out of the input of an aggregation over `of`.
  * flags: num_rows bytes of scratch, rows: num_rows ints, count_dev: one int. */
@@ -284,6 +301,15 @@ int eppgcn_update_listed(float *out, long long ld_out, const float *x, long long
                          int pad_cols, void *stream);
 int eppgcn_weight_grad_add(float *dw, const float *x, long long ldx, const float *d, long long ldd,
                            const int *rows, int num_rows, int k, int dout, int relu_x, void *stream);
+/* eppgcn_head_step: loss and gradients of a last layer z = s * w whose rows s are aggregated already, for k <= 16 and up
+ *   to 64 classes or k <= 32 and up to 48 (eppgcn_head_supported): adds {sum, count} to sums like eppgcn_masked_nll, the
+ *   weight's gradient sums over labelled rows with used[r] to dw [k][classes], and writes row_scale[r] * (dz * w^T) into
+ *   the rows r of grad with used[r] (zero without a label).  s and grad: rows of a multiple of 4 floats, 16-byte
+ *   aligned, zeros beyond k in s. */
+int eppgcn_head_supported(int k, int classes);
+int eppgcn_head_step(float *grad, long long ld_grad, float *dw, double *sums, const float *s, long long ld_s,
+                     const float *w, const long long *labels, const unsigned char *mask, const unsigned char *used,
+                     const float *row_scale, int num_rows, int k, int num_classes, void *stream);
 int eppgcn_masked_nll(float *grad, long long grad_ld, double *sums, const float *logits, long long ld,
                       const long long *labels, const unsigned char *mask, const unsigned char *used,
                       const float *row_scale, int num_rows, int num_classes, void *stream);

@@ -1,0 +1,131 @@
+"""The last layer of a training step as one kernel, and the aggregations that finish their rows, against float64."""
+import numpy as np
+import pytest
+import torch
+
+from eppgcn_b200 import capi, graphs
+from tests.helpers import degrees_of, random_csr, t
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(n, k, cuda, gen):
+    return torch.zeros(n, (k + 7) // 8 * 8, device=cuda)[:, :k].copy_(torch.randn(n, k, device=cuda, generator=gen))
+
+
+@pytest.mark.parametrize("n,k,classes", [(1, 1, 1), (15, 7, 3), (33, 16, 8), (2708, 16, 7), (4097, 16, 22), (3000, 9, 33),
+                                         (5001, 16, 47), (700, 16, 64), (1000, 17, 9), (3333, 32, 32), (5000, 32, 48),
+                                         (640_003, 16, 22), (320_001, 16, 47), (330_000, 32, 32)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_head_step(cuda, n, k, classes, offset):
+    """Ragged units of 16 rows, columns and classes; rows with a label, a gradient, both and neither; flags at odd addresses.
+    Bounds: a logit's sum of k products and a gradient's of the classes', 2^-23 each, in front of probabilities below 1."""
+    gen = torch.Generator(device=cuda).manual_seed(n + classes)
+    s, w = _rows(n, k, cuda, gen), torch.randn(k, classes, device=cuda, generator=gen)
+    y = torch.randint(classes, (n,), device=cuda, generator=gen)
+    y[::7] = -100                                      # ignored, as nll_loss does
+    mask = (torch.rand(n + offset, device=cuda, generator=gen) < 0.4)[offset:]
+    used = (torch.rand(n, device=cuda, generator=gen) < 0.6).to(torch.uint8)
+    scale = torch.rand(n, device=cuda, generator=gen) + 0.5
+    grad, dw, sums = capi.head_step(s, w, y, mask, used, scale)
+    labelled = mask & (y >= 0)
+    sd, wd = s.double(), w.double()
+    logp = torch.log_softmax(sd @ wd, 1)
+    loss = -logp.gather(1, y.clamp(min=0)[:, None])[labelled, 0].sum().item()
+    assert sums[1].item() == int(labelled.sum()) and abs(sums[0].item() - loss) <= 2e-6 * max(1.0, abs(loss))
+    g = logp.exp()
+    g[torch.arange(n, device=cuda), y.clamp(min=0)] -= 1.0
+    g *= (labelled & (used != 0))[:, None]
+    slack = 4e-6 * (sd.abs() @ wd.abs()).amax(1, keepdim=True) + 1e-6            # of a row's probabilities
+    want, mag = (g @ wd.T) * scale.double()[:, None], slack * wd.abs().sum(1) * scale.double()[:, None]
+    assert ((grad.double() - want).abs() <= mag + 1e-6).all()
+    want, mag = sd.T @ g, sd.abs().T @ (slack * (g.abs() + 1e-6)) + 2e-6 * (sd.abs().T @ g.abs())
+    assert ((dw.double() - want).abs() <= mag + 1e-6).all()
+    assert (grad.double() - (g @ wd.T) * scale.double()[:, None]).norm() <= 5e-7 * max(1.0, grad.double().norm())
+
+
+def test_head_step_leaves_other_rows_and_reports_wrong_labels(cuda):
+    n, k, c = 100, 16, 5
+    s, w = torch.randn(n, k, device=cuda), torch.randn(k, c, device=cuda)
+    y, mask = torch.zeros(n, dtype=torch.long, device=cuda), torch.ones(n, dtype=torch.bool, device=cuda)
+    used = torch.ones(n, dtype=torch.uint8, device=cuda)
+    used[::2] = 0
+    mask[50:] = False
+    grad, _, sums = capi.head_step(s, w, y, mask, used)
+    assert sums.isfinite().all() and (grad[::2] == 0).all() and (grad[51::2] == 0).all() and (grad[1:50:2] != 0).any(1).all()
+    y[3] = c                                           # no such class
+    assert capi.head_step(s, w, y, mask, used)[2][0].isnan()
+    assert capi.lib().eppgcn_head_supported(16, 65) == 0 and capi.lib().eppgcn_head_supported(33, 4) == 0
+
+
+@pytest.mark.parametrize("k,c", [(16, 22), (32, 7)])
+def test_head_step_with_infinite_weights(cuda, k, c):
+    """A class whose weights are -inf where s is positive has probability zero, not NaN; NaN stays NaN."""
+    n = 40
+    s, w = torch.rand(n, k, device=cuda) + 0.1, torch.randn(k, c, device=cuda)
+    y, ones = torch.ones(n, dtype=torch.long, device=cuda), torch.ones(n, dtype=torch.bool, device=cuda)
+    w[:, 2] = -float("inf")
+    grad, dw, sums = capi.head_step(s, w, y, ones, ones.to(torch.uint8))
+    p = torch.softmax(s.double() @ w.double(), 1)
+    want = -p[:, 1].log().sum()
+    assert abs(sums[0] - want) <= 1e-6 * want and dw.isfinite().all() and (dw[:, 2] == 0).all()
+    assert grad.isnan().all()                          # 0 * inf, as a plain product gives it
+    s[5, 0] = float("nan")
+    grad, dw, sums = capi.head_step(s, w, y, ones, ones.to(torch.uint8))
+    assert sums[0].isnan() and dw.isnan().all()
+
+
+@pytest.mark.parametrize("dim", [3, 8, 16, 24, 40])
+@pytest.mark.parametrize("graph", [dict(n=700, avg_deg=6.0, seed=3, hubs=3, hub_deg=650), dict(n=2000, avg_deg=1.0, seed=5, empty_frac=0.5)])
+def test_rows_leave_finished(cuda, dim, graph):
+    """relu and gate behind plain, narrow, empty and atomically added rows: the bits of the plain result, finished."""
+    indptr, indices = random_csr(**graph)
+    n, deg = len(indptr) - 1, t(degrees_of(indptr), cuda)
+    gen = torch.Generator(device=cuda).manual_seed(dim)
+    src = _rows(n, dim, cuda, gen)
+    gate = _rows(n, dim, cuda, gen).clamp(min=0)
+    full = torch.zeros(n, (dim + 7) // 8 * 8, device=cuda)
+    full[:, :dim] = gate
+    gate = full[:, :dim]
+    plan = capi.TilePlan.from_csr(t(indptr, cuda), t(indices, cuda))
+    y = capi.spmm_tiles(src, plan, deg)
+    close = torch.ones(n, dtype=torch.bool, device=cuda)
+    hubs = t(np.diff(indptr) > 64, cuda)               # summed in any order: a last bit of their largest term
+    for got, want in [(capi.spmm_tiles_finished(src, plan, deg), deg[:, None] * y.clamp(min=0)),
+                      (capi.spmm_tiles_finished(src, plan, deg, gate), deg[:, None] * y * (gate != 0))]:
+        assert torch.equal(got[~hubs], want[~hubs])
+        assert torch.allclose(got[hubs], want[hubs], rtol=1e-5, atol=1e-5)
+    some = torch.full((n, (dim + 3) // 4 * 4), 7.0, device=cuda)[:, :dim]
+    capi.spmm_tiles_finished(src, plan, deg, gate, every_row=False, out=some)
+    empty = t(np.diff(indptr) == 0, cuda)
+    assert (some[empty] == 7.0).all() and torch.equal(some[~empty & ~hubs], want[~empty & ~hubs]) and close.all()
+
+
+def test_edge_hashes_tell_transposed_lists(cuda):
+    rng = np.random.Generator(np.random.PCG64(1))
+    n = 3000
+    src, dst = rng.integers(0, n, 9000), rng.integers(0, n, 9000)
+    dst[::3] %= 4                                      # rows in many pieces
+    indptr, indices = graphs.csr_from_pairs(n, src, dst)
+    rows = np.repeat(np.arange(n), np.diff(indptr))
+    whole = capi.TilePlan.from_csr(t(indptr, cuda), t(indices, cuda))
+    mask = rng.random(n) < 0.2
+    on = mask[indices]
+    def path(keep):
+        return capi.TilePlan.from_ids(t(rows[keep].astype(np.int32), cuda), t(indices[keep], cuda), int(keep.sum()), n)
+    h = capi.edge_hashes(path(on), whole)
+    assert h[:2] == h[2:]
+    one = np.flatnonzero(on)[17]
+    on[one] = False                                    # an edge that the path does not have
+    h = capi.edge_hashes(path(on), whole)
+    assert h[0] != h[2] and h[1] != h[3]
+    indices = indices.copy()
+    on[one] = True
+    indices[one] = np.flatnonzero(mask)[(np.searchsorted(np.flatnonzero(mask), indices[one]) + 1) % mask.sum()]
+    h = capi.edge_hashes(path(on), whole)
+    assert h[:2] != h[2:]
+    key = np.unique(src * n + dst)                     # directed
+    directed = capi.TilePlan.from_csr(t(np.concatenate([[0], np.cumsum(np.bincount(key // n, minlength=n))]).astype(np.int32), cuda),
+                                      t((key % n).astype(np.int32), cuda))
+    h = capi.edge_hashes(directed, directed)
+    assert h[:2] != h[2:]

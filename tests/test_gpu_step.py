@@ -616,3 +616,30 @@ def test_long_rows_with_less_room_than_is_of_use(cuda):
         assert ((out.double() - want).abs() <= 1e-6 + 2e-6 * mag).all()
         assert room[given // 4:].isnan().all()                              # nothing beyond the room that was given
     assert lib.eppgcn_update_rows_scratch(*args(out), room.data_ptr() + 4, most, None) == capi.EPP_ERR_BAD_ARG
+
+
+def test_whole_steps_keep_their_plans(cuda):
+    """A step's plans outlive the cache's entry, follow lists that are replaced, and go with the step."""
+    import eppgcn_b200
+    from eppgcn_b200 import graphs, train
+    gnna = eppgcn_b200.load_gnnadvisor()
+    rng = np.random.Generator(np.random.PCG64(3))
+    n = 70_000                                         # beyond the size whose steps are replayed
+    graph = graphs.Graph(*graphs.csr_from_pairs(n, rng.integers(0, n, 100_000), rng.integers(0, n, 100_000)))
+
+    def trainer():
+        ds = graphs.SyntheticDataset(graph, 12, 5, 5, 0.3, seed=5)
+        ds.y = torch.randint(5, (n,), generator=torch.Generator().manual_seed(1))
+        return train.GCNTrainer(ds, hidden=16, seed=2)
+
+    tr = trainer()
+    want = [tr.train_epoch().item() for _ in range(2)]
+    others = [trainer() for _ in range(3)]             # 24 plans, more than are kept
+    for other in others:
+        assert [other.train_epoch().item() for _ in range(2)] == pytest.approx(want, rel=1e-5)
+    gnna.clear_plans()
+    tr.train_epoch()
+    assert gnna.num_plans() == 0
+    tr.back_props[-1].partPointer = tr.back_props[-1].partPointer.clone()       # another list: everything anew
+    tr.train_epoch()
+    assert gnna.num_plans() == 6

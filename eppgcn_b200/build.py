@@ -26,7 +26,7 @@ EXT_PATH = os.path.join(HERE, EXT_NAME + sysconfig.get_config_var("EXT_SUFFIX"))
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
-LIB_SOURCES = ["spmm.cu", "tiled_spmm.cu", "update.cu", "weight_grad.cu", "loss.cu", "optimizer.cu", "head.cu", "prep.cu", "exchange.cu", "host.cu"]
+LIB_SOURCES = ["spmm.cu", "tiled_spmm.cu", "update.cu", "weight_grad.cu", "loss.cu", "optimizer.cu", "head.cu", "layer_backward.cu", "prep.cu", "exchange.cu", "host.cu"]
 
 
 def _nvcc() -> str:

@@ -54,6 +54,9 @@ SIGNATURES = {
     "eppgcn_spmm_tiles_gated": (_I, [_P, _LL, _P, _LL, _P, _P, _P, _LL, _I, _I, _P]),
     "eppgcn_tile_plan_from_ids_of": (_I, [_P, _P, _SZ, _P, _P, _LL, _I, _I, _P, _P, _P]),
     "eppgcn_tile_plan_edge_hashes": (_I, [_P, _P, _P, _P]),
+    "eppgcn_tile_plan_empty_rows": (_I, [_P, _P, _P]),
+    "eppgcn_layer_backward_supported": (_I, [_I, _I]),
+    "eppgcn_layer_backward": (_I, [_P, _LL, _P, _P, _LL, _P, _LL, _P, _P, _P, _I, _P, _I, _I, _I, _P]),
     "eppgcn_head_supported": (_I, [_I, _I]),
     "eppgcn_head_step": (_I, [_P, _LL, _P, _P, _P, _LL, _P, _P, _P, _P, _P, _I, _I, _I, _P]),
     "eppgcn_masked_nll": (_I, [_P, _LL, _P, _P, _LL, _P, _P, _P, _P, _I, _I, _P]),
@@ -225,6 +228,20 @@ def head_step(s, w, labels, mask, used, scale=None):
                                  _dev(mask, torch.bool, "mask"), _dev(used, torch.uint8, "used"),
                                  _dev(scale, torch.float32, "scale"), n, k, c, _stream()))
     return grad[:, :k], dw, sums
+
+
+def layer_backward(d, x, w, scale=None, rows=None, zeros=None, out=None):
+    """``(out, dw)`` of ``eppgcn_layer_backward``; ``d``, ``x``, ``out``: rows padded to 4 floats."""
+    n = x.size(0) if rows is None else rows.numel()
+    if out is None:
+        out = torch.zeros(x.size(0), (w.size(0) + 7) // 8 * 8, device=x.device)
+    dw = torch.zeros_like(w)
+    check(lib().eppgcn_layer_backward(out.data_ptr(), out.stride(0), dw.data_ptr(), d.data_ptr(), _row_stride(d, "d"),
+                                      x.data_ptr(), _row_stride(x, "x"), _dev(w, torch.float32, "w"),
+                                      _dev(scale, torch.float32, "scale"), _dev(rows, torch.int32, "rows"), n,
+                                      _dev(zeros, torch.int32, "zeros"), 0 if zeros is None else zeros.numel(),
+                                      w.size(0), w.size(1), _stream()))
+    return out, dw
 
 
 def weight_grad(x, d, plan=None):

@@ -732,17 +732,39 @@ void run_backward(torch::Tensor grad, const torch::Tensor &x, const std::vector<
     int listed = 0;
     epp_check(eppgcn_tile_plan_active_rows(plans[i]->handle, &rows, &listed), "eppgcn_tile_plan_active_rows");
     const bool by_rows = i > 0 && d <= 256 && n >= 65536 && listed < n / 4 * 3;
+    const int64_t din = weights[i].size(0), ldi = padded_width(din);
+    const bool both = i > 0 && eppgcn_layer_backward_supported(static_cast<int>(din), static_cast<int>(d));
     {
       ScopedMark t(0, 2, static_cast<int>(i) + 1, clock_stream);
-      auto *tiles = i == 0 || by_rows ? eppgcn_spmm_tiles_active : eppgcn_spmm_tiles;
+      auto *tiles = i == 0 || by_rows || both ? eppgcn_spmm_tiles_active : eppgcn_spmm_tiles;
       epp_check(tiles(d_prime.data_ptr<float>(), ld, grad.data_ptr<float>(), grad.stride(0), plans[i]->handle,
                       degrees.data_ptr<float>(), static_cast<int>(ld), stream),
                 "eppgcn_spmm_tiles");
     }
     ScopedMark t(1, 3, 0, clock_stream);
+    if (both) {
+      // rows off the path: those that the next aggregation gathers all the same, or simply all become zero
+      auto next = buffers.rows(n, ldi, x).narrow(1, 0, din);
+      const int *zeros = nullptr;
+      int zero_count = 0;
+      torch::Tensor missing;
+      if (by_rows) {
+        std::tie(missing, zero_count) = missing_rows(plans[i], plans[i - 1], n, stream);
+        buffers.hold(missing);
+        if (zero_count) zeros = missing.data_ptr<int>();
+      } else {
+        epp_check(eppgcn_tile_plan_empty_rows(plans[i]->handle, &zeros, &zero_count), "eppgcn_tile_plan_empty_rows");
+      }
+      epp_check(eppgcn_layer_backward(next.data_ptr<float>(), ldi, sums + offsets[i], d_prime.data_ptr<float>(), ld,
+                                      acts[i - 1].data_ptr<float>(), acts[i - 1].stride(0), weights[i].data_ptr<float>(),
+                                      degrees.data_ptr<float>(), listed == n ? nullptr : rows, listed, zeros, zero_count,
+                                      static_cast<int>(din), static_cast<int>(d), stream),
+                "eppgcn_layer_backward");
+      grad = next;
+      continue;
+    }
     add_weight_grad(sums + offsets[i], i ? acts[i - 1] : x, d_prime, plans[i]->handle, /*relu_x=*/i > 0, stream);
     if (i == 0) break;
-    const int64_t din = weights[i].size(0), ldi = padded_width(din);
     auto next = buffers.rows(n, ldi, x).narrow(1, 0, din);
     const float *gate = acts[i - 1].data_ptr<float>();
     if (by_rows) {

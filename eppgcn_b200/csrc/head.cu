@@ -38,13 +38,6 @@ struct HeadArgs {
   ClockMark mark;
 };
 
-// An 8 x 8 tile of 16-bit pieces with rows and columns exchanged.
-__device__ __forceinline__ unsigned transpose8(unsigned v) {
-  unsigned r;
-  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
-  return r;
-}
-
 // KT pieces of 16 features, NT pieces of 8 classes; rows are looked over PER per lane at a time.
 template <int KT, int NT, int PER>
 __global__ void __launch_bounds__(kHeadWarps * 32, KT * NT <= 3 ? 2 : 1) head_kernel(const HeadArgs a) {

@@ -1,0 +1,315 @@
+// Both gradient products of a hidden layer in one pass over its rows:
+//
+//   dW[k][c] += sum over rows r of relu(x[r][k]) * d[r][c]
+//   out[r][k] = scale[r] * sum_c d[r][c] * W[k][c]   where x[r][k] > 0, else 0
+//
+// As two kernels (weight_grad.cu, update.cu) d and x were read twice, and the gate is x once more: 1.13 M rows x 16 -> 16
+// 44 + 74 us, 59 here (3.7 TB/s); 1 M rows 35 + 67 and 53; 19717 rows 4.3 + 6.5 and 6.3.  Bound by latency and
+// instructions: 24 tensor instructions, 8 splits and 24 transposes for 16 rows of 192 bytes.
+//
+// A warp takes 16 rows at a time, the next ones' loads in flight.  Fragments as in head.cu: four lanes hold a row, lane t
+// columns 4t .. 4t + 3 of every 16, of x and of d alike, so that a lane gates the results with the very values it
+// loaded; movmatrix turns rows into the contracted index for dW.
+#include "mma_split.cuh"
+
+namespace epp {
+namespace {
+
+constexpr int kLbWarps = 8;
+
+struct LayerBackwardArgs {
+  float *out;
+  long long ld_out;
+  float *dw;                       // [k][dout], added to
+  const float *d, *x;
+  long long ldd, ldx;
+  const float *w;                  // [k][dout]
+  const float *scale;
+  const int *rows, *zeros;         // rows of d, x and out that are meant, or NULL: all; rows of out that become zero
+  int n, zero_count, k, dout;
+  ClockMark mark;
+};
+
+template <int KT, int DT>
+struct LayerBackwardShape {        // 16 KT columns of x, 16 DT of d
+  static constexpr int AHEAD = 2;  // units of 16 rows: one in work, the other on its way (three: registers spill, 59 -> 67 us)
+  static constexpr int RESIDENT = KT * DT == 1 ? 2 : 1;            // blocks per SM
+};
+
+template <int KT, int DT>
+struct RowUnit {                   // of 16 rows this lane's part: rows g and g + 8
+  float4 x[2][KT], d[2][DT];
+  float scale[2];
+  int row[2];                      // -1: none
+};
+
+template <int KT, int DT, bool LIST>
+__global__ void __launch_bounds__(kLbWarps * 32, (LayerBackwardShape<KT, DT>::RESIDENT)) layer_backward_kernel(
+    const LayerBackwardArgs a) {
+  constexpr int AHEAD = LayerBackwardShape<KT, DT>::AHEAD, F = 16 * KT, C = 16 * DT;
+  __shared__ uint2 s_w[DT * 2 * KT * 96];      // fragments of W^T: [step over c][tile over k][piece][lane]
+  __shared__ float s_dw[F * C];
+  if (blockIdx.x == 0 && threadIdx.x == 0) clock_begin(a.mark);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  auto weight = [&](int f, int c) { return f < a.k && c < a.dout ? __ldg(a.w + static_cast<long long>(f) * a.dout + c) : 0.f; };
+  for (int e = threadIdx.x; e < DT * 2 * KT * 32; e += blockDim.x) {
+    const int l = e % 32, j = e / 32 % (2 * KT), c = 16 * (e / 32 / (2 * KT)) + 4 * (l & 3), n8 = l >> 2;
+    const int f = 16 * (j / 2) + 4 * (n8 / 2) + n8 % 2 + 2 * (j % 2);      // two tiles share 16 columns: a lane holds 4 in a row
+    uint2 *const at = s_w + e / 32 * 96 + l;
+    split3(weight(f, c), weight(f, c + 1), at[0].x, at[32].x, at[64].x);
+    split3(weight(f, c + 2), weight(f, c + 3), at[0].y, at[32].y, at[64].y);
+  }
+  const int quads = static_cast<int>(a.ld_out / 4);
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < static_cast<long long>(a.zero_count) * quads;
+       i += static_cast<long long>(gridDim.x) * blockDim.x)
+    *reinterpret_cast<float4 *>(a.out + __ldg(a.zeros + i / quads) * a.ld_out + i % quads * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
+
+  const int units = static_cast<int>((static_cast<long long>(a.n) + 15) / 16);
+  const int stride = static_cast<int>(gridDim.x) * kLbWarps, first = static_cast<int>(blockIdx.x) * kLbWarps + warp;
+  int ids[2];                                  // rows of the next unit to load
+  auto load_ids = [&](int unit) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const long long at = static_cast<long long>(unit) * 16 + 8 * h + g;
+      ids[h] = unit < units && at < a.n ? (LIST ? __ldg(a.rows + at) : static_cast<int>(at)) : -1;
+    }
+  };
+  // columns beyond the matrix count as zeros whatever the padding holds
+  auto load_row = [&](const float *p, int columns, int s) {
+    const int c = 16 * s + 4 * t;
+    if (c >= columns) return make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v = __ldg(reinterpret_cast<const float4 *>(p + c));
+    if (c + 1 >= columns) v.y = 0.f;
+    if (c + 2 >= columns) v.z = 0.f;
+    if (c + 3 >= columns) v.w = 0.f;
+    return v;
+  };
+  auto load = [&](RowUnit<KT, DT> &u, int next) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int row = ids[h];
+      u.row[h] = row;
+      u.scale[h] = row >= 0 && a.scale ? __ldg(a.scale + row) : 1.f;
+      const float *xp = a.x + static_cast<long long>(row) * a.ldx, *dp = a.d + static_cast<long long>(row) * a.ldd;
+#pragma unroll
+      for (int s = 0; s < KT; ++s) u.x[h][s] = row >= 0 ? load_row(xp, a.k, s) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int s = 0; s < DT; ++s) u.d[h][s] = row >= 0 ? load_row(dp, a.dout, s) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    load_ids(next);
+  };
+
+  float dw_top[KT][2 * DT][1][4], dw_rest[KT][2 * DT][1][4];
+#pragma unroll
+  for (int s = 0; s < KT; ++s)
+#pragma unroll
+    for (int j = 0; j < 2 * DT; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) dw_top[s][j][0][q] = dw_rest[s][j][0][q] = 0.f;
+
+  auto split_rows = [&](const float4 &v0, const float4 &v1, unsigned (&p)[3][4]) {
+    split3(v0.x, v0.y, p[0][0], p[1][0], p[2][0]);
+    split3(v1.x, v1.y, p[0][1], p[1][1], p[2][1]);
+    split3(v0.z, v0.w, p[0][2], p[1][2], p[2][2]);
+    split3(v1.z, v1.w, p[0][3], p[1][3], p[2][3]);
+  };
+  auto work = [&](const RowUnit<KT, DT> &u) {
+    unsigned xt[KT][1][3][4];                  // relu(x) with rows as the contracted index
+#pragma unroll
+    for (int s = 0; s < KT; ++s) {
+      unsigned p[3][4];
+      split_rows(relu4(u.x[0][s]), relu4(u.x[1][s]), p);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        xt[s][0][i][0] = transpose8(p[i][0]);
+        xt[s][0][i][1] = transpose8(p[i][2]);
+        xt[s][0][i][2] = transpose8(p[i][1]);
+        xt[s][0][i][3] = transpose8(p[i][3]);
+      }
+    }
+    float top[2 * KT][1][4], rest[2 * KT][1][4];
+#pragma unroll
+    for (int j = 0; j < 2 * KT; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) top[j][0][q] = rest[j][0][q] = 0.f;
+#pragma unroll
+    for (int s = 0; s < DT; ++s) {
+      unsigned p[1][3][4];
+      split_rows(u.d[0][s], u.d[1][s], p[0]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {            // positions 8i .. 8i + 7 of these 16 columns
+        uint2 b[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) b[q] = make_uint2(transpose8(p[0][q][2 * i]), transpose8(p[0][q][2 * i + 1]));
+#pragma unroll
+        for (int f = 0; f < KT; ++f) multiply_split(dw_top[f][2 * s + i], dw_rest[f][2 * s + i], xt[f], b[0], b[1], b[2]);
+      }
+#pragma unroll
+      for (int j = 0; j < 2 * KT; ++j) {
+        const uint2 *f = s_w + (s * 2 * KT + j) * 96 + lane;
+        multiply_split(top[j], rest[j], p, f[0], f[32], f[64]);
+      }
+    }
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < 2 * KT; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        top[j][0][q] += rest[j][0][q];
+        bad |= isnan(top[j][0][q]);
+      }
+    if (__any_sync(kFull, bad)) {              // an infinity has no pieces: as a plain sum gives it
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (u.row[h] < 0) continue;
+        const float *p = a.d + static_cast<long long>(u.row[h]) * a.ldd;
+#pragma unroll
+        for (int j = 0; j < 2 * KT; ++j)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int f = 16 * (j / 2) + 4 * t + 2 * (j % 2) + i;
+            if (f >= a.k || !isnan(top[j][0][2 * h + i])) continue;
+            float sum = 0.f;
+#pragma unroll 1
+            for (int c = 0; c < a.dout; ++c) sum = fmaf(__ldg(p + c), __ldg(a.w + static_cast<long long>(f) * a.dout + c), sum);
+            top[j][0][2 * h + i] = sum;
+          }
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (u.row[h] < 0) continue;
+#pragma unroll
+      for (int s = 0; s < KT; ++s) {
+        if (16 * s + 4 * t >= a.ld_out) continue;
+        const float4 &x = u.x[h][s];
+        float4 o;
+        o.x = x.x <= 0.f ? 0.f : top[2 * s][0][2 * h] * u.scale[h];
+        o.y = x.y <= 0.f ? 0.f : top[2 * s][0][2 * h + 1] * u.scale[h];
+        o.z = x.z <= 0.f ? 0.f : top[2 * s + 1][0][2 * h] * u.scale[h];
+        o.w = x.w <= 0.f ? 0.f : top[2 * s + 1][0][2 * h + 1] * u.scale[h];
+        *reinterpret_cast<float4 *>(a.out + static_cast<long long>(u.row[h]) * a.ld_out + 16 * s + 4 * t) = o;
+      }
+    }
+  };
+
+  RowUnit<KT, DT> u[AHEAD];
+  load_ids(first);
+#pragma unroll
+  for (int i = 0; i < AHEAD - 1; ++i) load(u[i], first + (i + 1) * stride);
+  for (int unit = first; unit < units; unit += AHEAD * stride) {
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+      load(u[(i + AHEAD - 1) % AHEAD], unit + (i + AHEAD) * stride);
+      if (unit + i * stride < units) work(u[i]);
+    }
+  }
+
+  // an entry of dW that is NaN: once more over this warp's rows, until all such are NaN here too or the rows end
+  bool bad = false;
+#pragma unroll
+  for (int s = 0; s < KT; ++s)
+#pragma unroll
+    for (int j = 0; j < 2 * DT; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        dw_top[s][j][0][q] += dw_rest[s][j][0][q];
+        bad |= isnan(dw_top[s][j][0][q]);
+      }
+  // column of the matrix that position `pos` of 16 stands for
+  auto column = [](int pos) { return 4 * (pos % 8 / 2) + pos % 2 + 2 * (pos / 8); };
+  if (__any_sync(kFull, bad)) {
+    float sum[KT][2 * DT][4] = {};
+    bool open = true;
+#pragma unroll 1
+    for (int unit = first; unit < units && __any_sync(kFull, open); unit += stride) {
+#pragma unroll 1
+      for (int r = 0; r < 16 && unit * 16LL + r < a.n; ++r) {
+        const long long at = unit * 16LL + r, row = LIST ? __ldg(a.rows + at) : at;
+#pragma unroll
+        for (int s = 0; s < KT; ++s)
+#pragma unroll
+          for (int j = 0; j < 2 * DT; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int f = 16 * s + column(g + 8 * (q / 2)), c = 16 * (j / 2) + column(8 * (j % 2) + 2 * t + q % 2);
+              if (f < a.k && c < a.dout)
+                sum[s][j][q] = fmaf(max_nan(__ldg(a.x + row * a.ldx + f), 0.f), __ldg(a.d + row * a.ldd + c), sum[s][j][q]);
+            }
+      }
+      open = false;
+#pragma unroll
+      for (int s = 0; s < KT; ++s)
+#pragma unroll
+        for (int j = 0; j < 2 * DT; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) open |= isnan(dw_top[s][j][0][q]) && !isnan(sum[s][j][q]);
+    }
+#pragma unroll
+    for (int s = 0; s < KT; ++s)
+#pragma unroll
+      for (int j = 0; j < 2 * DT; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (isnan(dw_top[s][j][0][q])) dw_top[s][j][0][q] = sum[s][j][q];
+  }
+#pragma unroll 1
+  for (int w = 0; w < kLbWarps; ++w) {         // the block's dW, warp after warp in one buffer
+    if (w == warp) {
+#pragma unroll
+      for (int s = 0; s < KT; ++s)
+#pragma unroll
+        for (int j = 0; j < 2 * DT; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int f = 16 * s + column(g + 8 * (q / 2)), c = 16 * (j / 2) + column(8 * (j % 2) + 2 * t + q % 2);
+            float *const at = s_dw + f * C + c;
+            *at = (w ? *at : 0.f) + dw_top[s][j][0][q];
+          }
+    }
+    __syncthreads();
+  }
+  for (int e = threadIdx.x; e < F * C; e += blockDim.x) {
+    const int f = e / C, c = e % C;
+    if (f < a.k && c < a.dout) atomicAdd(a.dw + static_cast<long long>(f) * a.dout + c, s_dw[e]);
+  }
+  if (threadIdx.x == 0) clock_end(a.mark);
+}
+
+template <int KT, int DT>
+int launch_layer_backward(const LayerBackwardArgs &a, int sms, cudaStream_t s) {
+  const long long blocks = ceil_div_ll(ceil_div_ll(a.n, 16), kLbWarps), most = static_cast<long long>(sms) * LayerBackwardShape<KT, DT>::RESIDENT;
+  const unsigned grid = static_cast<unsigned>(blocks < 1 ? 1 : blocks < most ? blocks : most);
+  if (a.rows) layer_backward_kernel<KT, DT, true><<<grid, kLbWarps * 32, 0, s>>>(a);
+  else layer_backward_kernel<KT, DT, false><<<grid, kLbWarps * 32, 0, s>>>(a);
+  EPP_CHECK_LAUNCH("layer_backward_kernel");
+  return EPP_OK;
+}
+
+}  // namespace
+}  // namespace epp
+
+EPP_EXPORT int eppgcn_layer_backward_supported(int k, int dout) { return k >= 1 && dout >= 1 && k <= 32 && dout <= 32; }
+
+EPP_EXPORT int eppgcn_layer_backward(float *out, long long ld_out, float *dw, const float *d, long long ldd, const float *x,
+                                     long long ldx, const float *w, const float *row_scale, const int *rows, int num_rows,
+                                     const int *zeros, int zero_count, int k, int dout, void *stream) {
+  using namespace epp;
+  EPP_REQUIRE(num_rows >= 0 && zero_count >= 0 && k >= 1 && dout >= 1, "negative size, k < 1 or dout < 1");
+  if (!eppgcn_layer_backward_supported(k, dout)) {
+    set_error("eppgcn_layer_backward handles at most 32 columns on both sides, got %d and %d", k, dout);
+    return EPP_ERR_TOO_LARGE;
+  }
+  if (num_rows == 0 && zero_count == 0) return EPP_OK;
+  EPP_REQUIRE(out && dw && d && x && w && (zeros || zero_count == 0), "null pointer");
+  EPP_REQUIRE(ldx % 4 == 0 && ldx >= (k + 3) / 4 * 4 && aligned(x, 16) && ldd % 4 == 0 && ldd >= (dout + 3) / 4 * 4 && aligned(d, 16) &&
+                  ld_out % 4 == 0 && ld_out >= (k + 3) / 4 * 4 && ld_out <= (k + 15) / 16 * 16 && aligned(out, 16),
+              "rows must be 16-byte aligned and padded to a multiple of 4 floats, those of out by less than 16");
+  int sms = 148;
+  if (const int rc = device_sm_count(&sms); rc != EPP_OK) return rc;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const LayerBackwardArgs a{out, ld_out, dw, d, x, ldd, ldx, w, row_scale, rows, zeros, num_rows, zero_count, k, dout, take_mark()};
+  if (k <= 16) return dout <= 16 ? launch_layer_backward<1, 1>(a, sms, s) : launch_layer_backward<1, 2>(a, sms, s);
+  return dout <= 16 ? launch_layer_backward<2, 1>(a, sms, s) : launch_layer_backward<2, 2>(a, sms, s);
+}

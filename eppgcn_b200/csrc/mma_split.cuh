@@ -65,6 +65,13 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const unsigned (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// An 8 x 8 tile of 16-bit pieces with rows and columns exchanged.
+__device__ __forceinline__ unsigned transpose8(unsigned v) {
+  unsigned r;
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
+
 // The six products of one 16 x 16 piece of x and one 16 x 8 piece of W.
 template <int M>
 __device__ __forceinline__ void multiply_split(float (&top)[M][4], float (&rest)[M][4], const unsigned (&x)[M][3][4],

@@ -979,6 +979,13 @@ EPP_EXPORT int eppgcn_tile_plan_active_rows(const eppgcn_tile_plan *plan, const 
   return EPP_OK;
 }
 
+EPP_EXPORT int eppgcn_tile_plan_empty_rows(const eppgcn_tile_plan *plan, const int **rows_dev, int *count) {
+  EPP_REQUIRE(plan && rows_dev && count, "null pointer");
+  *rows_dev = plan->zero_rows + plan->hub_rows;       // hub rows come first in the list
+  *count = plan->num_zero - plan->hub_rows;
+  return EPP_OK;
+}
+
 EPP_EXPORT int eppgcn_tile_plan_used(const eppgcn_tile_plan *plan, const unsigned char **used_dev) {
   EPP_REQUIRE(plan && used_dev, "null pointer");
   *used_dev = plan->used;

@@ -164,6 +164,8 @@ void eppgcn_tile_plan_destroy(eppgcn_tile_plan *plan);
 int eppgcn_tile_plan_info(const eppgcn_tile_plan *plan, long long *out8);
 /* The rows that have at least one edge, ascending (device int32 inside the plan's buffer). */
 int eppgcn_tile_plan_active_rows(const eppgcn_tile_plan *plan, const int **rows_dev, int *count);
+/* The rows without an edge, ascending, in the same way. */
+int eppgcn_tile_plan_empty_rows(const eppgcn_tile_plan *plan, const int **rows_dev, int *count);
 /* One byte per source row: 1 where an edge of the list names it (device memory inside the plan's buffer). */
 int eppgcn_tile_plan_used(const eppgcn_tile_plan *plan, const unsigned char **used_dev);
 int eppgcn_spmm_tiles(float *out, long long out_ld, const float *src, long long src_ld,
@@ -310,6 +312,14 @@ int eppgcn_head_supported(int k, int classes);
 int eppgcn_head_step(float *grad, long long ld_grad, float *dw, double *sums, const float *s, long long ld_s,
                      const float *w, const long long *labels, const unsigned char *mask, const unsigned char *used,
                      const float *row_scale, int num_rows, int k, int num_classes, void *stream);
+/* eppgcn_layer_backward: both gradient products of a hidden layer of at most 32 columns on either side, over num_rows rows
+ *   (a list, or 0 .. num_rows - 1 where rows is NULL): dw [k][dout] += relu(x)^T d and, in the rows of out,
+ *   row_scale * (d w^T) where x > 0 and zero elsewhere; the listed rows `zeros` of out become zero.  All rows of a
+ *   multiple of 4 floats, 16-byte aligned; those of out whole, with zeros beyond k. */
+int eppgcn_layer_backward_supported(int k, int dout);
+int eppgcn_layer_backward(float *out, long long ld_out, float *dw, const float *d, long long ldd, const float *x,
+                          long long ldx, const float *w, const float *row_scale, const int *rows, int num_rows,
+                          const int *zeros, int zero_count, int k, int dout, void *stream);
 int eppgcn_masked_nll(float *grad, long long grad_ld, double *sums, const float *logits, long long ld,
                       const long long *labels, const unsigned char *mask, const unsigned char *used,
                       const float *row_scale, int num_rows, int num_classes, void *stream);

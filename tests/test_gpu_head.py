@@ -75,6 +75,50 @@ def test_head_step_with_infinite_weights(cuda, k, c):
     assert sums[0].isnan() and dw.isnan().all()
 
 
+@pytest.mark.parametrize("n", [1, 15, 33, 4097, 80_001])
+@pytest.mark.parametrize("k,dout", [(1, 1), (5, 16), (16, 7), (16, 16), (16, 22), (17, 9), (32, 32), (31, 3)])
+def test_layer_backward(cuda, n, k, dout):
+    """Ragged units of 16 rows, columns on both sides, padding that is not zero, a row list and rows that become zero.
+    Bounds: sums of dout or n products, 2^-23 of their size each."""
+    gen = torch.Generator(device=cuda).manual_seed(n + k)
+    x, d = (torch.full((n, (c + 7) // 8 * 8), 3e38, device=cuda)[:, :c].copy_(torch.randn(n, c, device=cuda, generator=gen))
+            for c in (k, dout))
+    w, scale = torch.randn(k, dout, device=cuda, generator=gen), torch.rand(n, device=cuda, generator=gen) + 0.5
+    gate = (x > 0).double() * scale.double()[:, None]
+    want, mag = (d.double() @ w.double().T) * gate, (d.double().abs() @ w.double().abs().T) * gate
+    dwant, dmag = x.double().clamp(min=0).T @ d.double(), x.double().clamp(min=0).T @ d.double().abs()
+    out, dw = capi.layer_backward(d, x, w, scale)
+    assert ((out[:, :k].double() - want).abs() <= 1e-6 + 2e-6 * mag).all() and (out[:, k:] == 0).all()
+    assert ((dw.double() - dwant).abs() <= 1e-6 + 1e-6 * dmag).all()
+    rows = torch.arange(0, n, 3, device=cuda, dtype=torch.int32)
+    zeros = torch.arange(1, n, 3, device=cuda, dtype=torch.int32)
+    out, dw = capi.layer_backward(d, x, w, scale, rows, zeros, torch.full((n, (k + 7) // 8 * 8), 7.0, device=cuda))
+    assert ((out[::3, :k].double() - want[::3]).abs() <= 1e-6 + 2e-6 * mag[::3]).all()
+    assert (out[1::3] == 0).all() and (out[2::3] == 7.0).all()
+    dwant, dmag = x[::3].double().clamp(min=0).T @ d[::3].double(), x[::3].double().clamp(min=0).T @ d[::3].double().abs()
+    assert ((dw.double() - dwant).abs() <= 1e-6 + 1e-6 * dmag).all()
+
+
+@pytest.mark.parametrize("n,k,dout", [(70, 16, 16), (5000, 32, 9)])
+@pytest.mark.parametrize("value", ["inf", "-inf", "nan"])
+def test_layer_backward_with_infinities(cuda, n, k, dout, value):
+    """Infinities and NaN come out as plain sums of products give them."""
+    gen = torch.Generator(device=cuda).manual_seed(n)
+    for where in ("x", "d", "w", "all of w"):
+        x, d = (torch.zeros(n, (c + 7) // 8 * 8, device=cuda)[:, :c].copy_(torch.rand(n, c, device=cuda, generator=gen) + 0.1)
+                for c in (k, dout))
+        w = torch.randn(k, dout, device=cuda, generator=gen)
+        {"x": x, "d": d, "w": w}[where[-1]][(slice(None) if where == "all of w" else 3 % w.size(0))] = float(value)
+        out, dw = capi.layer_backward(d, x, w)
+        want = torch.where(x <= 0, 0.0, d.double() @ w.double().T)
+        dwant = x.double().clamp(min=0).T @ d.double()
+        for got, ref in ((out[:, :k], want), (dw, dwant)):
+            assert torch.equal(got.isnan(), ref.isnan())
+            ok = ref.isfinite()
+            assert torch.equal(got[~ok & ~ref.isnan()].double(), ref[~ok & ~ref.isnan()].double())
+            assert torch.allclose(got[ok].double(), ref[ok].double(), rtol=1e-5, atol=1e-4)
+
+
 @pytest.mark.parametrize("dim", [3, 8, 16, 24, 40])
 @pytest.mark.parametrize("graph", [dict(n=700, avg_deg=6.0, seed=3, hubs=3, hub_deg=650), dict(n=2000, avg_deg=1.0, seed=5, empty_frac=0.5)])
 def test_rows_leave_finished(cuda, dim, graph):

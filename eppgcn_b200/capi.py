@@ -50,8 +50,9 @@ SIGNATURES = {
     "eppgcn_tile_plan_missing": (_I, [_P, _P, _P, _P, _P, _P]),
     "eppgcn_zero_rows": (_I, [_P, _LL, _I, _P, _I, _P]),
     "eppgcn_weight_grad_add": (_I, [_P, _P, _LL, _P, _LL, _P, _I, _I, _I, _I, _P]),
-    "eppgcn_spmm_tiles_relu": (_I, [_P, _LL, _P, _LL, _P, _P, _I, _P]),
-    "eppgcn_spmm_tiles_gated": (_I, [_P, _LL, _P, _LL, _P, _P, _P, _LL, _I, _I, _P]),
+    "eppgcn_spmm_tiles_flags": (_I, [_P, _LL, _P, _LL, _P, _P, _P, _LL, _I, _I, _P]),
+    "eppgcn_clear_begin": (_I, [_P, _LL, _I, _P, _I, _P]),
+    "eppgcn_clear_end": (_I, []),
     "eppgcn_tile_plan_from_ids_of": (_I, [_P, _P, _SZ, _P, _P, _LL, _I, _I, _P, _P, _P]),
     "eppgcn_tile_plan_edge_hashes": (_I, [_P, _P, _P, _P]),
     "eppgcn_tile_plan_empty_rows": (_I, [_P, _P, _P]),
@@ -382,7 +383,10 @@ def spmm_tiles(src, plan, row_scale=None, out=None):
     return out
 
 
-def spmm_tiles_finished(src, plan, row_scale, gate=None, every_row=True, out=None):
+TILES_EVERY_ROW, TILES_RELU, TILES_CLEARED = 1, 2, 4
+
+
+def spmm_tiles_finished(src, plan, row_scale, gate=None, every_row=True, out=None, flags=0):
     """``y = spmm_tiles(src, plan, row_scale)`` as ``row_scale * relu(y)``, or with a gate as ``row_scale * y`` where the
     gate is not zero; ``out``: rows padded to 4 floats."""
     n, dim = plan.info["rows"], src.size(1)
@@ -390,10 +394,9 @@ def spmm_tiles_finished(src, plan, row_scale, gate=None, every_row=True, out=Non
         out = torch.empty(n, (dim + 3) // 4 * 4, device=src.device, dtype=torch.float32)[:, :dim]
     args = (out.data_ptr(), out.stride(0), src.data_ptr(), _row_stride(src, "src"), plan._handle,
             _dev(row_scale, torch.float32, "row_scale"))
-    if gate is None:
-        check(lib().eppgcn_spmm_tiles_relu(*args, dim, _stream()))
-    else:
-        check(lib().eppgcn_spmm_tiles_gated(*args, gate.data_ptr(), gate.stride(0), dim, int(every_row), _stream()))
+    flags |= (TILES_EVERY_ROW if every_row else 0) | (TILES_RELU if gate is None else 0)
+    check(lib().eppgcn_spmm_tiles_flags(*args, None if gate is None else gate.data_ptr(), 0 if gate is None else gate.stride(0),
+                                        dim, flags, _stream()))
     return out
 
 

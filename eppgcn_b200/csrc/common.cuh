@@ -113,6 +113,28 @@ __device__ __forceinline__ void clock_end(const ClockMark &m) {
 ClockMark take_mark();
 
 // ---------------------------------------------------------------------------
+// Rows that an aggregation adds to with atomics, and rows without an edge, are cleared in front of it.  A kernel of its
+// own for that costs its launch, 2 us in a recorded step and 4 - 6 between others, for a few thousand rows: the kernel that
+// runs before the aggregation clears them on its way (eppgcn_clear_begin).
+// ---------------------------------------------------------------------------
+struct ClearList {
+  float *out;                              // rows of ld floats, 16-byte aligned
+  long long ld;
+  const int *rows;
+  int count, quads;                        // rows; 16-byte pieces per row
+};
+__device__ __forceinline__ void clear_rows(const ClearList &c) {
+  const long long total = static_cast<long long>(c.count) * c.quads;
+  const long long block = blockIdx.x + static_cast<long long>(gridDim.x) * (blockIdx.y + static_cast<long long>(gridDim.y) * blockIdx.z);
+  const long long stride = static_cast<long long>(gridDim.x) * gridDim.y * gridDim.z * blockDim.x;
+  for (long long i = block * blockDim.x + threadIdx.x; i < total; i += stride)
+    *reinterpret_cast<float4 *>(c.out + __ldg(c.rows + i / c.quads) * c.ld + i % c.quads * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+// What the calling thread wants cleared, for its next kernel on the stream; and how it says so.
+ClearList take_clear(cudaStream_t s);
+void want_clear(const ClearList &c, cudaStream_t s);
+
+// ---------------------------------------------------------------------------
 // Tile descriptor of the chained (decoupled look-back) scans.
 // One 64-bit word per tile: bits 63..62 state, 61..31 field B, 30..0 field A.
 // Both fields are partial sums of int32 totals that the host has checked to be

@@ -63,6 +63,26 @@ struct ScopedMark {
   ~ScopedMark() { eppgcn_mark_end(); }
 };
 
+// While it lives the next kernel clears what an aggregation over `plan` into `out` wants cleared.
+struct ScopedClear {
+  ScopedClear(const torch::Tensor &out, int64_t dim, const eppgcn_tile_plan *plan, bool every_row, void *stream) {
+    epp_check(eppgcn_clear_begin(out.data_ptr<float>(), out.stride(0), static_cast<int>(dim), plan, every_row ? 1 : 0, stream),
+              "eppgcn_clear_begin");
+  }
+  int flags() {                        // for the aggregation; ends the wish
+    open_ = false;
+    return eppgcn_clear_end() ? EPP_TILES_CLEARED : 0;
+  }
+  ~ScopedClear() {
+    if (open_) (void)eppgcn_clear_end();
+  }
+  ScopedClear(const ScopedClear &) = delete;
+  ScopedClear &operator=(const ScopedClear &) = delete;
+
+ private:
+  bool open_ = true;
+};
+
 int padded_width(int64_t dim) { return static_cast<int>((dim + 7) / 8 * 8); }
 
 // ---------------------------------------------------------------------------
@@ -597,32 +617,41 @@ std::vector<torch::Tensor> run_forward(const torch::Tensor &x, const std::vector
   const int64_t n = x.size(0);
   std::vector<torch::Tensor> acts;
   for (size_t i = 0; i < weights.size(); ++i) {
-    if (head && i + 1 == weights.size()) {
-      const int64_t k = weights[i].size(0), ld = padded_width(k);
-      auto out = buffers.rows(n, ld, x).narrow(1, 0, k);
-      ScopedMark t(0, 0, 0, clock_stream);
-      epp_check(eppgcn_spmm_tiles(out.data_ptr<float>(), ld, acts.back().data_ptr<float>(), ld, plan,
-                                  degrees.data_ptr<float>(), static_cast<int>(ld), stream),
-                "eppgcn_spmm_tiles");
-      acts.push_back(out);
-      break;
-    }
     const torch::Tensor &in = i ? acts.back() : x, &w = weights[i];
     const int64_t k = in.size(1), d = w.size(1), ld = padded_width(d), ld_out = dense_last && i + 1 == weights.size() ? d : ld;
     auto tmp = buffers.rows(n, ld, x);
+    // padded rows are aggregated whole (their padding is zero on both sides): 16-byte stores, plain clearing
+    auto out = buffers.rows(n, ld_out, x).narrow(1, 0, d);
+    int flags = 0;
     {
       ScopedMark t(0, 1, 0, clock_stream);
+      ScopedClear clear(out, ld_out, plan, true, stream);
       update_rows(tmp.data_ptr<float>(), ld, in, std::max(in.stride(0), k), w.data_ptr<float>(), d, 1,
                   degrees.data_ptr<float>(), nullptr, 0, i > 0, n, k, d, ld - d, buffers, stream);
+      flags = clear.flags();
     }
-    auto out = buffers.rows(n, ld_out, x).narrow(1, 0, d);
-    ScopedMark t(1, 0, 0, clock_stream);
-    // padded rows are aggregated whole (their padding is zero on both sides): 16-byte stores, plain clearing
-    auto *tiles = head && i + 2 == weights.size() ? eppgcn_spmm_tiles_relu : eppgcn_spmm_tiles;
-    epp_check(tiles(out.data_ptr<float>(), ld_out, tmp.data_ptr<float>(), ld, plan, degrees.data_ptr<float>(),
-                    static_cast<int>(ld_out), stream),
-              "eppgcn_spmm_tiles");
+    auto aggregate = [&](const torch::Tensor &to, const torch::Tensor &from, int dim, int with) {
+      epp_check(eppgcn_spmm_tiles_flags(to.data_ptr<float>(), to.stride(0), from.data_ptr<float>(), from.stride(0), plan,
+                                        degrees.data_ptr<float>(), nullptr, 0, dim, with | EPP_TILES_EVERY_ROW, stream),
+                "eppgcn_spmm_tiles_flags");
+    };
     acts.push_back(out);
+    if (!head || i + 2 < weights.size()) {
+      ScopedMark t(1, 0, 0, clock_stream);
+      aggregate(out, tmp, static_cast<int>(ld_out), flags);
+      continue;
+    }
+    auto rows = buffers.rows(n, ld, x).narrow(1, 0, d);      // the last layer's, of the hidden width
+    {
+      ScopedMark t(1, 0, 0, clock_stream);
+      ScopedClear clear(rows, ld, plan, true, stream);
+      aggregate(out, tmp, static_cast<int>(ld), flags | EPP_TILES_RELU);
+      flags = clear.flags();
+    }
+    ScopedMark t(0, 0, 0, clock_stream);
+    aggregate(rows, out, static_cast<int>(ld), flags);
+    acts.push_back(rows);
+    break;
   }
   return acts;
 }
@@ -686,99 +715,135 @@ std::vector<int64_t> sum_offsets(const std::vector<torch::Tensor> &weights, int6
   return at;
 }
 
+// How the backward of layer i goes: over the path's rows only, or both gradient products in one kernel.
+//
+// Rows off the path are zero in d' and in the next gradient.  Where they are many, neither is written nor read: the
+// weight gradient and the update walk the path's rows, and only rows that the next aggregation gathers all the same
+// (none on a symmetric graph) are cleared.  Social graphs of 6 edges per vertex, us per epoch over all rows and over the
+// path's: 500 K vertices, 16 columns, a path of 8, then 66 % of the rows: 491 and 448, of 32 and 78 %: 517 and 492;
+// 64 columns 1346 and 1167, 1408 and 1300; 200 K 632 and 553.  Beyond 80 % of the rows it loses 1 - 3 %.  Steps of up to
+// 65,536 vertices are replayed; there the two differ by 2 % either way at 16 columns, and wide ones gain up to 9 %,
+// which this line leaves.
+struct LayerWay {
+  const int *rows = nullptr;           // of the path
+  int listed = 0;
+  bool by_rows = false, both = false;
+};
+LayerWay layer_way(size_t i, int64_t din, int64_t d, const Plan &plan, int64_t n) {
+  LayerWay w;
+  epp_check(eppgcn_tile_plan_active_rows(plan.handle, &w.rows, &w.listed), "eppgcn_tile_plan_active_rows");
+  w.by_rows = i > 0 && d <= 256 && n >= 65536 && w.listed < n / 4 * 3;
+  w.both = i > 0 && eppgcn_layer_backward_supported(static_cast<int>(din), static_cast<int>(d));
+  return w;
+}
+
+// What the backward aggregation of a layer writes: d', or with a head, of the last layer, the next gradient.
+struct BackwardTarget {
+  torch::Tensor out;
+  int64_t ld;
+  int flags;                           // EPP_TILES_EVERY_ROW, EPP_TILES_CLEARED
+  LayerWay way;
+};
+BackwardTarget backward_target(size_t i, const std::vector<torch::Tensor> &weights, const std::vector<PlanPtr> &plans, bool head,
+                               const torch::Tensor &x, NetBuffers &buffers) {
+  const int64_t din = weights[i].size(0), d = weights[i].size(1), n = x.size(0);
+  const bool last = head && i + 1 == weights.size();
+  BackwardTarget t;
+  t.way = layer_way(i, din, last ? din : d, *plans[i], n);
+  const int64_t width = last ? din : d;
+  t.ld = padded_width(width);
+  t.out = buffers.rows(n, t.ld, x).narrow(1, 0, width);
+  t.flags = t.way.by_rows || (!last && (i == 0 || t.way.both)) ? 0 : EPP_TILES_EVERY_ROW;
+  return t;
+}
+// The wish that the next kernel clears it.
+struct TargetClear : ScopedClear {
+  TargetClear(BackwardTarget &t, const PlanPtr &plan, void *stream)
+      : ScopedClear(t.out, t.ld, plan->handle, (t.flags & EPP_TILES_EVERY_ROW) != 0, stream), target(t) {}
+  void done() { target.flags |= flags(); }
+  BackwardTarget &target;
+};
+
 // Adds the weight gradients' sums to `sums` (cleared; laid out by sum_offsets).
-void run_backward(torch::Tensor grad, const torch::Tensor &x, const std::vector<torch::Tensor> &weights,
+void run_backward(torch::Tensor grad, BackwardTarget target, const torch::Tensor &x, const std::vector<torch::Tensor> &weights,
                   const std::vector<torch::Tensor> &acts, const torch::Tensor &degrees, const std::vector<PlanPtr> &plans,
                   float *sums, const std::vector<int64_t> &offsets, bool head, NetBuffers &buffers, void *stream,
                   void *clock_stream) {
   const int64_t n = x.size(0);
-  auto clear_missing = [&](const torch::Tensor &rows_of, size_t i) {      // rows off path i that path i - 1 gathers
-    const auto [zeros, count] = missing_rows(plans[i], plans[i - 1], n, stream);
-    buffers.hold(zeros);
+  auto missing = [&](size_t i) {                     // rows off path i that path i - 1 gathers
+    auto found = missing_rows(plans[i], plans[i - 1], n, stream);
+    buffers.hold(found.first);
+    return found;
+  };
+  auto clear_missing = [&](const torch::Tensor &rows_of, size_t i) {
+    const auto [zeros, count] = missing(i);
     const int ld = static_cast<int>(rows_of.stride(0));
     if (count)
       epp_check(eppgcn_zero_rows(rows_of.data_ptr<float>(), ld, ld, zeros.data_ptr<int>(), count, stream), "eppgcn_zero_rows");
   };
   for (size_t i = weights.size(); i-- > 0;) {
-    if (head && i + 1 == weights.size()) {
+    const bool last = head && i + 1 == weights.size();
+    const LayerWay way = target.way;
+    const auto result = target.out;
+    const int64_t ld = target.ld, d = weights[i].size(1), din = weights[i].size(0), ldi = padded_width(din);
+    auto aggregate = [&](const float *gate, int64_t ld_gate) {
+      epp_check(eppgcn_spmm_tiles_flags(result.data_ptr<float>(), ld, grad.data_ptr<float>(), grad.stride(0), plans[i]->handle,
+                                        degrees.data_ptr<float>(), gate, ld_gate, static_cast<int>(ld), target.flags, stream),
+                "eppgcn_spmm_tiles_flags");
+    };
+    BackwardTarget ahead;                            // of layer i - 1
+    if (i > 0) ahead = backward_target(i - 1, weights, plans, head, x, buffers);
+    if (last) {
       // grad already is the gradient of the aggregated rows: aggregated, gated and scaled in one pass
-      const int64_t k = weights[i].size(0), ld = padded_width(k);
-      const int *rows = nullptr;
-      int listed = 0;
-      epp_check(eppgcn_tile_plan_active_rows(plans[i]->handle, &rows, &listed), "eppgcn_tile_plan_active_rows");
-      const bool by_rows = n >= 65536 && listed < n / 4 * 3;
-      auto next = buffers.rows(n, ld, x).narrow(1, 0, k);
-      {
-        ScopedMark t(1, 2, static_cast<int>(i) + 1, clock_stream);
-        epp_check(eppgcn_spmm_tiles_gated(next.data_ptr<float>(), ld, grad.data_ptr<float>(), grad.stride(0), plans[i]->handle,
-                                          degrees.data_ptr<float>(), acts[i - 1].data_ptr<float>(), acts[i - 1].stride(0),
-                                          static_cast<int>(ld), by_rows ? 0 : 1, stream),
-                  "eppgcn_spmm_tiles_gated");
-      }
-      if (by_rows) clear_missing(next, i);
-      grad = next;
+      ScopedMark t(1, 2, static_cast<int>(i) + 1, clock_stream);
+      TargetClear clear(ahead, plans[i - 1], stream);
+      aggregate(acts[i - 1].data_ptr<float>(), acts[i - 1].stride(0));
+      clear.done();
+      if (way.by_rows) clear_missing(result, i);
+      grad = result;
+      target = ahead;
       continue;
     }
-    const int64_t d = weights[i].size(1), ld = padded_width(d);
-    auto d_prime = buffers.rows(n, ld, x).narrow(1, 0, d);
-    // Rows off the path are zero in d' and in the next gradient.  Where they are many, neither is written nor read: the
-    // weight gradient and the update walk the path's rows, and only rows that the next aggregation gathers all the same
-    // (none on a symmetric graph) are cleared.  Social graphs of 6 edges per vertex, us per epoch over all rows and over the
-    // path's: 500 K vertices, 16 columns, a path of 8, then 66 % of the rows: 491 and 448, of 32 and 78 %: 517 and 492;
-    // 64 columns 1346 and 1167, 1408 and 1300; 200 K 632 and 553.  Beyond 80 % of the rows it loses 1 - 3 %.  Steps of up to
-    // 65,536 vertices are replayed; there the two differ by 2 % either way at 16 columns, and wide ones gain up to 9 %,
-    // which this line leaves.
-    const int *rows = nullptr;
-    int listed = 0;
-    epp_check(eppgcn_tile_plan_active_rows(plans[i]->handle, &rows, &listed), "eppgcn_tile_plan_active_rows");
-    const bool by_rows = i > 0 && d <= 256 && n >= 65536 && listed < n / 4 * 3;
-    const int64_t din = weights[i].size(0), ldi = padded_width(din);
-    const bool both = i > 0 && eppgcn_layer_backward_supported(static_cast<int>(din), static_cast<int>(d));
     {
       ScopedMark t(0, 2, static_cast<int>(i) + 1, clock_stream);
-      auto *tiles = i == 0 || by_rows || both ? eppgcn_spmm_tiles_active : eppgcn_spmm_tiles;
-      epp_check(tiles(d_prime.data_ptr<float>(), ld, grad.data_ptr<float>(), grad.stride(0), plans[i]->handle,
-                      degrees.data_ptr<float>(), static_cast<int>(ld), stream),
-                "eppgcn_spmm_tiles");
+      aggregate(nullptr, 0);
     }
     ScopedMark t(1, 3, 0, clock_stream);
-    if (both) {
+    if (!way.both) add_weight_grad(sums + offsets[i], i ? acts[i - 1] : x, result, plans[i]->handle, /*relu_x=*/i > 0, stream);
+    if (i == 0) break;
+    auto next = buffers.rows(n, ldi, x).narrow(1, 0, din);
+    const float *gate = acts[i - 1].data_ptr<float>(), *w = weights[i].data_ptr<float>();
+    TargetClear clear(ahead, plans[i - 1], stream);
+    if (way.both) {
       // rows off the path: those that the next aggregation gathers all the same, or simply all become zero
-      auto next = buffers.rows(n, ldi, x).narrow(1, 0, din);
       const int *zeros = nullptr;
       int zero_count = 0;
-      torch::Tensor missing;
-      if (by_rows) {
-        std::tie(missing, zero_count) = missing_rows(plans[i], plans[i - 1], n, stream);
-        buffers.hold(missing);
-        if (zero_count) zeros = missing.data_ptr<int>();
+      torch::Tensor list;
+      if (way.by_rows) {
+        std::tie(list, zero_count) = missing(i);
+        if (zero_count) zeros = list.data_ptr<int>();
       } else {
         epp_check(eppgcn_tile_plan_empty_rows(plans[i]->handle, &zeros, &zero_count), "eppgcn_tile_plan_empty_rows");
       }
-      epp_check(eppgcn_layer_backward(next.data_ptr<float>(), ldi, sums + offsets[i], d_prime.data_ptr<float>(), ld,
-                                      acts[i - 1].data_ptr<float>(), acts[i - 1].stride(0), weights[i].data_ptr<float>(),
-                                      degrees.data_ptr<float>(), listed == n ? nullptr : rows, listed, zeros, zero_count,
-                                      static_cast<int>(din), static_cast<int>(d), stream),
+      epp_check(eppgcn_layer_backward(next.data_ptr<float>(), ldi, sums + offsets[i], result.data_ptr<float>(), ld, gate,
+                                      acts[i - 1].stride(0), w, degrees.data_ptr<float>(), way.listed == n ? nullptr : way.rows,
+                                      way.listed, zeros, zero_count, static_cast<int>(din), static_cast<int>(d), stream),
                 "eppgcn_layer_backward");
-      grad = next;
-      continue;
-    }
-    add_weight_grad(sums + offsets[i], i ? acts[i - 1] : x, d_prime, plans[i]->handle, /*relu_x=*/i > 0, stream);
-    if (i == 0) break;
-    auto next = buffers.rows(n, ldi, x).narrow(1, 0, din);
-    const float *gate = acts[i - 1].data_ptr<float>();
-    if (by_rows) {
-      epp_check(eppgcn_update_listed(next.data_ptr<float>(), ldi, d_prime.data_ptr<float>(), ld,
-                                     weights[i].data_ptr<float>(), 1, d, degrees.data_ptr<float>(), gate,
-                                     acts[i - 1].stride(0), 0, rows, listed, static_cast<int>(d), static_cast<int>(din),
-                                     static_cast<int>(ldi - din), stream),
+      clear.done();
+    } else if (way.by_rows) {
+      epp_check(eppgcn_update_listed(next.data_ptr<float>(), ldi, result.data_ptr<float>(), ld, w, 1, d,
+                                     degrees.data_ptr<float>(), gate, acts[i - 1].stride(0), 0, way.rows, way.listed,
+                                     static_cast<int>(d), static_cast<int>(din), static_cast<int>(ldi - din), stream),
                 "eppgcn_update_listed");
+      clear.done();
       clear_missing(next, i);
     } else {
-      update_rows(next.data_ptr<float>(), ldi, d_prime, ld, weights[i].data_ptr<float>(), 1, d, degrees.data_ptr<float>(), gate,
-                  acts[i - 1].stride(0), false, n, d, din, ldi - din, buffers, stream);
+      update_rows(next.data_ptr<float>(), ldi, result, ld, w, 1, d, degrees.data_ptr<float>(), gate, acts[i - 1].stride(0), false,
+                  n, d, din, ldi - din, buffers, stream);
+      clear.done();
     }
     grad = next;
+    target = ahead;
   }
 }
 
@@ -863,8 +928,8 @@ std::vector<torch::Tensor> net_backward(torch::Tensor grad, torch::Tensor sums, 
   const auto offsets = sum_offsets(weights, &total);
   auto dw_sums = at::zeros({total}, x.options());
   NetBuffers buffers;
-  run_backward(grad, aligned16(x), weights, acts, degrees, plans, dw_sums.data_ptr<float>(), offsets, false, buffers,
-               current_stream(), current_stream());
+  run_backward(grad, backward_target(weights.size() - 1, weights, plans, false, x, buffers), aligned16(x), weights, acts, degrees,
+               plans, dw_sums.data_ptr<float>(), offsets, false, buffers, current_stream(), current_stream());
   return finish_step(weights, dw_sums.data_ptr<float>(), sums.data_ptr<double>(), offsets, current_stream());
 }
 
@@ -940,11 +1005,14 @@ class NetStep {
       float *sums = sums_.data_ptr<float>();
       auto acts = run_forward(x16, weights, plan->handle, degrees, false, head, buffers, on, stream);
       auto *loss = reinterpret_cast<double *>(sums);
+      auto target = backward_target(weights.size() - 1, weights, plans_, head, x16, buffers);
+      TargetClear clear(target, plans_.back(), on);
       auto grad = head ? run_head(acts.back(), weights.back(), labels, mask, degrees, plans_.back()->handle,
                                   sums + offsets_.back(), loss, buffers, on, stream)
                        : run_loss(acts.back(), labels, mask, degrees, plans_.back()->handle, loss, buffers, on);
+      clear.done();
       acts.pop_back();
-      run_backward(grad, x16, weights, acts, degrees, plans_, sums, offsets_, head, buffers, on, stream);
+      run_backward(grad, std::move(target), x16, weights, acts, degrees, plans_, sums, offsets_, head, buffers, on, stream);
     };
     sums_ = at::empty({total_}, x.options());
     const auto x16 = aligned16(x);

@@ -35,6 +35,7 @@ struct HeadArgs {
   double *sums;                                // {loss, labelled rows}, added to
   int n, k, classes;
   bool flags_vec;                              // four flags in one load
+  ClearList clear;
   ClockMark mark;
 };
 
@@ -49,6 +50,7 @@ __global__ void __launch_bounds__(kHeadWarps * 32, KT * NT <= 3 ? 2 : 1) head_ke
   __shared__ double s_loss[kHeadWarps];
   __shared__ int s_count[kHeadWarps];
   if (blockIdx.x == 0 && threadIdx.x == 0) clock_begin(a.mark);
+  clear_rows(a.clear);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   auto weight = [&](int f, int c) { return f < a.k && c < a.classes ? __ldg(a.w + static_cast<long long>(f) * a.classes + c) : 0.f; };
   for (int e = threadIdx.x; e < KT * NT * 32; e += blockDim.x) {
@@ -407,7 +409,8 @@ EPP_EXPORT int eppgcn_head_step(float *grad, long long ld_grad, float *dw, doubl
   int sms = 148;
   if (const int rc = device_sm_count(&sms); rc != EPP_OK) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const HeadArgs a{s, ld_s, w, labels, mask, used, row_scale, grad, ld_grad, dw, sums, num_rows, k, num_classes, aligned(mask, 4) && aligned(used, 4), take_mark()};
+  const HeadArgs a{s, ld_s, w, labels, mask, used, row_scale, grad, ld_grad, dw, sums, num_rows, k, num_classes, aligned(mask, 4) && aligned(used, 4), take_clear(st),
+                   take_mark()};
   const int nt = (num_classes + 7) / 8;
   if (k <= 16) {
     switch (nt) {

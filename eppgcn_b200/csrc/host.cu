@@ -407,3 +407,32 @@ EPP_EXPORT int eppgcn_clear_time(void) {
   t.acc[4] = mask;
   return EPP_OK;
 }
+
+// ---------------------------------------------------------------------------
+// Rows to be cleared by the calling thread's next kernel (see ClearList).
+// ---------------------------------------------------------------------------
+namespace epp {
+namespace {
+thread_local ClearList t_clear{};
+thread_local cudaStream_t t_clear_stream = nullptr;
+thread_local bool t_clear_open = false, t_clear_done = false;
+}  // namespace
+void want_clear(const ClearList &c, cudaStream_t s) {
+  t_clear = c;
+  t_clear_stream = s;
+  t_clear_open = c.count > 0;
+  t_clear_done = c.count == 0;
+}
+ClearList take_clear(cudaStream_t s) {
+  if (!t_clear_open || s != t_clear_stream) return ClearList{};
+  t_clear_open = false;
+  t_clear_done = true;
+  return t_clear;
+}
+}  // namespace epp
+
+EPP_EXPORT int eppgcn_clear_end(void) {
+  const bool done = epp::t_clear_done;
+  epp::t_clear_open = epp::t_clear_done = false;
+  return done;
+}

@@ -25,8 +25,9 @@ struct LayerBackwardArgs {
   long long ldd, ldx;
   const float *w;                  // [k][dout]
   const float *scale;
-  const int *rows, *zeros;         // rows of d, x and out that are meant, or NULL: all; rows of out that become zero
-  int n, zero_count, k, dout;
+  const int *rows;                 // rows of d, x and out that are meant, or NULL: all
+  int n, k, dout;
+  ClearList zero, clear;           // of out, and of the next aggregation's result
   ClockMark mark;
 };
 
@@ -59,10 +60,8 @@ __global__ void __launch_bounds__(kLbWarps * 32, (LayerBackwardShape<KT, DT>::RE
     split3(weight(f, c), weight(f, c + 1), at[0].x, at[32].x, at[64].x);
     split3(weight(f, c + 2), weight(f, c + 3), at[0].y, at[32].y, at[64].y);
   }
-  const int quads = static_cast<int>(a.ld_out / 4);
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < static_cast<long long>(a.zero_count) * quads;
-       i += static_cast<long long>(gridDim.x) * blockDim.x)
-    *reinterpret_cast<float4 *>(a.out + __ldg(a.zeros + i / quads) * a.ld_out + i % quads * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+  clear_rows(a.zero);
+  clear_rows(a.clear);
   __syncthreads();
 
   const int units = static_cast<int>((static_cast<long long>(a.n) + 15) / 16);
@@ -309,7 +308,8 @@ EPP_EXPORT int eppgcn_layer_backward(float *out, long long ld_out, float *dw, co
   int sms = 148;
   if (const int rc = device_sm_count(&sms); rc != EPP_OK) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const LayerBackwardArgs a{out, ld_out, dw, d, x, ldd, ldx, w, row_scale, rows, zeros, num_rows, zero_count, k, dout, take_mark()};
+  const LayerBackwardArgs a{out, ld_out, dw, d, x, ldd, ldx, w, row_scale, rows, num_rows, k, dout,
+                            ClearList{out, ld_out, zeros, zero_count, static_cast<int>(ld_out / 4)}, take_clear(s), take_mark()};
   if (k <= 16) return dout <= 16 ? launch_layer_backward<1, 1>(a, sms, s) : launch_layer_backward<1, 2>(a, sms, s);
   return dout <= 16 ? launch_layer_backward<2, 1>(a, sms, s) : launch_layer_backward<2, 2>(a, sms, s);
 }

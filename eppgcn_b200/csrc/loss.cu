@@ -51,7 +51,8 @@ __global__ void __launch_bounds__(256) masked_nll_kernel(const float *__restrict
                                                          const unsigned char *__restrict__ mask, int n, int classes,
                                                          float *__restrict__ grad, long long ldg,
                                                          const unsigned char *__restrict__ used,
-                                                         const float *__restrict__ scale, double *sums, int align) {
+                                                         const float *__restrict__ scale, double *sums, int align, const ClearList clear) {
+  clear_rows(clear);
   constexpr int kUnlabelled = -1, kWrongLabel = -2;
   __shared__ int s_row[8][64], s_label[8][64];        // row | top bit where its gradient is wanted; label
   const int lane = threadIdx.x & 31, warp_in_block = threadIdx.x >> 5;
@@ -154,7 +155,8 @@ __global__ void __launch_bounds__(256) masked_nll_wide_kernel(const float *__res
                                                               const unsigned char *__restrict__ mask, int n, int classes,
                                                               float *__restrict__ grad, long long ldg,
                                                               const unsigned char *__restrict__ used,
-                                                              const float *__restrict__ scale, double *sums, int align) {
+                                                              const float *__restrict__ scale, double *sums, int align, const ClearList clear) {
+  clear_rows(clear);
   const int lane = threadIdx.x & 31;
   const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
@@ -267,8 +269,10 @@ EPP_EXPORT int eppgcn_masked_nll(float *grad, long long grad_ld, double *sums, c
   long long blocks = ceil_div_ll(num_rows, 256);
   if (blocks > 148 * 8) blocks = 148 * 8;
   const unsigned g = static_cast<unsigned>(blocks);
+  const ClearList clear = take_clear(s);
   auto run = [&](auto kernel) {
-    kernel<<<g, 256, 0, s>>>(logits, ld, labels, mask, num_rows, num_classes, grad, grad_ld, used, row_scale, sums, align);
+    kernel<<<g, 256, 0, s>>>(logits, ld, labels, mask, num_rows, num_classes, grad, grad_ld, used, row_scale, sums, align,
+                          clear);
   };
   // a lane holds a gradient row, padding included, while that leaves room for the warps that hide each other's loads
   if (grad_ld <= 8) run(masked_nll_kernel<2>);

@@ -366,7 +366,9 @@ __global__ void __launch_bounds__(256) zero_listed_rows_kernel(float *out, long 
 
 // Rows that were summed with atomics, once all of their pieces are in.
 template <int F>
-__global__ void __launch_bounds__(256) finish_rows_kernel(const TileArgs a, const int *__restrict__ rows, int count) {
+__global__ void __launch_bounds__(256) finish_rows_kernel(const TileArgs a, const int *__restrict__ rows, int count,
+                                                          const ClearList clear) {
+  clear_rows(clear);
   const int quads = (a.dim + 3) / 4;
   const long long total = static_cast<long long>(count) * quads;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -627,8 +629,10 @@ template <int SV>
 __global__ void __launch_bounds__(256) pack_scaled_rows_kernel(float *dst, long long dst_ld, const float *__restrict__ x,
                                                                long long ldx, const float *__restrict__ scale,
                                                                const unsigned char *__restrict__ used,
-                                                               int num_rows, int dim, const ClockMark mark) {
+                                                               int num_rows, int dim, const ClearList clear,
+                                                               const ClockMark mark) {
   if (blockIdx.x == 0 && threadIdx.x == 0) clock_begin(mark);
+  clear_rows(clear);
   const int per_row = (dim + 3) / 4;
   const long long total = static_cast<long long>(num_rows) * per_row;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -953,12 +957,13 @@ EPP_EXPORT int eppgcn_pack_scaled_rows(float *dst, long long dst_ld, const float
   const unsigned g = static_cast<unsigned>(blocks);
   const unsigned char *used = plan ? plan->used : nullptr;
   const ClockMark mark = take_mark();
+  const ClearList clear = take_clear(s);
   if (ldx % 4 == 0 && aligned(x, 16))
-    pack_scaled_rows_kernel<4><<<g, 256, 0, s>>>(dst, dst_ld, x, ldx, scale, used, num_rows, dim, mark);
+    pack_scaled_rows_kernel<4><<<g, 256, 0, s>>>(dst, dst_ld, x, ldx, scale, used, num_rows, dim, clear, mark);
   else if (ldx % 2 == 0 && aligned(x, 8))
-    pack_scaled_rows_kernel<2><<<g, 256, 0, s>>>(dst, dst_ld, x, ldx, scale, used, num_rows, dim, mark);
+    pack_scaled_rows_kernel<2><<<g, 256, 0, s>>>(dst, dst_ld, x, ldx, scale, used, num_rows, dim, clear, mark);
   else
-    pack_scaled_rows_kernel<1><<<g, 256, 0, s>>>(dst, dst_ld, x, ldx, scale, used, num_rows, dim, mark);
+    pack_scaled_rows_kernel<1><<<g, 256, 0, s>>>(dst, dst_ld, x, ldx, scale, used, num_rows, dim, clear, mark);
   EPP_CHECK_LAUNCH("pack_scaled_rows_kernel");
   return EPP_OK;
 }
@@ -1034,10 +1039,12 @@ static int run_tiles(float *out, long long out_ld, const float *src, long long s
                                          : launch_columns<kPlain>(a, cols, ovec, s);
     if (rc != EPP_OK) return rc;
     if (finish.how == kPlain || plan->hub_rows == 0) continue;
-    const long long blocks = std::min<long long>(ceil_div_ll(static_cast<long long>(plan->hub_rows) * ((a.dim + 3) / 4), 256), 148 * 8);
+    const ClearList clear = take_clear(s);
+    const long long work = std::max(static_cast<long long>(plan->hub_rows) * ((a.dim + 3) / 4), static_cast<long long>(clear.count) * clear.quads);
+    const unsigned blocks = static_cast<unsigned>(std::min<long long>(ceil_div_ll(work, 256), 148 * 8));
     a.mark = take_mark();
-    if (finish.how == kRelu) finish_rows_kernel<kRelu><<<static_cast<unsigned>(blocks), 256, 0, s>>>(a, plan->zero_rows, plan->hub_rows);
-    else finish_rows_kernel<kGate><<<static_cast<unsigned>(blocks), 256, 0, s>>>(a, plan->zero_rows, plan->hub_rows);
+    if (finish.how == kRelu) finish_rows_kernel<kRelu><<<blocks, 256, 0, s>>>(a, plan->zero_rows, plan->hub_rows, clear);
+    else finish_rows_kernel<kGate><<<blocks, 256, 0, s>>>(a, plan->zero_rows, plan->hub_rows, clear);
     EPP_CHECK_LAUNCH("finish_rows_kernel");
   }
   return EPP_OK;
@@ -1045,7 +1052,8 @@ static int run_tiles(float *out, long long out_ld, const float *src, long long s
 
 // `every_row`: rows without edges become zero; else they are left as they are.
 static int aggregate(float *out, long long out_ld, const float *src, long long src_ld, const eppgcn_tile_plan *plan,
-                     const float *row_scale, int dim, bool every_row, const FinishBy &finish, void *stream) {
+                     const float *row_scale, int dim, bool every_row, bool cleared, const FinishBy &finish,
+                     void *stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   EPP_REQUIRE(plan, "null plan");
   EPP_REQUIRE(dim >= 1, "dim < 1");
@@ -1064,7 +1072,8 @@ static int aggregate(float *out, long long out_ld, const float *src, long long s
   }
   // rows without edges and rows that are summed with atomics start from zero
   const int num_zero = every_row ? plan->num_zero : plan->hub_rows;      // hub rows come first in the list
-  if (every_row && plan->zero_all) {
+  if (cleared) {
+  } else if (every_row && plan->zero_all) {
     if (out_ld == dim) EPP_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(float) * static_cast<size_t>(n) * dim, s));
     else if (const int rc = zero_column_block(out, out_ld, dim, n, s); rc != EPP_OK) return rc;
   } else if (num_zero > 0) {
@@ -1084,23 +1093,29 @@ static int aggregate(float *out, long long out_ld, const float *src, long long s
 
 EPP_EXPORT int eppgcn_spmm_tiles(float *out, long long out_ld, const float *src, long long src_ld,
                                  const eppgcn_tile_plan *plan, const float *row_scale, int dim, void *stream) {
-  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, true, {kPlain, nullptr, 0}, stream);
+  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, true, false, {kPlain, nullptr, 0}, stream);
 }
 
 EPP_EXPORT int eppgcn_spmm_tiles_active(float *out, long long out_ld, const float *src, long long src_ld,
                                         const eppgcn_tile_plan *plan, const float *row_scale, int dim, void *stream) {
-  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, false, {kPlain, nullptr, 0}, stream);
+  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, false, false, {kPlain, nullptr, 0}, stream);
 }
 
-EPP_EXPORT int eppgcn_spmm_tiles_relu(float *out, long long out_ld, const float *src, long long src_ld,
-                                      const eppgcn_tile_plan *plan, const float *row_scale, int dim, void *stream) {
-  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, true, {kRelu, nullptr, 0}, stream);
-}
-
-EPP_EXPORT int eppgcn_spmm_tiles_gated(float *out, long long out_ld, const float *src, long long src_ld,
+EPP_EXPORT int eppgcn_spmm_tiles_flags(float *out, long long out_ld, const float *src, long long src_ld,
                                        const eppgcn_tile_plan *plan, const float *row_scale, const float *gate,
-                                       long long ld_gate, int dim, int every_row, void *stream) {
-  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, every_row != 0, {kGate, gate, ld_gate}, stream);
+                                       long long ld_gate, int dim, int flags, void *stream) {
+  EPP_REQUIRE(!(gate && (flags & EPP_TILES_RELU)), "rows are finished by relu or by a gate");
+  return aggregate(out, out_ld, src, src_ld, plan, row_scale, dim, (flags & EPP_TILES_EVERY_ROW) != 0,
+                   (flags & EPP_TILES_CLEARED) != 0, {gate ? kGate : (flags & EPP_TILES_RELU) ? kRelu : kPlain, gate, ld_gate},
+                   stream);
+}
+
+EPP_EXPORT int eppgcn_clear_begin(float *out, long long out_ld, int dim, const eppgcn_tile_plan *plan, int every_row, void *stream) {
+  EPP_REQUIRE(out && plan && dim >= 1 && out_ld >= dim, "bad argument");
+  (void)eppgcn_clear_end();
+  if (out_ld % 4 == 0 && dim % 4 == 0 && aligned(out, 16))
+    want_clear({out, out_ld, plan->zero_rows, every_row ? plan->num_zero : plan->hub_rows, dim / 4}, static_cast<cudaStream_t>(stream));
+  return EPP_OK;
 }
 
 // Rows that `of` names as sources and `plan` has no edge for.

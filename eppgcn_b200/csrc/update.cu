@@ -34,6 +34,7 @@ struct UpdateArgs {
   bool relu_x;
   bool x_vec, out_vec;                 // 16-byte pieces possible
   bool whole_cols, gate_vec;           // the same over all columns rounded up to a multiple of 8
+  ClearList clear;
   ClockMark mark;
 };
 
@@ -133,6 +134,7 @@ template <int NT, bool LIST>
 __global__ void __launch_bounds__(kMmaWarps * 32, ManyRowsShape<NT>::RESIDENT) update_many_rows_kernel(const UpdateArgs a) {
   constexpr int AHEAD = ManyRowsShape<NT>::AHEAD;
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) clock_begin(a.mark);
+  clear_rows(a.clear);
   extern __shared__ __align__(16) uint2 mma_w[];       // [step][n tile][piece][lane]
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int steps = (a.k + 15) / 16;
@@ -414,6 +416,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, few_rows_resident(NT)) update_
   };
 #pragma unroll
   for (int u = 0; u < S - 1; ++u) stage();
+  clear_rows(a.clear);
 
   float top[NT][M][4], rest[NT][M][4];
 #pragma unroll
@@ -693,6 +696,7 @@ static int update_impl(float *out, long long ld_out, const float *x, long long l
   if (a.parts < 1) a.parts = 1;
   a.scratch = static_cast<float *>(scratch);
   a.scratch_cols = static_cast<int>(u.row_floats());
+  a.clear = take_clear(s);
   a.mark = take_mark();
   int rc;
   switch (u.nt) {

@@ -173,14 +173,20 @@ int eppgcn_spmm_tiles(float *out, long long out_ld, const float *src, long long 
 /* eppgcn_spmm_tiles without clearing the rows that have no edge (they keep what they hold). */
 int eppgcn_spmm_tiles_active(float *out, long long out_ld, const float *src, long long src_ld,
                              const eppgcn_tile_plan *plan, const float *row_scale, int dim, void *stream);
-/* eppgcn_spmm_tiles whose rows y = row_scale * sum leave finished: as the source rows of a next aggregation,
- * row_scale * relu(y); or, backward, row_scale * y where gate != 0 and zero elsewhere (rows without an edge are cleared
- * with every_row != 0).  16-byte aligned result and gate rows, padded to a multiple of 4 floats. */
-int eppgcn_spmm_tiles_relu(float *out, long long out_ld, const float *src, long long src_ld,
-                           const eppgcn_tile_plan *plan, const float *row_scale, int dim, void *stream);
-int eppgcn_spmm_tiles_gated(float *out, long long out_ld, const float *src, long long src_ld,
+/* eppgcn_spmm_tiles (with EPP_TILES_EVERY_ROW) or eppgcn_spmm_tiles_active whose rows y = row_scale * sum may leave
+ * finished: with EPP_TILES_RELU as the source rows of a next aggregation, row_scale * relu(y); with a gate, backward, as
+ * row_scale * y where gate != 0 and zero elsewhere.  Those want 16-byte aligned rows, padded to a multiple of 4 floats.
+ * EPP_TILES_CLEARED: the rows that eppgcn_clear_begin names have been cleared. */
+enum { EPP_TILES_EVERY_ROW = 1, EPP_TILES_RELU = 2, EPP_TILES_CLEARED = 4 };
+int eppgcn_spmm_tiles_flags(float *out, long long out_ld, const float *src, long long src_ld,
                             const eppgcn_tile_plan *plan, const float *row_scale, const float *gate, long long ld_gate,
-                            int dim, int every_row, void *stream);
+                            int dim, int flags, void *stream);
+/* Between the two calls the calling thread's next update, packing, loss, head or layer-backward kernel on the stream, or the
+ * last kernel of an aggregation that finishes its rows, also clears the rows of `out` that an aggregation over `plan` wants
+ * cleared (with every_row those without an edge too).  eppgcn_clear_end: whether one has, or there was nothing to clear;
+ * the wish ends with it. */
+int eppgcn_clear_begin(float *out, long long out_ld, int dim, const eppgcn_tile_plan *plan, int every_row, void *stream);
+int eppgcn_clear_end(void);
 /* sums_dev[0..1]: two 64-bit hash sums over the edges (row, source) of `plan`; sums_dev[2..3]: the same over the edges of
  * `of` taken as (source, row), of the rows that `plan` names as sources.  Equal pairs: what `plan` gathers from a row,
  * `of` gathers into it -- `plan` is the transposed of those rows of `of` (up to hash collisions, 2^-64 each). */

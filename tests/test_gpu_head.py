@@ -145,6 +145,50 @@ def test_rows_leave_finished(cuda, dim, graph):
     assert (some[empty] == 7.0).all() and torch.equal(some[~empty & ~hubs], want[~empty & ~hubs]) and close.all()
 
 
+@pytest.mark.parametrize("by", ["update", "few rows", "packing", "finish", "head", "layer"])
+def test_the_kernel_before_an_aggregation_clears_its_rows(cuda, by):
+    """Hub rows and empty rows are cleared by whichever kernel comes before; a wish ends with its bracket."""
+    lib = capi.lib()
+    indptr, indices = random_csr(n=2000, avg_deg=3.0, seed=5, empty_frac=0.5, hubs=3, hub_deg=900)
+    n, dim, deg = len(indptr) - 1, 16, t(degrees_of(indptr), cuda)
+    plan = capi.TilePlan.from_csr(t(indptr, cuda), t(indices, cuda))
+    src = torch.randn(n, dim, device=cuda)
+    want = capi.spmm_tiles(src, plan, deg)
+    stream = torch.cuda.current_stream().cuda_stream
+    for every_row in (1, 0):
+        out = torch.full((n, dim), 5.0, device=cuda)
+        capi.check(lib.eppgcn_clear_begin(out.data_ptr(), dim, dim, plan._handle, every_row, stream))
+        if by == "update":
+            capi.update_rows(torch.randn(40_000, 16, device=cuda), torch.randn(16, 16, device=cuda))
+        elif by == "few rows":
+            capi.update_rows(torch.randn(50, 1433, device=cuda), torch.randn(1433, 16, device=cuda))
+        elif by == "packing":
+            capi.pack_scaled_rows(src, deg, plan)
+        elif by == "finish":
+            capi.spmm_tiles_finished(src, plan, deg)
+        elif by == "head":
+            ones = torch.ones(n, dtype=torch.bool, device=cuda)
+            capi.head_step(src, torch.randn(16, 5, device=cuda), ones.long(), ones, ones.to(torch.uint8))
+        else:
+            capi.layer_backward(src, src, torch.randn(16, 16, device=cuda))
+        assert lib.eppgcn_clear_end() == 1 and lib.eppgcn_clear_end() == 0
+        touched = t((np.diff(indptr) > 64) | ((np.diff(indptr) == 0) & (every_row == 1)), cuda)
+        assert (out[touched] == 0).all() and (out[~touched] == 5.0).all()
+        flags = capi.TILES_CLEARED | every_row
+        capi.check(lib.eppgcn_spmm_tiles_flags(out.data_ptr(), dim, src.data_ptr(), dim, plan._handle, deg.data_ptr(), None, 0, dim,
+                                               flags, stream))
+        rows = torch.ones(n, dtype=torch.bool, device=cuda) if every_row else t(np.diff(indptr) > 0, cuda)
+        assert torch.allclose(out[rows], want[rows], rtol=1e-5, atol=1e-5) and (out[~rows] == 5.0).all()
+    out = torch.full((n, dim), 5.0, device=cuda)
+    capi.check(lib.eppgcn_clear_begin(out.data_ptr(), dim, dim, plan._handle, 1, stream))
+    assert lib.eppgcn_clear_end() == 0
+    capi.layer_backward(src, src, torch.randn(16, 16, device=cuda))           # no wish any more
+    side = torch.cuda.Stream()
+    capi.check(lib.eppgcn_clear_begin(out.data_ptr(), dim, dim, plan._handle, 1, side.cuda_stream))
+    capi.layer_backward(src, src, torch.randn(16, 16, device=cuda))           # another stream's
+    assert lib.eppgcn_clear_end() == 0 and (out == 5.0).all()
+
+
 def test_edge_hashes_tell_transposed_lists(cuda):
     rng = np.random.Generator(np.random.PCG64(1))
     n = 3000

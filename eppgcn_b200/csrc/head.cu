@@ -7,8 +7,8 @@
 // the hidden layer instead of the classes', and leaves the layer's products to the rows that the loss looks at; their
 // results stay in registers: the logits, their gradient and the layer's two gradient products cost no memory traffic
 // beyond s and grad.  As separate kernels (update of every row, loss, weight gradient, update of the path's rows) 16 -> 22
-// on 1.13 M rows, half of them labelled, took 258 us, 66 here; 16 -> 47 on 1 M rows, 30 % labelled, 334 and 71.  Bound by
-// instructions (1000 for 16 rows, issue slots 52 % busy at 16 warps per SM): 2.5 and 3.5 times the time of its bytes.
+// on 1.13 M rows, half of them labelled, took 258 us, 66 here; 16 -> 47 on 1 M rows, 30 % labelled, 334 and 64.  Bound by
+// instructions (1000 for 16 rows, issue slots 52 % busy at 16 warps per SM): 2.5 and 3 times the time of its bytes.
 //
 // A warp queues rows that have something to do (as the loss kernel does) and takes 16 at a time, the next 16 on their way.
 // Everything is in the fragment layouts of mma.m16n8k16 (mma_split.cuh): four lanes hold a row, lane t its features
@@ -19,7 +19,12 @@
 namespace epp {
 namespace {
 
-constexpr int kHeadWarps = 8;
+// Warps per block and blocks per SM that leave each warp the registers it needs (1 M rows, 47 classes: 69 us with 8 warps,
+// 64 with 12, 71 with 16).
+template <int KT, int NT>
+struct HeadShape {
+  static constexpr int WARPS = KT * NT <= 3 || KT * NT > 6 ? 8 : 12, RESIDENT = KT * NT <= 3 ? 2 : 1;
+};
 constexpr long long kNoLabel = -100;          // nll_loss's ignore_index
 
 struct HeadArgs {
@@ -41,14 +46,14 @@ struct HeadArgs {
 
 // KT pieces of 16 features, NT pieces of 8 classes; rows are looked over PER per lane at a time.
 template <int KT, int NT, int PER>
-__global__ void __launch_bounds__(kHeadWarps * 32, KT * NT <= 3 ? 2 : 1) head_kernel(const HeadArgs a) {
-  constexpr int CT = (NT + 1) / 2, F = 16 * KT;
+__global__ void __launch_bounds__(HeadShape<KT, NT>::WARPS * 32, (HeadShape<KT, NT>::RESIDENT)) head_kernel(const HeadArgs a) {
+  constexpr int CT = (NT + 1) / 2, F = 16 * KT, WARPS = HeadShape<KT, NT>::WARPS;
   constexpr int kUnlabelled = -1, kWrongLabel = -2;
   __shared__ uint2 s_w[KT * NT * 96], s_wt[CT * 2 * KT * 96];      // fragments: [step][tile][piece][lane]
   __shared__ float s_dw[F * 8 * NT];
-  __shared__ int2 s_queue[kHeadWarps][256];    // row | top bit where its gradient is wanted; whether it has a label
-  __shared__ double s_loss[kHeadWarps];
-  __shared__ int s_count[kHeadWarps];
+  __shared__ int2 s_queue[WARPS][256];    // row | top bit where its gradient is wanted; whether it has a label
+  __shared__ double s_loss[WARPS];
+  __shared__ int s_count[WARPS];
   if (blockIdx.x == 0 && threadIdx.x == 0) clock_begin(a.mark);
   clear_rows(a.clear);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
@@ -262,8 +267,8 @@ __global__ void __launch_bounds__(kHeadWarps * 32, KT * NT <= 3 ? 2 : 1) head_ke
   };
 
   int2 *const queue = s_queue[warp];
-  const long long stride = static_cast<long long>(gridDim.x) * kHeadWarps * kWarp * PER;
-  long long base = (static_cast<long long>(blockIdx.x) * kHeadWarps + warp) * kWarp * PER;
+  const long long stride = static_cast<long long>(gridDim.x) * WARPS * kWarp * PER;
+  long long base = (static_cast<long long>(blockIdx.x) * WARPS + warp) * kWarp * PER;
   int first = 0, queued = 0;                   // the queue: a ring of 256
   unsigned f_used = 0, f_mask = 0;             // flags of the next rows, one or four per lane, on their way
   auto flags = [&]() {
@@ -343,7 +348,7 @@ __global__ void __launch_bounds__(kHeadWarps * 32, KT * NT <= 3 ? 2 : 1) head_ke
     s_count[warp] = count;
   }
 #pragma unroll 1
-  for (int w = 0; w < kHeadWarps; ++w) {
+  for (int w = 0; w < WARPS; ++w) {
     if (w == warp) {
 #pragma unroll
       for (int s = 0; s < KT; ++s)
@@ -359,7 +364,7 @@ __global__ void __launch_bounds__(kHeadWarps * 32, KT * NT <= 3 ? 2 : 1) head_ke
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    for (int i = 1; i < kHeadWarps; ++i) {
+    for (int i = 1; i < WARPS; ++i) {
       s_loss[0] += s_loss[i];
       s_count[0] += s_count[i];
     }
@@ -378,9 +383,9 @@ __global__ void __launch_bounds__(kHeadWarps * 32, KT * NT <= 3 ? 2 : 1) head_ke
 template <int KT, int NT>
 int launch_head(const HeadArgs &a, int sms, cudaStream_t s) {
   // four flags per lane on large graphs, whose labelled rows are far between; on small ones as many warps as there are 32 rows
-  const long long most = static_cast<long long>(sms) * (KT * NT <= 3 ? 2 : 1), chunks = ceil_div_ll(a.n, kHeadWarps * kWarp);
-  if (chunks >= 8 * most) head_kernel<KT, NT, 4><<<static_cast<unsigned>(most), kHeadWarps * 32, 0, s>>>(a);
-  else head_kernel<KT, NT, 1><<<static_cast<unsigned>(chunks < most ? chunks : most), kHeadWarps * 32, 0, s>>>(a);
+  const long long most = static_cast<long long>(sms) * HeadShape<KT, NT>::RESIDENT, chunks = ceil_div_ll(a.n, HeadShape<KT, NT>::WARPS * kWarp);
+  if (chunks >= 8 * most) head_kernel<KT, NT, 4><<<static_cast<unsigned>(most), HeadShape<KT, NT>::WARPS * 32, 0, s>>>(a);
+  else head_kernel<KT, NT, 1><<<static_cast<unsigned>(chunks < most ? chunks : most), HeadShape<KT, NT>::WARPS * 32, 0, s>>>(a);
   EPP_CHECK_LAUNCH("head_kernel");
   return EPP_OK;
 }

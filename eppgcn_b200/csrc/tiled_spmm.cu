@@ -601,10 +601,11 @@ __global__ void __launch_bounds__(256) fill_slots_kernel(const int *__restrict__
   int k = 0;
   while (k + 1 < t.count && at >= t.slot_off[k + 1]) ++k;
   const int w = t.width[k];
-  const long long in_class = at - t.slot_off[k];
+  const unsigned quad = static_cast<unsigned>((at - t.slot_off[k]) >> 2);    // 32 bits hold it and divide in a third of the time
   int v[4];
   if (w >= 4) {
-    const int rank = t.rank_off[k] + static_cast<int>(in_class / w), j = static_cast<int>(in_class % w);
+    const unsigned per = static_cast<unsigned>(w) >> 2, in_class = quad / per;
+    const int rank = t.rank_off[k] + static_cast<int>(in_class), j = static_cast<int>(quad - in_class * per) * 4;
     const int len = __ldg(seg_len + rank) - j;
     const int *p = col + __ldg(seg_start + rank) + j;
 #pragma unroll
@@ -612,7 +613,7 @@ __global__ void __launch_bounds__(256) fill_slots_kernel(const int *__restrict__
   } else {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int rank = t.rank_off[k] + static_cast<int>((in_class + q) / w), j = static_cast<int>((in_class + q) % w);
+      const int rank = t.rank_off[k] + static_cast<int>(w == 2 ? 2 * quad + q / 2 : 4 * quad + q), j = w == 2 ? q % 2 : 0;
       v[q] = j < __ldg(seg_len + rank) ? __ldg(col + __ldg(seg_start + rank) + j) : -1;
     }
   }
@@ -724,10 +725,12 @@ __global__ void __launch_bounds__(256) hash_edges_kernel(const int *__restrict__
     const int w = t.width[k];
     const int4 ids = __ldg(reinterpret_cast<const int4 *>(slots + at));
     const int c[4] = {ids.x, ids.y, ids.z, ids.w};
+    const unsigned quad = static_cast<unsigned>((at - t.slot_off[k]) >> 2);
+    const int *const rank = row_of + t.rank_off[k] + (w >= 4 ? quad / (static_cast<unsigned>(w) >> 2) : 4u / static_cast<unsigned>(w) * quad);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       if (c[q] < 0) continue;
-      const int row = static_cast<int>(static_cast<unsigned>(__ldg(row_of + t.rank_off[k] + (at + q - t.slot_off[k]) / w)) & ~kAtomicBit);
+      const int row = static_cast<int>(static_cast<unsigned>(__ldg(rank + (w >= 4 ? 0 : w == 2 ? q / 2 : q))) & ~kAtomicBit);
       if (only && !only[row]) continue;
       const unsigned long long e = only ? static_cast<unsigned long long>(c[q]) << 32 | static_cast<unsigned>(row)
                                         : static_cast<unsigned long long>(row) << 32 | static_cast<unsigned>(c[q]);

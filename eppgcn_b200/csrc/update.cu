@@ -39,6 +39,7 @@ struct UpdateArgs {
 };
 
 constexpr int kMmaWarps = 8;
+constexpr int kClearNT = 6;            // many-row kernels of wider results have no register to spare: 346 -> 363 us at 64 columns
 constexpr int kMmaMaxK = 256;          // W's fragments fit into shared memory (96 KB at 64 columns)
 
 // The arguments of one block of columns, c0 .. c0 + width - 1.
@@ -126,15 +127,15 @@ __device__ __forceinline__ bool all_nan(const float *w, long long w_row, long lo
 // ---------------------------------------------------------------------------
 template <int NT>
 struct ManyRowsShape {
-  static constexpr int AHEAD = NT == 1 ? 4 : NT == 2 || NT == 4 ? 3 : 2;        // 16-k steps of x in flight, 2 KB each
-  static constexpr int RESIDENT = NT <= 3 ? 2 : 1;     // blocks per SM
+  static constexpr int AHEAD = NT == 1 ? 4 : 2;         // 16-k steps of x in flight, 2 KB each (three of 2 M x 128 -> 16: 241 us, 228)
+  static constexpr int RESIDENT = NT <= 4 ? 2 : 1;     // blocks per SM (1 M x 64 -> 32 with one and three steps: 150 us, 119)
 };
 
 template <int NT, bool LIST>
 __global__ void __launch_bounds__(kMmaWarps * 32, ManyRowsShape<NT>::RESIDENT) update_many_rows_kernel(const UpdateArgs a) {
   constexpr int AHEAD = ManyRowsShape<NT>::AHEAD;
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) clock_begin(a.mark);
-  clear_rows(a.clear);
+  if constexpr (NT <= kClearNT) clear_rows(a.clear);
   extern __shared__ __align__(16) uint2 mma_w[];       // [step][n tile][piece][lane]
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int steps = (a.k + 15) / 16;
@@ -589,6 +590,12 @@ UpdateShape update_shape(int n, int k, int dout, bool listed, int sms) {
   const int blocks = (dout + 63) / 64;
   u.nt = ((dout + blocks - 1) / blocks + 7) / 8;
   u.col_blocks = (dout + 8 * u.nt - 1) / (8 * u.nt);
+  // Listed rows of more than 32 results have their gate and ids to wait for besides: two blocks of half the columns per SM
+  // (0.8 M listed rows x 64 -> 64 292 us, 231; without list or gate 1 M x 64 -> 64 214 and 215, x 128 -> 64 346 and 389).
+  if (listed && u.nt > 4) {
+    u.nt = 4;
+    u.col_blocks = (dout + 31) / 32;
+  }
   // From one tile of 32 rows per resident warp on, the many-row kernel keeps the chip busy; results of more than four
   // blocks go through the other, which does not hold W's fragments for every block.
   u.many_rows = listed || (k <= kMmaMaxK && n >= 32 * kMmaWarps * sms && u.col_blocks <= 4);
@@ -696,7 +703,7 @@ static int update_impl(float *out, long long ld_out, const float *x, long long l
   if (a.parts < 1) a.parts = 1;
   a.scratch = static_cast<float *>(scratch);
   a.scratch_cols = static_cast<int>(u.row_floats());
-  a.clear = take_clear(s);
+  if (!u.many_rows || u.nt <= kClearNT) a.clear = take_clear(s);
   a.mark = take_mark();
   int rc;
   switch (u.nt) {

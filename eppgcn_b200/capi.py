@@ -58,6 +58,8 @@ SIGNATURES = {
     "eppgcn_tile_plan_empty_rows": (_I, [_P, _P, _P]),
     "eppgcn_layer_backward_supported": (_I, [_I, _I]),
     "eppgcn_layer_backward": (_I, [_P, _LL, _P, _P, _LL, _P, _LL, _P, _P, _P, _I, _P, _I, _I, _I, _P]),
+    "eppgcn_prepare_lists_scratch_bytes": (_SZ, [_I, _I, _I]),
+    "eppgcn_prepare_lists": (_I, [_I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _I, _P, _SZ, _P, _P]),
     "eppgcn_head_supported": (_I, [_I, _I]),
     "eppgcn_head_step": (_I, [_P, _LL, _P, _P, _P, _LL, _P, _P, _P, _P, _P, _I, _I, _I, _P]),
     "eppgcn_masked_nll": (_I, [_P, _LL, _P, _P, _LL, _P, _P, _P, _P, _I, _I, _P]),

@@ -1423,6 +1423,78 @@ std::tuple<std::vector<torch::Tensor>, std::vector<int>> split_back_parts(std::v
   return {parts, counts};
 }
 
+// compact_back_edges, the part size by `rule` (0: constant, 1: map, 2: bucket; at least 1) and split_back_parts with one
+// synchronisation: (ids, edge_lists, valid_lens, part sizes, part_pointers, part counts).
+std::tuple<std::vector<torch::Tensor>, std::vector<torch::Tensor>, std::vector<int>, std::vector<int>, std::vector<torch::Tensor>,
+           std::vector<int>>
+prepare_paths(std::vector<torch::Tensor> edge_masks, torch::Tensor column_index, std::vector<torch::Tensor> node_degs, int num_edges,
+              int rule, int constant) {
+  const size_t lists = edge_masks.size();
+  TORCH_CHECK(lists >= 1 && lists <= 16 && node_degs.size() == lists, "1 to 16 lists, one node_deg per edge_mask");
+  CHECK_INPUT(column_index); CHECK_I32(column_index);
+  const int64_t length = column_index.numel(), nodes = node_degs[0].numel();
+  TORCH_CHECK(length >= 1 && nodes >= 1 && length < (1LL << 31) && nodes < (1LL << 31), "count exceeds int32, or nothing to prepare");
+  TORCH_CHECK(num_edges >= 0 && num_edges < 0x7fffffff, "num_edges must be non-negative");
+  c10::cuda::CUDAGuard guard(column_index.device());
+  std::vector<torch::Tensor> ids, edges, parts;
+  std::vector<const int *> masks, degs;
+  std::vector<int *> out_ids, out_edges, out_parts;
+  for (size_t i = 0; i < lists; ++i) {
+    CHECK_INPUT(edge_masks[i]); CHECK_INPUT(node_degs[i]); CHECK_I32(edge_masks[i]); CHECK_I32(node_degs[i]);
+    TORCH_CHECK(edge_masks[i].numel() == length, "edge_mask and column_index must have equal length");
+    TORCH_CHECK(node_degs[i].numel() == nodes, "node_degs must have equal lengths");
+    ids.push_back(at::empty_like(edge_masks[i]));
+    edges.push_back(at::empty_like(column_index));
+    parts.push_back(at::empty({num_edges + 1}, node_degs[i].options()));
+    masks.push_back(edge_masks[i].data_ptr<int>());
+    degs.push_back(node_degs[i].data_ptr<int>());
+    out_ids.push_back(ids.back().data_ptr<int>());
+    out_edges.push_back(edges.back().data_ptr<int>());
+    out_parts.push_back(parts.back().data_ptr<int>());
+  }
+  const size_t bytes = eppgcn_prepare_lists_scratch_bytes(static_cast<int>(lists), static_cast<int>(length), static_cast<int>(nodes));
+  auto scratch = at::empty({static_cast<int64_t>(bytes / 8)}, column_index.options().dtype(at::kLong));
+  auto results = at::empty({static_cast<int64_t>(6 * lists)}, column_index.options());
+  epp_check(eppgcn_prepare_lists(static_cast<int>(lists), masks.data(), column_index.data_ptr<int>(), degs.data(), out_ids.data(),
+                                 out_edges.data(), static_cast<int>(length), static_cast<int>(nodes), rule, constant,
+                                 out_parts.data(), num_edges + 1, scratch.data_ptr(), bytes, results.data_ptr<int>(),
+                                 current_stream()),
+            "eppgcn_prepare_lists");
+  const auto host = results.cpu();
+  const int *r = host.data_ptr<int>(), *split = r + 4 * lists;
+  std::vector<int> valid, sizes, counts;
+  for (size_t i = 0; i < lists; ++i) {
+    int len = r[4 * i], size = r[4 * i + 3];
+    const int active = r[4 * i + 2];
+    bool again = split[2 * i + 1] != EPP_OK;
+    if (r[4 * i + 1] != EPP_OK) {        // a bounded wait ran out: once more, list by list, which repeats without waiting
+      Compacted c = compact_edges(edge_masks[i], column_index);
+      ids[i] = c.id;
+      edges[i] = c.edge_list;
+      len = c.valid_len;
+      again = true;
+    }
+    if (rule == EPP_PART_SIZE_MAP) {     // refuses a list without active vertices
+      int from_counts = 0;
+      epp_check(eppgcn_map_back_part_size(active, len, &from_counts), "eppgcn_map_back_part_size");
+      if (r[4 * i + 1] != EPP_OK) size = std::max(from_counts, 1);
+    } else if (rule == EPP_PART_SIZE_BUCKET && r[4 * i + 1] != EPP_OK) {
+      const int d = len / std::max(active, 1);
+      size = d < 4 ? 4 : d < 16 ? 8 : d < 64 ? 16 : d < 256 ? 32 : 64;
+    }
+    int count = split[2 * i];
+    if (again) {
+      Split one = split_parts(node_degs[i], num_edges, size);
+      parts[i] = one.part_pointer;
+      count = one.num_parts;
+    }
+    valid.push_back(len);
+    sizes.push_back(size);
+    counts.push_back(count);
+  }
+  return {ids, edges, valid, sizes, parts, counts};
+}
+
 // The rule of get_map_back_part_size where the number of active vertices is known.
 int map_back_part_size(int active, int valid_len) {
   int ps = 0;
@@ -1490,6 +1562,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("net_backward", &net_backward, "loss and weight gradients of a stack of layers (not in the reference)");
   m.def("compact_back_edges", &compact_back_edges, "compact_back_edge of several layers at once (not in the reference)");
   m.def("split_back_parts", &split_back_parts, "split_back_part of several layers at once (not in the reference)");
+  m.def("prepare_paths", &prepare_paths, "compaction, part sizes and splitting of several layers at once (not in the reference)");
   m.def("map_back_part_size", &map_back_part_size, "the rule of get_map_back_part_size from counts (not in the reference)");
   py::class_<NetStep>(m, "NetStep", "a training step's forward, loss and backward in one call (not in the reference)")
       .def(py::init<>())

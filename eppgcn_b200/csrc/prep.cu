@@ -19,6 +19,7 @@ constexpr int kCompactItems = 8;                                  // per thread
 constexpr int kCompactTile = kScanThreads * kCompactItems;        // 4096 edges
 constexpr int kSplitItems = 4;
 constexpr int kSplitTile = kScanThreads * kSplitItems;            // 2048 vertices
+constexpr int kOneWaveTiles = 148 * 4;                            // that fit onto the chip together
 constexpr int kMaxPolls = 1 << 21;                                // bounded look-back wait
 
 enum ScanMode { kLookback = 0, kCountOnly = 1, kGivenOffsets = 2 };
@@ -290,8 +291,9 @@ __global__ void __launch_bounds__(kScanThreads) compact_mask_kernel(const Compac
   }
 }
 
-// Exclusive scan of packed tile totals by one block (fallback mode).
-__global__ void __launch_bounds__(1024) scan_tiles_kernel(unsigned long long *desc, int num_tiles) {
+// Exclusive scan of packed tile totals, one block per list; the lists' arrays lie `stride` words apart.
+__global__ void __launch_bounds__(1024) scan_tiles_kernel(unsigned long long *desc, int num_tiles, size_t stride) {
+  desc += blockIdx.x * stride;
   __shared__ unsigned long long s_warp[33];
   __shared__ unsigned long long s_carry;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -341,6 +343,7 @@ struct SplitArgs {
   unsigned long long *desc;
   int *num_parts, *status;
   int part_size, out_len, part2node_len;
+  const int *part_size_dev;          // where it lies, or NULL: part_size
 };
 struct SplitBatch {                 // one list per blockIdx.y
   SplitArgs list[kBatch];
@@ -363,7 +366,7 @@ __global__ void __launch_bounds__(kScanThreads) split_parts_kernel(const SplitBa
   int *__restrict__ part_pointer = a.part_pointer;
   int *__restrict__ part2node = a.part2node;
   const int num_nodes = batch.num_nodes, num_tiles = batch.num_tiles;
-  const int part_size = a.part_size, out_len = a.out_len, part2node_len = a.part2node_len;
+  const int part_size = a.part_size_dev ? __ldg(a.part_size_dev) : a.part_size, out_len = a.out_len, part2node_len = a.part2node_len;
   ScanHeader *hdr = a.hdr;
   unsigned long long *desc = a.desc;
   __shared__ unsigned s_warp[kScanWarps + 1][2];
@@ -593,7 +596,7 @@ EPP_EXPORT int eppgcn_compact_mask(const int *edge_mask, const int *col_idx, int
   } else {
     compact_mask_kernel<kCountOnly><<<tiles, kScanThreads, 0, s>>>(b);
     EPP_CHECK_LAUNCH("compact_mask_kernel<count>");
-    scan_tiles_kernel<<<1, 1024, 0, s>>>(b.list[0].desc, tiles);
+    scan_tiles_kernel<<<1, 1024, 0, s>>>(b.list[0].desc, tiles, 0);
     EPP_CHECK_LAUNCH("scan_tiles_kernel");
     compact_mask_kernel<kGivenOffsets><<<tiles, kScanThreads, 0, s>>>(b);
     EPP_CHECK_LAUNCH("compact_mask_kernel<scatter>");
@@ -634,8 +637,19 @@ EPP_EXPORT int eppgcn_compact_masks(int lists, const int *const *edge_masks, con
   EPP_CUDA_TRY(cudaMemsetAsync(results_dev, 0, sizeof(int) * 4 * lists, s));
   if (length > 0) {
     EPP_CUDA_TRY(cudaMemsetAsync(scratch, 0, lists * list_scratch_bytes(tiles), s));
-    compact_mask_kernel<kLookback><<<dim3(tiles, lists), kScanThreads, 0, s>>>(b);
-    EPP_CHECK_LAUNCH("compact_mask_kernel<lookback, batch>");
+    // Tiles that all start at once look back over each other in one launch.  Where there are more, waiting for the tiles
+    // before costs more than counting first and reading the masks twice (3 x 13 M edges: 227 us, 169).
+    if (static_cast<long long>(tiles) * lists <= kOneWaveTiles) {
+      compact_mask_kernel<kLookback><<<dim3(tiles, lists), kScanThreads, 0, s>>>(b);
+      EPP_CHECK_LAUNCH("compact_mask_kernel<lookback, batch>");
+    } else {
+      compact_mask_kernel<kCountOnly><<<dim3(tiles, lists), kScanThreads, 0, s>>>(b);
+      EPP_CHECK_LAUNCH("compact_mask_kernel<count, batch>");
+      scan_tiles_kernel<<<lists, 1024, 0, s>>>(b.list[0].desc, tiles, list_scratch_bytes(tiles) / sizeof(unsigned long long));
+      EPP_CHECK_LAUNCH("scan_tiles_kernel");
+      compact_mask_kernel<kGivenOffsets><<<dim3(tiles, lists), kScanThreads, 0, s>>>(b);
+      EPP_CHECK_LAUNCH("compact_mask_kernel<scatter, batch>");
+    }
   }
   if (num_nodes > 0) {
     count_nonzero_kernel<<<dim3(tail_grid(num_nodes), lists), 256, 0, s>>>(n);
@@ -736,7 +750,7 @@ static int launch_split(const SplitArgs &a, int num_nodes, int mode, cudaStream_
   } else {
     split_parts_kernel<kCountOnly><<<b.num_tiles, kScanThreads, 0, s>>>(b);
     EPP_CHECK_LAUNCH("split_parts_kernel<count>");
-    scan_tiles_kernel<<<1, 1024, 0, s>>>(a.desc, b.num_tiles);
+    scan_tiles_kernel<<<1, 1024, 0, s>>>(a.desc, b.num_tiles, 0);
     EPP_CHECK_LAUNCH("scan_tiles_kernel");
     split_parts_kernel<kGivenOffsets><<<b.num_tiles, kScanThreads, 0, s>>>(b);
     EPP_CHECK_LAUNCH("split_parts_kernel<scatter>");
@@ -755,6 +769,26 @@ EPP_EXPORT size_t eppgcn_split_lists_scratch_bytes(int lists, int num_nodes) {
   return lists < 1 ? 0 : static_cast<size_t>(lists) * list_scratch_bytes(ceil_div_ll(num_nodes < 0 ? 0 : num_nodes, kSplitTile));
 }
 
+// part_sizes: on the host, or -- one of the two -- in device memory, `size_stride` ints apart.
+static int split_lists(int lists, const int *const *node_degs, int num_nodes, const int *part_sizes, const int *part_sizes_dev,
+                       int size_stride, int *const *part_pointers, int out_len, void *scratch, int *results_dev,
+                       int result_stride, cudaStream_t s) {
+  SplitBatch b{};
+  b.num_nodes = num_nodes;
+  b.num_tiles = static_cast<int>(ceil_div_ll(num_nodes, kSplitTile));
+  for (int i = 0; i < lists; ++i) {
+    EPP_REQUIRE(node_degs[i] && part_pointers[i] && (!part_sizes || part_sizes[i] >= 1), "null pointer or part size < 1");
+    b.list[i] = split_args(node_degs[i], part_sizes ? part_sizes[i] : 0, part_pointers[i], out_len, nullptr, 0,
+                           static_cast<char *>(scratch) + i * list_scratch_bytes(b.num_tiles), results_dev + result_stride * i,
+                           results_dev + result_stride * i + 1);
+    if (!part_sizes) b.list[i].part_size_dev = part_sizes_dev + size_stride * i;
+  }
+  EPP_CUDA_TRY(cudaMemsetAsync(scratch, 0, lists * list_scratch_bytes(b.num_tiles), s));
+  split_parts_kernel<kLookback><<<dim3(b.num_tiles, lists), kScanThreads, 0, s>>>(b);
+  EPP_CHECK_LAUNCH("split_parts_kernel<lookback, batch>");
+  return zero_split_tails(b, lists, out_len, s);
+}
+
 EPP_EXPORT int eppgcn_split_lists(int lists, const int *const *node_degs, int num_nodes, const int *part_sizes,
                                   int *const *part_pointers, int out_len, void *scratch, size_t scratch_bytes,
                                   int *results_dev, void *stream) {
@@ -764,20 +798,56 @@ EPP_EXPORT int eppgcn_split_lists(int lists, const int *const *node_degs, int nu
   EPP_REQUIRE(node_degs && part_sizes && part_pointers && scratch && results_dev, "null pointer");
   EPP_REQUIRE(scratch_bytes >= eppgcn_split_lists_scratch_bytes(lists, num_nodes), "scratch too small");
   EPP_REQUIRE(reinterpret_cast<uintptr_t>(scratch) % 8 == 0, "scratch must be 8-byte aligned");
-  SplitBatch b{};
-  b.num_nodes = num_nodes;
-  b.num_tiles = static_cast<int>(ceil_div_ll(num_nodes, kSplitTile));
-  for (int i = 0; i < lists; ++i) {
-    EPP_REQUIRE(node_degs[i] && part_pointers[i] && part_sizes[i] >= 1, "null pointer or part size < 1");
-    b.list[i] = split_args(node_degs[i], part_sizes[i], part_pointers[i], out_len, nullptr, 0,
-                           static_cast<char *>(scratch) + i * list_scratch_bytes(b.num_tiles), results_dev + 2 * i,
-                           results_dev + 2 * i + 1);
-  }
   EPP_CUDA_TRY(cudaMemsetAsync(results_dev, 0, sizeof(int) * 2 * lists, s));
-  EPP_CUDA_TRY(cudaMemsetAsync(scratch, 0, lists * list_scratch_bytes(b.num_tiles), s));
-  split_parts_kernel<kLookback><<<dim3(b.num_tiles, lists), kScanThreads, 0, s>>>(b);
-  EPP_CHECK_LAUNCH("split_parts_kernel<lookback, batch>");
-  return zero_split_tails(b, lists, out_len, s);
+  return split_lists(lists, node_degs, num_nodes, part_sizes, nullptr, 0, part_pointers, out_len, scratch, results_dev, 2, s);
+}
+
+// The part size of every list from its counts, as eppgcn_map_back_part_size and the bucket rule give it, at least 1.
+// results: {valid, status, active, size, ...} per list.
+__global__ void part_sizes_kernel(int *results, int stride, int lists, int rule, int constant) {
+  const int i = threadIdx.x;
+  if (i >= lists) return;
+  int *const r = results + i * stride;
+  const int valid = r[0], active = r[2];
+  int size = constant;
+  if (rule == EPP_PART_SIZE_MAP && active > 0) {      // rounded like the host's sum: no fused multiply-add
+    const double degree = __ddiv_rn(static_cast<double>(valid), static_cast<double>(active));
+    double sum = __dadd_rn(0.65538, __dmul_rn(1.67431e-5, static_cast<double>(active)));
+    sum = __dadd_rn(sum, __dmul_rn(-2.24342e-6, static_cast<double>(valid)));
+    sum = __dadd_rn(sum, __dmul_rn(0.63641, degree));
+    size = static_cast<int>(round(sum));
+  } else if (rule == EPP_PART_SIZE_BUCKET) {
+    const int d = valid / max(active, 1);
+    size = d < 4 ? 4 : d < 16 ? 8 : d < 64 ? 16 : d < 256 ? 32 : 64;
+  }
+  r[3] = max(size, 1);
+}
+
+EPP_EXPORT size_t eppgcn_prepare_lists_scratch_bytes(int lists, int length, int num_nodes) {
+  return eppgcn_compact_masks_scratch_bytes(lists, length) + eppgcn_split_lists_scratch_bytes(lists, num_nodes);
+}
+
+EPP_EXPORT int eppgcn_prepare_lists(int lists, const int *const *edge_masks, const int *col_idx, const int *const *node_degs,
+                                    int *const *out_ids, int *const *out_edges, int length, int num_nodes, int rule, int constant,
+                                    int *const *part_pointers, int out_len, void *scratch, size_t scratch_bytes,
+                                    int *results_dev, void *stream) {
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  EPP_REQUIRE(lists >= 0 && lists <= kBatch && num_nodes >= 1 && length >= 1 && out_len >= 1, "bad size (at most 16 lists)");
+  if (lists == 0) return EPP_OK;
+  EPP_REQUIRE(rule == EPP_PART_SIZE_CONSTANT || rule == EPP_PART_SIZE_MAP || rule == EPP_PART_SIZE_BUCKET, "unknown rule");
+  EPP_REQUIRE(part_pointers && scratch && results_dev, "null pointer");
+  EPP_REQUIRE(scratch_bytes >= eppgcn_prepare_lists_scratch_bytes(lists, length, num_nodes), "scratch too small");
+  const size_t compact_bytes = eppgcn_compact_masks_scratch_bytes(lists, length);
+  int *const split_results = results_dev + 4 * lists;
+  if (const int rc = eppgcn_compact_masks(lists, edge_masks, col_idx, node_degs, out_ids, out_edges, length, num_nodes, scratch,
+                                          compact_bytes, results_dev, stream);
+      rc != EPP_OK)
+    return rc;
+  EPP_CUDA_TRY(cudaMemsetAsync(split_results, 0, sizeof(int) * 2 * lists, s));
+  part_sizes_kernel<<<1, kBatch, 0, s>>>(results_dev, 4, lists, rule, constant);
+  EPP_CHECK_LAUNCH("part_sizes_kernel");
+  return split_lists(lists, node_degs, num_nodes, nullptr, results_dev + 3, 4, part_pointers, out_len,
+                     static_cast<char *>(scratch) + compact_bytes, split_results, 2, s);
 }
 
 EPP_EXPORT int eppgcn_split_parts(const int *node_deg, int num_nodes, int part_size, int *part_pointer,

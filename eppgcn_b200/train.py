@@ -251,10 +251,17 @@ class GCNTrainer:
         if (hasattr(GNNA, "compact_back_edges") and self.layers <= 16
                 and not _replaced(self, "choose_back_size", _CHOOSE_BACK_SIZE)
                 and self.backsize_mode in ("map", "bucket", "constant")):
-            # all layers in one go: two synchronisations instead of three per layer
-            ids, edges, valid, active = GNNA.compact_back_edges(ds.edge_masks, self.inputInfo.column_index, ds.node_degs)
-            sizes = [self._part_size(a, v) for a, v in zip(active, valid)]
-            parts, counts = GNNA.split_back_parts(ds.node_degs, ds.num_edges, sizes)
+            if (hasattr(GNNA, "prepare_paths") and not _replaced(self, "_part_size", _PART_SIZE)
+                    and ds.num_edges > 0 and ds.num_nodes > 0):
+                # all layers in one go, the part sizes taken on the device: one synchronisation
+                ids, edges, valid, sizes, parts, counts = GNNA.prepare_paths(
+                    ds.edge_masks, self.inputInfo.column_index, ds.node_degs, ds.num_edges,
+                    ("constant", "map", "bucket").index(self.backsize_mode), max(int(self.backsize), 1))
+            else:
+                # two synchronisations instead of three per layer
+                ids, edges, valid, active = GNNA.compact_back_edges(ds.edge_masks, self.inputInfo.column_index, ds.node_degs)
+                sizes = [self._part_size(a, v) for a, v in zip(active, valid)]
+                parts, counts = GNNA.split_back_parts(ds.node_degs, ds.num_edges, sizes)
             for prop, i, e, v, p, size, n in zip(self.back_props, ids, edges, valid, parts, sizes, counts):
                 prop.fillProperty(i, p, e, size, n)
                 prop.valid_len = v
@@ -360,7 +367,7 @@ class GCNTrainer:
         return loss
 
 
-_TRAINER_FORWARD, _CHOOSE_BACK_SIZE = GCNTrainer.forward, GCNTrainer.choose_back_size
+_TRAINER_FORWARD, _CHOOSE_BACK_SIZE, _PART_SIZE = GCNTrainer.forward, GCNTrainer.choose_back_size, GCNTrainer._part_size
 
 
 def build_parser() -> argparse.ArgumentParser:

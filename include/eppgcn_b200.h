@@ -376,6 +376,15 @@ size_t eppgcn_split_lists_scratch_bytes(int lists, int num_nodes);
 int eppgcn_split_lists(int lists, const int *const *node_degs, int num_nodes, const int *part_sizes,
                        int *const *part_pointers, int out_len, void *scratch, size_t scratch_bytes,
                        int *results_dev, void *stream);
+/* Both, with the part size of a list taken on the device from its counts: by the rule of eppgcn_map_back_part_size, by the
+ * buckets 4, 8, 16, 32, 64 for averages below 4, 16, 64, 256 and the rest, or constant; at least 1.  results_dev (6 ints
+ * per list): {valid_len, status, active vertices, part size} of every list, then {num_parts, status} of every list. */
+enum { EPP_PART_SIZE_CONSTANT = 0, EPP_PART_SIZE_MAP = 1, EPP_PART_SIZE_BUCKET = 2 };
+size_t eppgcn_prepare_lists_scratch_bytes(int lists, int length, int num_nodes);
+int eppgcn_prepare_lists(int lists, const int *const *edge_masks, const int *col_idx, const int *const *node_degs,
+                         int *const *out_ids, int *const *out_edges, int length, int num_nodes, int rule, int constant,
+                         int *const *part_pointers, int out_len, void *scratch, size_t scratch_bytes,
+                         int *results_dev, void *stream);
 
 /* ------------------------------------------------------------------------
  * Stable compaction of the marked edges.

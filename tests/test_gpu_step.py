@@ -197,6 +197,45 @@ def test_batched_preparation(cuda, n, avg, part_size):
         assert np.array_equal(parts[i].cpu().numpy(), w["partPointer"])
 
 
+@pytest.mark.parametrize("n,pairs", [(1, 0), (50, 80), (20_000, 90_000), (300_000, 400_000), (300_000, 5_000_000)])
+def test_paths_prepared_at_once(cuda, n, pairs):
+    """One call for compaction, part sizes and splitting gives the lists of the separate ones, bit for bit: one tile, one wave
+    of tiles (a look-back) and more (counted first); every rule, and a list without a marked edge."""
+    import eppgcn_b200
+    from eppgcn_b200 import graphs
+    gnna = eppgcn_b200.load_gnnadvisor()
+    rng = np.random.Generator(np.random.PCG64(n + pairs))
+    src, dst = rng.integers(0, n, pairs), rng.integers(0, n, pairs)
+    dst[::5] //= 1000
+    indptr, indices = graphs.csr_from_pairs(n, src, dst)
+    col, e = torch.from_numpy(indices).to(cuda), len(indices)
+    rows = torch.repeat_interleave(torch.arange(n, device=cuda), torch.from_numpy(np.diff(indptr)).to(cuda)).int()
+    masks, degs = [], []
+    for share in (0.03, 0.4, 1.0, 0.0):
+        on = torch.rand(n, device=cuda) < share
+        on[0] = share > 0
+        masks.append(torch.where(on[col.long()], rows, -1))
+        degs.append(torch.zeros(n, dtype=torch.int32, device=cuda).index_add_(0, rows.long(), on[col.long()].int()))
+    for rule, lists in (("map", 3), ("bucket", 4), ("constant", 4)):
+        ids, edges, valid, active = gnna.compact_back_edges(masks[:lists], col, degs[:lists])
+        sizes = []
+        for a, v in zip(active, valid):
+            d = v // max(a, 1)
+            sizes.append(7 if rule == "constant" else max(gnna.map_back_part_size(a, v), 1) if rule == "map" else
+                         4 if d < 4 else 8 if d < 16 else 16 if d < 64 else 32 if d < 256 else 64)
+        parts, counts = gnna.split_back_parts(degs[:lists], e, sizes)
+        got = gnna.prepare_paths(masks[:lists], col, degs[:lists], e, ("constant", "map", "bucket").index(rule), 7)
+        assert got[2] == valid and got[3] == sizes and got[5] == counts
+        for a, b in zip(got[0] + got[1] + got[4], ids + edges + parts):
+            assert torch.equal(a, b)
+        for i in range(lists):
+            keep = masks[i] != -1
+            assert valid[i] == int(keep.sum()) and torch.equal(ids[i][:valid[i]], rows[keep]) and not ids[i][valid[i]:].any()
+            assert torch.equal(edges[i][:valid[i]], col[keep]) and not edges[i][valid[i]:].any()
+    with pytest.raises(RuntimeError, match="no active vertex"):
+        gnna.prepare_paths(masks, col, degs, e, 1, 7)
+
+
 @pytest.mark.parametrize("symmetric", [True, False])
 def test_backward_over_the_paths_rows(cuda, symmetric, monkeypatch):
     """Large enough that only the rows of the path are cleared, updated and gathered; on a graph that is not symmetric the

@@ -78,6 +78,28 @@ def test_rows_padded_to_32_bytes(cuda, graph, dim):
     assert_close(got, want, 2e-5, 2e-6, what=f"tiled forward {graph} dim {dim}, rows of {(dim + 7) // 8 * 8}")
 
 
+@pytest.mark.parametrize("n,pairs", [(500, 4000), (60_000, 200_000)])
+@pytest.mark.parametrize("dim", [4, 8, 16, 22, 25, 31, 47, 64, 121])
+def test_few_and_many_rows(cuda, n, pairs, dim):
+    """Fewer tiles than warps and several per warp, rows of every width, dense results and padded ones."""
+    from eppgcn_b200 import graphs
+    rng = np.random.Generator(np.random.PCG64(n))
+    src, dst = rng.integers(0, n, pairs), (rng.pareto(0.8, pairs) * 5).astype(np.int64) % n
+    indptr, indices = graphs.csr_from_pairs(n, src, dst)
+    assert np.diff(indptr).max() > 64 and np.diff(indptr).min() <= 8
+    feat, deg = torch.randn(n, dim, device=cuda), t(degrees_of(indptr), cuda)
+    col, ld = t(indices, cuda), (dim + 7) // 8 * 8
+    plan = capi.TilePlan.from_csr(t(indptr, cuda), col)
+    padded = torch.zeros(n, ld, device=cuda)[:, :dim].copy_(feat * deg[:, None])
+    rows = torch.repeat_interleave(torch.arange(n, device=cuda), torch.from_numpy(np.diff(indptr)).to(cuda))
+    add = lambda m: deg.double()[:, None] * torch.zeros(n, dim, dtype=torch.float64, device=cuda).index_add_(  # noqa: E731
+        0, rows, (deg.double()[:, None] * m)[col.long()])
+    want, mag = add(feat.double()), add(feat.double().abs())
+    for out in (None, torch.empty(n, ld, device=cuda)[:, :dim]):
+        got = capi.spmm_tiles(padded, plan, deg, out=out)
+        assert ((got.double() - want).abs() <= 1e-6 + 2e-6 * mag).all()
+
+
 def test_plan_counts(cuda):
     indptr, indices = random_csr(**GRAPHS["hubs"])
     n = len(indptr) - 1

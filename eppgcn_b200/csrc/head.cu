@@ -7,8 +7,8 @@
 // the hidden layer instead of the classes', and leaves the layer's products to the rows that the loss looks at; their
 // results stay in registers: the logits, their gradient and the layer's two gradient products cost no memory traffic
 // beyond s and grad.  As separate kernels (update of every row, loss, weight gradient, update of the path's rows) 16 -> 22
-// on 1.13 M rows, half of them labelled, took 258 us, 66 here; 16 -> 47 on 1 M rows, 30 % labelled, 334 and 64.  Bound by
-// instructions (1000 for 16 rows, issue slots 52 % busy at 16 warps per SM): 2.5 and 3 times the time of its bytes.
+// on 1.13 M rows, half of them labelled, took 258 us, 73 here; 16 -> 47 on 1 M rows, 30 % labelled, 334 and 69.  Bound by
+// instructions (1100 for 16 rows, issue slots 52 % busy at 16 warps per SM): 4 and 5 times the time of its bytes.
 //
 // A warp queues rows that have something to do (as the loss kernel does) and takes 16 at a time, the next 16 on their way.
 // Everything is in the fragment layouts of mma.m16n8k16 (mma_split.cuh): four lanes hold a row, lane t its features
@@ -19,8 +19,8 @@
 namespace epp {
 namespace {
 
-// Warps per block and blocks per SM that leave each warp the registers it needs (1 M rows, 47 classes: 69 us with 8 warps,
-// 64 with 12, 71 with 16).
+// Warps per block and blocks per SM that leave each warp the registers it needs (1 M rows, 47 classes: 12 warps take 8 %
+// less than 8, 10 % less than 16).
 template <int KT, int NT>
 struct HeadShape {
   static constexpr int WARPS = KT * NT <= 3 || KT * NT > 6 ? 8 : 12, RESIDENT = KT * NT <= 3 ? 2 : 1;
@@ -152,22 +152,22 @@ __global__ void __launch_bounds__(HeadShape<KT, NT>::WARPS * 32, (HeadShape<KT, 
           float &e = z[j][2 * h + q];
           e -= top;
           if (8 * j + q == at) picked = e;
-          e = j == NT - 1 && 8 * j + q >= own ? 0.f : expf(e);
-          sum += e;
+          sum += j == NT - 1 && 8 * j + q >= own ? 0.f : expf(e);
         }
       sum += __shfl_xor_sync(kFull, sum, 1);
       sum += __shfl_xor_sync(kFull, sum, 2);
+      // exp(z - top) / sum would save an exponential and 7 us of 73, and left the gradients up to 15 % further from float64
+      const float log_sum = logf(sum);
       const bool labelled = y[h] != kUnlabelled;
-      if (labelled && y[h] >= 0 && (y[h] & 7) >> 1 == t) loss += static_cast<double>(logf(sum) - picked);
+      if (labelled && y[h] >= 0 && (y[h] & 7) >> 1 == t) loss += static_cast<double>(log_sum - picked);
       if (y[h] == kWrongLabel && t == 0) loss += static_cast<double>(NAN);
       count += labelled && t == 0;
-      const float inv = 1.f / sum;
 #pragma unroll
       for (int j = 0; j < NT; ++j)
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           float &e = z[j][2 * h + q];
-          e = fmaf(e, inv, 8 * j + q == at ? -1.f : 0.f);
+          e = (j == NT - 1 && 8 * j + q >= own ? 0.f : expf(e - log_sum)) - (8 * j + q == at ? 1.f : 0.f);
         }
       if (entry[h] >= 0 || !labelled) {        // no gradient of these, whatever their logits
 #pragma unroll

@@ -122,7 +122,8 @@ __device__ __forceinline__ void block_scan_pair(unsigned a, unsigned b, unsigned
 // 128 at a time.  One group per eight lanes left every edge behind a chain of three dependent loads with a handful of
 // edges to hide them.  BITS: the source mask as one bit per vertex, an eighth of the bytes to gather from (140 KB for
 // 1.13 M vertices: L1 holds it).  13 M edges: 148 us before, 97 now (121 with the bits in shared memory: one block of 32
-// warps per SM hides less).
+// warps per SM hides less).  The group of an edge was searched for among 32 ends, five shuffles per 32 edges; counting the
+// ends in front of it takes a third of that: 68 -> 52 us where issue is the bound (first and last step).
 constexpr int kMaskUnroll = 4;
 
 template <bool BITS>
@@ -153,32 +154,38 @@ __global__ void __launch_bounds__(256) mask_forward_kernel(
   const int beg = __ldg(part_ptr + (has ? g : num_parts)), end = __ldg(part_ptr + (has ? g + 1 : num_parts));
   const bool mark = has && !is_last && end > beg && in_mask<BITS>(src_mask, src_bits, r + row_offset);
   const int all_beg = __shfl_sync(kFull, beg, 0), all_end = __shfl_sync(kFull, end, kWarp - 1);
+  const bool some_empty = __any_sync(kFull, has && end == beg);
   int count = 0;
-  for (long long base = all_beg; base < all_end; base += kMaskUnroll * kWarp) {
+  for (int base = all_beg; base < all_end; base += min(kMaskUnroll * kWarp, all_end - base)) {
     int c[kMaskUnroll];
     bool hit[kMaskUnroll];
 #pragma unroll
     for (int u = 0; u < kMaskUnroll; ++u) {
-      const long long e = base + u * kWarp + lane;
-      c[u] = e < all_end ? __ldg(edge_list + e) : -1;
+      const int at = u * kWarp + lane;
+      c[u] = at < all_end - base ? __ldg(edge_list + base + at) : -1;
     }
 #pragma unroll
     for (int u = 0; u < kMaskUnroll; ++u) hit[u] = c[u] >= 0 && in_mask<BITS>(src_mask, src_bits, c[u]);
 #pragma unroll
     for (int u = 0; u < kMaskUnroll; ++u) {
-      const long long e0 = base + u * kWarp;
-      if (e0 >= all_end) break;
+      if (u * kWarp >= all_end - base) break;
+      const int e0 = base + u * kWarp;
       // this lane's group covers bits [lo, hi) of the 32 edges
-      const long long lo = beg > e0 ? beg - e0 : 0, hi = end - e0 < kWarp ? end - e0 : kWarp;
-      const unsigned below_hi = hi >= kWarp ? kFull : (hi > 0 ? (1u << hi) - 1u : 0u);
-      const unsigned below_lo = lo >= kWarp ? kFull : (1u << lo) - 1u;
+      const int lo = min(max(beg - e0, 0), kWarp), hi = min(max(end - e0, 0), kWarp);
+      const unsigned below_hi = hi >= kWarp ? kFull : (1u << hi) - 1u, below_lo = lo >= kWarp ? kFull : (1u << lo) - 1u;
       count += __popc(__ballot_sync(kFull, hit[u]) & below_hi & ~below_lo);
-      // the group of this lane's edge: the first whose end lies behind it
-      const long long e = e0 + lane;
+      // the group of this lane's edge: as many groups end at or before it.  Their ends as bits, where no two coincide;
+      // else the first group whose end lies behind the edge, by search.
+      const int e = e0 + lane;
       int owner = 0;
+      if (!some_empty) {
+        const unsigned ends = __reduce_or_sync(kFull, hi > 0 && hi < kWarp ? 1u << hi : 0u);
+        owner = min(__popc(__ballot_sync(kFull, hi == 0)) + __popc(ends & ((2u << lane) - 1u)), kWarp - 1);
+      } else {
 #pragma unroll
-      for (int step = kWarp / 2; step >= 1; step >>= 1)
-        if (__shfl_sync(kFull, end, owner + step - 1) <= e) owner += step;
+        for (int step = kWarp / 2; step >= 1; step >>= 1)
+          if (__shfl_sync(kFull, end, owner + step - 1) <= e) owner += step;
+      }
       const int row = __shfl_sync(kFull, r, owner);
       const bool marks = __shfl_sync(kFull, static_cast<int>(mark), owner) != 0;
       if (hit[u]) back_edge_mask[e] = row;
@@ -425,8 +432,14 @@ __global__ void __launch_bounds__(kScanThreads) split_parts_kernel(const SplitBa
   // stretch of slots; where vertices have several parts each, the owner of a
   // lane's next slot, 32 further on, is a few steps away from the last one
   // (11 M parts of one edge: 77 us by searching every slot, 34 by walking).
+  if (part_size == 1 && !part2node) {      // a part is an edge: its pointer is its place (3 x 1.13 M vertices, size 1: 99 us by search, 38)
+    for (unsigned j = threadIdx.x; j < tot_c; j += kScanThreads) {
+      const long long slot = static_cast<long long>(pc) + j;
+      if (slot < out_len) part_pointer[slot] = static_cast<int>(pe + j);
+    }
+  }
   const unsigned per_warp = (tot_c + kScanThreads - 1) / kScanThreads * kWarp;
-  const unsigned stop = min(tot_c, (threadIdx.x / kWarp + 1) * per_warp);
+  const unsigned stop = part_size == 1 && !part2node ? 0u : min(tot_c, (threadIdx.x / kWarp + 1) * per_warp);
   const bool walk = tot_c >= 4u * kSplitTile;
   int lo = -1;
   for (unsigned j = threadIdx.x / kWarp * per_warp + threadIdx.x % kWarp; j < stop; j += kWarp) {

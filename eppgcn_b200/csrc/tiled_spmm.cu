@@ -618,9 +618,41 @@ __global__ void __launch_bounds__(256) fill_slots_kernel(const int *__restrict__
     }
   }
   *reinterpret_cast<int4 *>(slots + at) = make_int4(v[0], v[1], v[2], v[3]);
+  if (!used) return;
 #pragma unroll
   for (int q = 0; q < 4; ++q)
     if (v[q] >= 0 && v[q] < num_sources && used[v[q]] == 0) used[v[q]] = 1;     // most are there already
+}
+
+// Long lists: which sources are named, first as bits in each SM's shared memory, then as bits of all, then as bytes.  A
+// byte of global memory looked at per edge took four times as long as the whole copy of the ids (13 M edges, 1.13 M
+// sources: 130 us; 24 and 4 here).
+constexpr int kMarkThreads = 1024;
+constexpr size_t kMarkSmem = 200 * 1024;
+__global__ void __launch_bounds__(kMarkThreads) mark_sources_kernel(const int *__restrict__ slots, long long count, int num_sources,
+                                                                    unsigned *bits) {
+  extern __shared__ unsigned s_bits[];
+  const int words = (num_sources + 31) / 32;
+  for (int w = threadIdx.x; w < words; w += kMarkThreads) s_bits[w] = 0u;
+  __syncthreads();
+  for (long long at = (static_cast<long long>(blockIdx.x) * kMarkThreads + threadIdx.x) * 4; at < count;
+       at += static_cast<long long>(gridDim.x) * kMarkThreads * 4) {
+    const int4 ids = __ldg(reinterpret_cast<const int4 *>(slots + at));
+    const int v[4] = {ids.x, ids.y, ids.z, ids.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (v[q] < 0 || v[q] >= num_sources) continue;
+      const unsigned bit = 1u << (v[q] & 31);
+      if (!(s_bits[v[q] >> 5] & bit)) atomicOr(s_bits + (v[q] >> 5), bit);
+    }
+  }
+  __syncthreads();
+  for (int w = threadIdx.x; w < words; w += kMarkThreads)
+    if (s_bits[w]) atomicOr(bits + w, s_bits[w]);
+}
+__global__ void __launch_bounds__(256) spread_bits_kernel(const unsigned *__restrict__ bits, int num_sources, unsigned char *used) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v <= num_sources) used[v] = v < num_sources ? __ldg(bits + (v >> 5)) >> (v & 31) & 1u : 0u;
 }
 
 // dst[r][0..dim) = scale[r] * x[r][0..dim) for the rows an edge list names
@@ -847,7 +879,10 @@ int build_plan(eppgcn_tile_plan **out_plan, void *dev_buf, size_t dev_bytes, con
   plan.num_zero = totals[kHubs] + totals[kEmpty];
   plan.zero_all = plan.num_zero > num_rows / 2;       // mostly empty result: one memset beats a long list
 
-  EPP_CUDA_TRY(cudaMemsetAsync(plan.used, 0, static_cast<size_t>(num_sources) + 1, s));
+  // the bits lie where the ranks' lengths lay, once the slots are filled
+  const size_t mark_bytes = (static_cast<size_t>(num_sources) + 31) / 32 * 4;
+  const bool by_bits = slot_off >= (1 << 20) && mark_bytes <= kMarkSmem && mark_bytes <= 4 * bound.ranks;
+  if (!by_bits) EPP_CUDA_TRY(cudaMemsetAsync(plan.used, 0, static_cast<size_t>(num_sources) + 1, s));
   if (num_rows > 0) {
     const size_t rb = sizeof(int) * static_cast<size_t>(rank_off);
     if (rb) {
@@ -859,8 +894,21 @@ int build_plan(eppgcn_tile_plan **out_plan, void *dev_buf, size_t dev_bytes, con
   }
   if (slot_off > 0) {
     fill_slots_kernel<<<static_cast<unsigned>(ceil_div_ll(slot_off, 4 * 256)), 256, 0, s>>>(
-        col_dev, plan.seg_start, plan.seg_len, plan.slots, t, slot_off, plan.used, num_sources);
+        col_dev, plan.seg_start, plan.seg_len, plan.slots, t, slot_off, by_bits ? nullptr : plan.used, num_sources);
     EPP_CHECK_LAUNCH("fill_slots_kernel");
+    if (by_bits) {
+      int sms = 148;
+      if (const int rc = device_sm_count(&sms); rc != EPP_OK) return rc;
+      static SmemOptIn memo;
+      if (const int rc = smem_opt_in(memo, reinterpret_cast<const void *>(mark_sources_kernel), static_cast<int>(kMarkSmem)); rc != EPP_OK)
+        return rc;
+      auto *bits = reinterpret_cast<unsigned *>(plan.seg_len);
+      EPP_CUDA_TRY(cudaMemsetAsync(bits, 0, mark_bytes, s));
+      mark_sources_kernel<<<sms, kMarkThreads, mark_bytes, s>>>(plan.slots, slot_off, num_sources, bits);
+      EPP_CHECK_LAUNCH("mark_sources_kernel");
+      spread_bits_kernel<<<static_cast<unsigned>(num_sources / 256 + 1), 256, 0, s>>>(bits, num_sources, plan.used);
+      EPP_CHECK_LAUNCH("spread_bits_kernel");
+    }
   }
   unsigned long long sums[4] = {0};
   if (of) {                                           // seg_start, at least 64 words, has served its purpose

@@ -217,3 +217,19 @@ def test_edge_hashes_tell_transposed_lists(cuda):
                                       t((key % n).astype(np.int32), cuda))
     h = capi.edge_hashes(directed, directed)
     assert h[:2] != h[2:]
+
+
+@pytest.mark.parametrize("n,sources", [(300_000, 300_000), (200_000, 1_000_001), (30_000, 2_000_000), (700, 31)])
+def test_sources_named_by_long_lists(cuda, n, sources):
+    """Sources marked through shared memory (lists of a million slots and up to 1.6 M sources) or one by one."""
+    rng = np.random.Generator(np.random.PCG64(n))
+    edges = 1_100_000
+    indptr = np.sort(rng.integers(0, edges + 1, n + 1)).astype(np.int32)
+    indptr[0], indptr[-1] = 0, edges
+    indices = (rng.integers(0, sources, edges) // 3 * 3).clip(max=sources - 1).astype(np.int32)
+    plan = capi.TilePlan.from_csr(t(indptr, cuda), t(indices, cuda), num_sources=sources)
+    x = torch.ones(sources, 4, device=cuda)
+    got = capi.pack_scaled_rows(x, torch.ones(sources, device=cuda), plan, out=torch.zeros(sources, 4, device=cuda))
+    want = np.zeros(sources, dtype=bool)
+    want[indices] = True
+    assert np.array_equal((got[:, 0] != 0).cpu().numpy(), want)

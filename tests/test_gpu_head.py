@@ -133,7 +133,6 @@ def test_rows_leave_finished(cuda, dim, graph):
     gate = full[:, :dim]
     plan = capi.TilePlan.from_csr(t(indptr, cuda), t(indices, cuda))
     y = capi.spmm_tiles(src, plan, deg)
-    close = torch.ones(n, dtype=torch.bool, device=cuda)
     hubs = t(np.diff(indptr) > 64, cuda)               # summed in any order: a last bit of their largest term
     for got, want in [(capi.spmm_tiles_finished(src, plan, deg), deg[:, None] * y.clamp(min=0)),
                       (capi.spmm_tiles_finished(src, plan, deg, gate), deg[:, None] * y * (gate != 0))]:
@@ -142,7 +141,7 @@ def test_rows_leave_finished(cuda, dim, graph):
     some = torch.full((n, (dim + 3) // 4 * 4), 7.0, device=cuda)[:, :dim]
     capi.spmm_tiles_finished(src, plan, deg, gate, every_row=False, out=some)
     empty = t(np.diff(indptr) == 0, cuda)
-    assert (some[empty] == 7.0).all() and torch.equal(some[~empty & ~hubs], want[~empty & ~hubs]) and close.all()
+    assert (some[empty] == 7.0).all() and torch.equal(some[~empty & ~hubs], want[~empty & ~hubs])
 
 
 @pytest.mark.parametrize("by", ["update", "few rows", "packing", "finish", "head", "layer"])

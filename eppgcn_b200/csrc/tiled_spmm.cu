@@ -148,6 +148,10 @@ __device__ __forceinline__ void add_cols(float (&acc)[C], const float (&v)[C]) {
   for (int i = 0; i < C; ++i) acc[i] += v[i];
 }
 
+// A row's gate, asked for with its edges but without registers that would wait for it (6.6 M edges on 1.13 M vertices:
+// 110 us without, 96).
+__device__ __forceinline__ void fetch_ahead(const float *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 template <int F>
 __device__ __forceinline__ void finish_piece(float (&y)[4], float scale, const float4 &gate) {
   const float g[4] = {gate.x, gate.y, gate.z, gate.w};
@@ -214,6 +218,7 @@ __device__ __forceinline__ void close_narrow(const TileArgs &a, float *out_lane,
     }
 #endif
     if (rid[r] != -1 && a.row_scale) scale[r] = __ldg(a.row_scale + row);
+    if (F == kGate && rid[r] != -1) fetch_ahead(a.gate + fcol + static_cast<long long>(row) * a.ld_gate);
   }
 #pragma unroll
   for (int r = 0; r < PER; ++r) {
@@ -313,6 +318,7 @@ __global__ void __launch_bounds__(kTileThreads, kTileResident) tiled_spmm_kernel
       }
 #endif
       const float scale = (rid != -1 && a.row_scale) ? __ldg(a.row_scale + row) : 1.f;
+      if (F == kGate && rid >= 0) fetch_ahead(a.gate + fcol + static_cast<long long>(row) * a.ld_gate);
       float acc[C] = {};
       const int *cp = a.slots + pos.slot;
 #pragma unroll 1

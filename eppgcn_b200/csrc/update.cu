@@ -206,6 +206,18 @@ __global__ void __launch_bounds__(kMmaWarps * 32, ManyRowsShape<NT>::RESIDENT) u
         for (int m = 0; m < 2; ++m)
 #pragma unroll
           for (int q = 0; q < 4; ++q) top[j][m][q] = rest[j][m][q] = 0.f;
+      if (LIST && a.gate) {          // on its way while the products are formed (listed 64 -> 64: 241 us, 232; unlisted
+                                     // rows follow each other, and there the addresses' registers cost more: 121, 138)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          long long row = static_cast<long long>(tile) * 32 + 8 * i + g;
+          if (row >= a.n) continue;
+          const float *gate = a.gate + __ldg(a.rows + row) * a.ld_gate + blockIdx.y * 8 * NT;
+#pragma unroll
+          for (int c = 0; c < 8 * NT; c += 32)         // a sector per lane
+            if (blockIdx.y * 8 * NT + c + 8 * t < a.dout) asm volatile("prefetch.global.L1 [%0];" ::"l"(gate + c + 8 * t));
+        }
+      }
     }
     if (a.relu_x) {
 #pragma unroll
